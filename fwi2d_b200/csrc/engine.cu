@@ -430,12 +430,15 @@ static void upload_model_values(fwi2d_ctx *ctx, const float *model)
     up(M.p1, model + nxz);
     if (kind != KIND_ACOUSTIC) up(M.p2, model + 2 * nxz);
     else M.p2.release();
-    M.c13.release();
-    M.eps.release();
-    M.fxx.release();
-    M.lbis.release();
-    M.gv2.release();
-    M.gv3.release();
+    // a live plan's graphs hold these addresses: an update keeps the buffers
+    if (kind != KIND_VTI) {
+        M.c13.release();
+        M.eps.release();
+        M.fxx.release();
+        M.lbis.release();
+        M.gv2.release();
+        M.gv3.release();
+    }
     if (kind == KIND_VTI) {
         const float *lam = M.hp(0), *mu = M.hp(1), *c13 = M.hp(3), *eps = M.hp(4);
         std::vector<float> fxx(nxz), lbis(nxz), v2(nxz), v3(nxz);

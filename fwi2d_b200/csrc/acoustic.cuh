@@ -269,6 +269,7 @@ __global__ void ae_couple(const ShotDev *__restrict__ E, const ShotDev *__restri
     const long long nxz = (long long)e.nx * e.ldz;
     float *n1 = e.u[it & 1] + nxz;              // next uz, row 0
     float *na = w.u[it & 1] + (w.nz - 1);       // next potential, last fluid row
+    float amax = 0.f;   // of the coupled row, which the elastic kernel's maximum has not seen
     for (int ix = blockIdx.x * blockDim.x + threadIdx.x; ix < e.nx; ix += gridDim.x * blockDim.x) {
         const long long ie = (long long)ix * e.ldz, ia = (long long)ix * w.ldz;
         const float p1 = e.halo_save[ix], pa = w.halo_save[ix];
@@ -280,6 +281,7 @@ __global__ void ae_couple(const ShotDev *__restrict__ E, const ShotDev *__restri
         na[ia] = a * w.tz[w.nz - 1] * w.tx[ix];
         const float a1 = b * e.tz[0] * e.tx[ix];
         n1[ie] = a1;
+        amax = fmaxf(amax, fabsf(a1));
         const int tt = e.nt - 1 - (it + 1);
         if ((flags & F_GRAD) && tt % C.sub == 0 && tt / C.sub != 0) {
             // density term at snapshot itf with the coupled next field, as the
@@ -310,6 +312,11 @@ __global__ void ae_couple(const ShotDev *__restrict__ E, const ShotDev *__restri
             else
                 *g2 = (float)((double)*g2 + wdt * (double)(a0 * (-f0 + fm0) + a1 * (-f1 + fm1)));
         }
+    }
+    if ((flags & F_AMAX) && (it + 1) % C.sub == 0) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        if ((threadIdx.x & 31) == 0 && amax > 0.f) atomicMax(e.snap_amax + (it + 1) / C.sub, __float_as_uint(amax));
     }
 }
 

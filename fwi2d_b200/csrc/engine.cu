@@ -174,6 +174,16 @@ __global__ void k_grad_flush(const ShotDev *__restrict__ shots, int ncompg, int 
     }
 }
 
+// 1/rho for the corrected division of the fused step (fused.cu div_by); 0 where
+// rho lies outside the range its proof covers
+__global__ void k_reciprocal(const float *__restrict__ rho, float *__restrict__ out, long long n)
+{
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const float r = rho[i];
+        out[i] = r >= 9.5367431640625e-7f && r <= 1048576.f ? 1.f / r : 0.f;
+    }
+}
+
 void launch_to_time_major(const float *in, float *out, int rows, int nt, cudaStream_t st)
 {
     dim3 g((nt + 31) / 32, (rows + 31) / 32), b(32, 8);
@@ -198,6 +208,7 @@ struct ModelState {
     float dx = 0, dz = 0;
     std::vector<float> host;   // converted model as given, [npar][nx][nz]
     DevBuf p0, p1, p2, c13, eps, fxx, lbis, gv2, gv3;
+    DevBuf irho, zclos;        // elastic kinds: 1/rho and the z-closure sums of mu (fused.cu)
     DevBuf stage;              // unpitched upload staging, [nx][nz]
     ModelDev dev() const
     {
@@ -214,6 +225,8 @@ struct ModelState {
         m.lbis = lbis.as<float>();
         m.gv2 = gv2.as<float>();
         m.gv3 = gv3.as<float>();
+        m.irho = irho.as<float>();
+        m.zclos = zclos.as<float>();
         return m;
     }
     const float *hp(int i) const { return host.data() + (size_t)i * nx * nz; }
@@ -253,6 +266,7 @@ struct ShotPlan {
     DevBuf d_inj_f, d_inj_f_off, d_inj_a, d_inj_a_off, d_ext_f, d_ext_f_off, d_ext_none_off;
     DevBuf d_mrow_f, d_mrow_a;
     DevBuf den, tz, tx, snap, amax, grad, gwt;
+    DevBuf xclos;                  // fused plans: x-closure sums of this shot's columns
     DevBuf gcomp;                  // compensated accumulation: running sum pair (hi, lo) of the gradient
     DevBuf r0, r1, ckpt;           // checkpoint-and-recompute: replay fields and checkpoints
     DevBuf halo;                   // acoustic-elastic: prev of the interface row [nx]
@@ -266,6 +280,7 @@ struct Plan {
     int tshape = 0, TZ = 32, TX = 16;   // tile shape of the tile kernel's units
     bool march = false;            // interior rows on the marching kernel
     bool framed = false;           // interior on the tile kernel's interior path, frame on the band kernels
+    bool fused = false;            // one launch per step over bands and interior (fused.cu)
     bool band_split = false;       // frame on the band kernels that split a cell's components over two warps
     int ishape = 0;                // framed: tile shape of the interior tiles
     int nth = 0, lx = 0;           // marching: threads (z window) per unit, rows per unit
@@ -428,8 +443,18 @@ static void upload_model_values(fwi2d_ctx *ctx, const float *model)
     // device copies straight from the caller's array (which may be pinned)
     up(M.p0, model);
     up(M.p1, model + nxz);
-    if (kind != KIND_ACOUSTIC) up(M.p2, model + 2 * nxz);
-    else M.p2.release();
+    if (kind != KIND_ACOUSTIC) {
+        up(M.p2, model + 2 * nxz);
+        M.irho.ensure(pitched * sizeof(float));
+        k_reciprocal<<<592, 256, 0, ctx->st>>>(M.p2.as<float>(), M.irho.as<float>(), (long long)pitched);
+        M.zclos.ensure((size_t)96 * nx * sizeof(float));
+        launch_closures(M.p1.as<float>(), M.zclos.as<float>(), nx, nx, nz, M.ldz, 1, ctx->st);
+        CK(cudaGetLastError());
+    } else {
+        M.p2.release();
+        M.irho.release();
+        M.zclos.release();
+    }
     // a live plan's graphs hold these addresses: an update keeps the buffers
     if (kind != KIND_VTI) {
         M.c13.release();
@@ -494,6 +519,7 @@ static const MarchShape kMarchShapes[] = {{224, 64}, {256, 64}, {192, 64}, {128,
 static const int kNumMarch = sizeof(kMarchShapes) / sizeof(kMarchShapes[0]);
 static const int kBandTile = 3;    // (TZ, TX) = (32, 8): band windows of 8 columns own 6
 static const int kBand = 6;
+static const int kFusedZ0 = 4;     // first row of the fused step's interior windows
 // Framed tile plans: the tile kernel's interior path on windows of one of
 // these tile shapes over the cells clear of all four boundary bands, and the
 // band kernels of the marching plans on the frame.  Shape indices follow the
@@ -519,9 +545,11 @@ static bool band_split_for(int nshots, int nz)
     return (long long)nshots * 2 * ((nz + 31) / 32) <= kSplitMaxBandWindows;
 }
 
-static int shape_count() { return elastic_tile_count() + kNumMarch + kNumFramed; }
+// The last shape is the fused step: one launch for bands and interior.
+static int fused_shape() { return elastic_tile_count() + kNumMarch + kNumFramed; }
+static int shape_count() { return fused_shape() + 1; }
 static bool is_march_shape(int s) { return s >= elastic_tile_count() && s < elastic_tile_count() + kNumMarch; }
-static bool is_framed_shape(int s) { return s >= elastic_tile_count() + kNumMarch && s < shape_count(); }
+static bool is_framed_shape(int s) { return s >= elastic_tile_count() + kNumMarch && s < fused_shape(); }
 static int framed_tile_shape(int s) { return kFramedShapes[s - elastic_tile_count() - kNumMarch]; }
 
 // Work units of one shot.  Units are numbered per shot: tiles first, then
@@ -529,6 +557,7 @@ static int framed_tile_shape(int s) { return kFramedShapes[s - elastic_tile_coun
 struct ShotUnits {
     bool march = false;            // marching plan: x-band tiles, bands, marching units
     bool framed = false;           // framed tile plan: x-band tiles, bands, interior tiles
+    bool fused = false;            // the same units for the fused step, whose interior windows are not flush
     int nx = 0, nz = 0;
     int TX = 0, TZ = 0, tiles_x = 0, tiles_z = 0;
     int lx = 0, nseg = 0, nwin = 0;
@@ -543,11 +572,13 @@ struct ShotUnits {
     int nunits() const { return (int)(tiles.size() + bands.size() + marches.size() + itiles.size()); }
     int unit_of(int x, int z) const
     {
-        if (!march && !framed) return owner_tile(z, nz, TZ) * tiles_x + owner_tile(x, nx, TX);
+        if (!march && !framed && !fused) return owner_tile(z, nz, TZ) * tiles_x + owner_tile(x, nx, TX);
         if (x < kBand) return owner_tile(z, nz, TZ);
         if (x >= nx - kBand) return tiles_z + owner_tile(z, nz, TZ);
         const int nt = (int)tiles.size();
         if (z < kBand || z >= nz - kBand) return nt + 2 * ((x - kBand) / zrows) + (z < kBand ? 0 : 1);
+        if (fused)
+            return nt + (int)bands.size() + ((z - kFusedZ0) / kFusedZ) * itiles_x + (x - kBand) / kFusedX;
         if (framed) {
             const int zi = z - kBand;
             const int kz = zi >= izlast ? itiles_z - 1 : zi / ITZ;
@@ -605,6 +636,7 @@ static bool shape_fits(int shape, int nx, int nz)
     }
     elastic_tile_shape(kBandTile, &tz, &tx);
     const bool frame = axis_fits(tz, nz) && nx >= 2 * tx && nx > 2 * kBand && nz >= 40;
+    if (shape == fused_shape()) return frame;
     if (is_framed_shape(shape)) {
         int itz, itx;
         elastic_tile_shape(framed_tile_shape(shape), &itz, &itx);
@@ -618,14 +650,16 @@ static ShotUnits make_units(int shape, int shot, int nx, int nz, bool band_split
     ShotUnits U;
     U.nx = nx;
     U.nz = nz;
-    U.zrows = zband_rows(band_split);
     const bool framed = is_framed_shape(shape);
     const bool march = is_march_shape(shape);
+    const bool fused = shape == fused_shape();
+    U.zrows = fused ? kFusedBand : zband_rows(band_split);
     U.march = march;
     U.framed = framed;
-    elastic_tile_shape(march || framed ? kBandTile : shape, &U.TZ, &U.TX);
+    U.fused = fused;
+    elastic_tile_shape(march || framed || fused ? kBandTile : shape, &U.TZ, &U.TX);
     U.tiles_z = (nz + U.TZ - 1) / U.TZ;
-    if (!march && !framed) {
+    if (!march && !framed && !fused) {
         U.tiles_x = (nx + U.TX - 1) / U.TX;
         for (int tzi = 0; tzi < U.tiles_z; tzi++)
             for (int txi = 0; txi < U.tiles_x; txi++) {
@@ -662,6 +696,22 @@ static ShotUnits make_units(int shape, int shot, int nx, int nz, bool band_split
             roff += b.xe - b.xb + 1;
             U.bands.push_back(b);
         }
+    if (fused) {
+        U.itiles_x = (nx - 2 * kBand + kFusedX - 1) / kFusedX;
+        for (int wz = kFusedZ0; wz < nz - kBand; wz += kFusedZ)
+            for (int txi = 0; txi < U.itiles_x; txi++) {
+                TileRef r;
+                r.shot = shot;
+                r.unit = (int)(U.tiles.size() + U.bands.size() + U.itiles.size());
+                r.wx0 = r.ox0 = kBand + txi * kFusedX;
+                r.ox1 = std::min(r.ox0 + kFusedX, nx - kBand);
+                r.wz0 = wz;
+                r.oz0 = std::max(wz, kBand);
+                r.oz1 = std::min(wz + kFusedZ, nz - kBand);
+                U.itiles.push_back(r);
+            }
+        return U;
+    }
     if (framed) {
         // interior windows, tiled as the tile plans tile a whole grid, offset by
         // the band; along z every window starts on an even row (the kernel's
@@ -931,6 +981,7 @@ static void shot_dev(const Plan &P, const ShotPlan &s, const ModelState &M, bool
     d.grad = s.grad.as<float>();
     d.gcomp = s.gcomp.as<float>();
     d.gwt = s.gwt.as<float>();
+    d.xclos = s.xclos.as<float>();
     d.halo_save = s.halo.as<float>();
     (void)P;
 }
@@ -1144,6 +1195,22 @@ static void plan_waves(Plan &P, bool one_wave)
     }
 }
 
+// x-closure sums of every shot of a fused plan from the resident model.
+static void build_xclos(fwi2d_ctx *ctx, Plan &P)
+{
+    if (!P.fused) return;
+    const ModelState &M = ctx->M;
+    const size_t n = (size_t)96 * M.ldz;
+    for (auto &S : P.shots) {
+        S->xclos.ensure((M.kind == KIND_VTI ? 2 : 1) * n * sizeof(float));
+        const long long o = (long long)S->x0 * M.ldz;
+        launch_closures(M.p1.as<float>() + o, S->xclos.as<float>(), M.nz, M.ldz, S->nx, 1, M.ldz, ctx->st);
+        if (M.kind == KIND_VTI)
+            launch_closures(M.fxx.as<float>() + o, S->xclos.as<float>() + n, M.nz, M.ldz, S->nx, 1, M.ldz, ctx->st);
+    }
+    CK(cudaGetLastError());
+}
+
 static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, const fwi2d_shot *shots)
 {
     ModelState &M = ctx->M;
@@ -1212,16 +1279,16 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
     // shape: the requested one, else the marching kernel where it has enough
     // units to fill the GPU, else the first tile shape that fits every shot
     auto shape_ok = [&](int i) {
-        if ((acoustic || ae) && !acoustic_shape_ok(i)) return false;
+        if ((acoustic || ae) && !acoustic_shape_ok(i) && !(ae && i == fused_shape())) return false;
         for (int s = 0; s < nshots; s++)
             if (!shape_fits(i, shots[s].nx, M.nz)) return false;
         return true;
     };
     int shape = p.tile_shape;
     if (shape < 0 || shape >= shape_count()) {
-        shape = -1;
+        shape = shape_ok(fused_shape()) ? fused_shape() : -1;
         const int m0 = elastic_tile_count();
-        if (!acoustic && !ae && shape_ok(m0)) {
+        if (shape < 0 && !acoustic && !ae && shape_ok(m0)) {
             long long units = 0;
             for (int s = 0; s < nshots; s++)
                 units += (long long)make_units(m0, s, shots[s].nx, M.nz, false).marches.size();
@@ -1235,7 +1302,8 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
     P->shape = shape;
     P->march = is_march_shape(shape);
     P->framed = is_framed_shape(shape);
-    P->tshape = P->march || P->framed ? kBandTile : shape;
+    P->fused = shape == fused_shape();
+    P->tshape = P->march || P->framed || P->fused ? kBandTile : shape;
     if (P->framed) P->ishape = framed_tile_shape(shape);
     P->band_split = (P->march || P->framed) && band_split_for(nshots, M.nz);
     elastic_tile_shape(P->tshape, &P->TZ, &P->TX);
@@ -1324,7 +1392,7 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
             W->nt = sh.nt;
             W->ncomp = 1;
             W->nr = sh.rcv_water.ntr;
-            const ShotUnits UW = make_units(shape, s, sh.nx, p.nza, P->band_split);
+            const ShotUnits UW = make_units(P->tshape, s, sh.nx, p.nza, P->band_split);
             int wa[2] = {0, 0}, wb[2] = {0, 0};
             build_inj(src_fluid ? sh.src_water : none, 1, wa, wb, UW, W->inj_f, W->inj_f_off, W->inj_f_roff);
             build_inj(sh.rcv_water, 1, wa, wb, UW, W->inj_a, W->inj_a_off, W->inj_a_roff);
@@ -1421,6 +1489,7 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
         P->shots.push_back(std::move(S));
     }
     P->have_snapshots = p.sub > 0;
+    build_xclos(ctx, *P);
     plan_waves(*P, p.checkpoint_every > 0);
     P->d_tiles.upload(P->tiles, ctx->st);
     P->d_march.upload(P->marches, ctx->st);
@@ -1516,10 +1585,11 @@ static void queue_timeout_check(fwi2d_ctx *ctx, Plan &P)
 // One time step of every shot.  Tile-only plans: one launch.  Marching
 // plans: the marching kernel on `st` while the tile kernel computes the
 // boundary bands on the context's side stream; the two branches write
-// disjoint cells and join before the next step.  Returns the number of
-// launches.
+// disjoint cells and join before the next step.  Fused plans: one launch,
+// with `chain` (the previous operation on `st` was this plan's previous step)
+// overlapping that one.  Returns the number of launches.
 static int launch_step(fwi2d_ctx *ctx, const Plan &P, const ShotDev *shots, const ModelDev &md, int it, int flags,
-                       cudaStream_t st, const Plan::Wave *wave = nullptr)
+                       cudaStream_t st, const Plan::Wave *wave = nullptr, bool chain = false)
 {
     // the units of the wave's shots (the kernels index the shot tables by the
     // units' own shot numbers)
@@ -1533,13 +1603,22 @@ static int launch_step(fwi2d_ctx *ctx, const Plan &P, const ShotDev *shots, cons
         const ShotDev *wshots = (adj ? P.d_wshots_a : P.d_wshots_f).as<ShotDev>();
         launch_ae_fluid_step(P.tshape, wshots, P.d_wtiles.as<TileRef>() + R.w0, R.w1 - R.w0, P.wdev(), P.Cw, it,
                              flags & STEP_EXTRACT, st);
-        launch_ae_elastic_step(P.tshape, shots, tiles, ntiles, md, P.C, it, flags, P.dtg, st);
+        if (P.fused)
+            CK(launch_fused_step(P.kind, shots, tiles, ntiles, P.d_bands.as<BandRef>() + R.b0, R.b1 - R.b0,
+                                 P.d_itiles.as<TileRef>() + R.i0, R.i1 - R.i0, md, P.C, it, flags, P.dtg, false, st));
+        else
+            launch_ae_elastic_step(P.tshape, shots, tiles, ntiles, md, P.C, it, flags, P.dtg, st);
         launch_ae_couple(shots + R.s0, wshots + R.s0, R.s1 - R.s0, P.nx_max, md, P.C, it, flags, P.dtg, P.Kw, P.val0,
                          adj ? -1 : 1, st);
         return 3;
     }
     if (P.kind == KIND_ACOUSTIC) {
         launch_acoustic_step(P.tshape, shots, tiles, ntiles, md, P.C, it, flags, P.dtg, st);
+        return 1;
+    }
+    if (P.fused) {
+        CK(launch_fused_step(P.kind, shots, tiles, ntiles, P.d_bands.as<BandRef>() + R.b0, R.b1 - R.b0,
+                             P.d_itiles.as<TileRef>() + R.i0, R.i1 - R.i0, md, P.C, it, flags, P.dtg, chain, st));
         return 1;
     }
     if (!P.march && !P.framed) {
@@ -1587,7 +1666,8 @@ static float time_forward_steps(fwi2d_ctx *ctx, int steps, int it0 = 0)
     CK(cudaEventCreate(&a));
     CK(cudaEventCreate(&b));
     CK(cudaEventRecord(a, ctx->st));
-    for (int it = it0; it < it0 + nsteps; it++) launch_step(ctx, P, shots, md, it, STEP_EXTRACT, ctx->st);
+    for (int it = it0; it < it0 + nsteps; it++)
+        launch_step(ctx, P, shots, md, it, STEP_EXTRACT, ctx->st, nullptr, it > it0);
     CK(cudaEventRecord(b, ctx->st));
     CK(cudaEventSynchronize(b));
     float ms = 0.f;
@@ -1646,7 +1726,7 @@ static float time_adjoint_steps(fwi2d_ctx *ctx, int steps)
     CK(cudaEventCreate(&a));
     CK(cudaEventCreate(&b));
     CK(cudaEventRecord(a, ctx->st));
-    for (int k = 0; k < steps; k++) launch_step(ctx, P, shots, md, it, STEP_GRAD, ctx->st);
+    for (int k = 0; k < steps; k++) launch_step(ctx, P, shots, md, it, STEP_GRAD, ctx->st, nullptr, k > 0);
     CK(cudaEventRecord(b, ctx->st));
     CK(cudaEventSynchronize(b));
     float ms = 0.f;
@@ -1874,12 +1954,14 @@ static long long capture_checkpointed(fwi2d_ctx *ctx, Plan &P, bool adj, cudaStr
         if (P.par.snapshot_precision != FWI2D_SNAP_FP32) flags |= STEP_AMAX;
         int kn = 1;
         for (int it = 0; it < nt - 1; it++) {
+            bool chain = it > 0;
             if (kn < nseg && it == P.cuts[kn] - 1) {
                 launch_checkpoint(shots, nshots, ncomp, kn - 1, false, cst);
                 n++;
                 kn++;
+                chain = false;
             }
-            n += launch_step(ctx, P, shots, md, it, flags, cst);
+            n += launch_step(ctx, P, shots, md, it, flags, cst, nullptr, chain);
         }
         launch_finalize(shots, nshots, P.C, ncomp, STEP_EXTRACT, cst);
         return n + 1;
@@ -1903,14 +1985,17 @@ static long long capture_checkpointed(fwi2d_ctx *ctx, Plan &P, bool adj, cudaStr
         }
         n++;
         const int t0 = k == 0 ? 0 : P.cuts[k] - 1, t1 = P.cuts[k + 1];
-        for (int it = t0; it < t1; it++) n += launch_step(ctx, P, rs, md, it, STEP_STORE, cst);
+        for (int it = t0; it < t1; it++) n += launch_step(ctx, P, rs, md, it, STEP_STORE, cst, nullptr, it > t0);
         launch_finalize(rs, nshots, P.C, ncomp, STEP_STORE, cst, t1);
         n++;
         const int lo = k == nseg - 1 ? 0 : nt - 1 - P.cuts[k + 1] + a;
         const int hi = k == 0 ? nt - 2 : nt - 2 - P.cuts[k] + a;
+        bool chain = false;
         for (int it = lo; it <= hi; it++) {
-            n += launch_step(ctx, P, as, md, it, STEP_GRAD, cst);
-            n += grad_flush(P, P.all, ++nadj, false, cst);
+            n += launch_step(ctx, P, as, md, it, STEP_GRAD, cst, nullptr, chain);
+            const int flushed = grad_flush(P, P.all, ++nadj, false, cst);
+            n += flushed;
+            chain = flushed == 0;
         }
         last_adj = as;
     }
@@ -1978,9 +2063,12 @@ static void capture(fwi2d_ctx *ctx, Plan &P, int mode, int w = 0)
     if (P.ckpt > 0 && (store || adj)) {
         n += capture_checkpointed(ctx, P, adj, cst);
     } else {
+        bool chain = false;
         for (int it = 0; it < R.nt_max - 1; it++) {
-            n += launch_step(ctx, P, shots, md, it, flags, cst, &R);
-            if (adj) n += grad_flush(P, R, it + 1, false, cst);
+            n += launch_step(ctx, P, shots, md, it, flags, cst, &R, chain);
+            const int flushed = adj ? grad_flush(P, R, it + 1, false, cst) : 0;
+            n += flushed;
+            chain = flushed == 0;
         }
         if (!adj) {
             launch_finalize(shots + R.s0, nshots, P.C, ncomp, STEP_EXTRACT | (store ? STEP_STORE : 0), cst);
@@ -2325,6 +2413,7 @@ static void update_model(fwi2d_ctx *ctx, const float *model)
         }
         S->den.upload(den, ctx->st);
     }
+    build_xclos(ctx, P);
     init_factors(M, P);
     upload_init_cells(P, ctx->st);
     CK(cudaStreamSynchronize(ctx->st));
@@ -2644,6 +2733,7 @@ int fwi2d_ctx_create(int device, fwi2d_ctx **out)
     c->st = c->own;
     const SbpTables &t = sbp_tables();
     upload_sbp_tables(&t.b1[0][0], &t.b2[0][0][0], t.c2, t.c1, t.sc, t.hc);
+    upload_fused_tables(&t.b1[0][0], &t.b2[0][0][0], t.c2, t.c1, t.sc);
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
     *out = c.release();
@@ -2755,7 +2845,7 @@ int fwi2d_snapshot(fwi2d_ctx *ctx, int shot, int slot, float *out)
     if (prec != FWI2D_SNAP_FP32) {
         float m;
         std::memcpy(&m, &amax, 4);
-        if (m > 0.f) inv = 1.f / std::ldexp(1.f, 14 - (std::ilogb(m) + 1));
+        if (m > 0.f) inv = 1.f / std::ldexp(1.f, std::min(14 - (std::ilogb(m) + 1), 126));
     }
     for (int c = 0; c < S.ncomp; c++)
         for (int ix = 0; ix < S.nx; ix++)
@@ -2867,6 +2957,10 @@ int fwi2d_tile_shape(int index, int *tz, int *tx)
     REQ(index >= 0 && index < shape_count() && tz && tx, "no such tile shape");
     if (index < elastic_tile_count()) elastic_tile_shape(index, tz, tx);
     else if (is_framed_shape(index)) elastic_tile_shape(framed_tile_shape(index), tz, tx);
+    else if (index == fused_shape()) {
+        *tz = kFusedZ;
+        *tx = kFusedX;
+    }
     else {
         *tz = kMarchShapes[index - elastic_tile_count()].nth;
         *tx = kMarchShapes[index - elastic_tile_count()].lx;

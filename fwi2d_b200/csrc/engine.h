@@ -72,6 +72,7 @@ struct ShotDev {
     float *gcomp;         // compensated accumulation: running sum pair hi [3 or 2][nx][ldz], then lo; or nullptr
     float *halo_save;     // interface scratch (acoustic-elastic) or nullptr
     const float *gwt;     // gradient time-damping weight per snapshot index
+    const float *xclos;   // fused plans: x-closure sums of mu [2 sides][6][8][ldz]; VTI: then those of fxx
     float *ckpt;          // checkpoints [k][2][ncomp][nx][ldz] (checkpoint-and-recompute) or nullptr
 };
 
@@ -83,6 +84,8 @@ struct ModelDev {
     const float *fxx;            // VTI: (1+2eps)*2mu ; elastic: unused
     const float *lbis;           // VTI: (1+2eps)*lambda
     const float *gv2, *gv3;      // VTI gradient: dC13/dlambda, dC13/dmu
+    const float *irho;           // elastic kinds: 1/rho rounded, 0 where rho lies outside [2^-20, 2^20]
+    const float *zclos;          // z-closure sums of mu [top, bottom][6][8][nx]
 };
 
 // Scalars of one propagation, each computed on the host exactly as the

@@ -24,6 +24,17 @@ void launch_elastic_step(int shape, bool vti, const ShotDev *shots, const TileRe
 bool march_threads_ok(int nth);
 void launch_elastic_march(bool vti, const ShotDev *shots, const MarchRef *units, int nunits, int nth,
                           const ModelDev &M, const StepConst &C, int it, int flags, float dtg, cudaStream_t st);
+// fused.cu: one launch per step over x-band, z-band and interior units; chain:
+// the launch may start beside the previous launch of the stream, which must be
+// a fused step too.  Interior windows of kFusedZ x kFusedX cells start at
+// z = 4 + kFusedZ k (rows of 16-byte multiples) and x = 6 + kFusedX k.
+constexpr int kFusedZ = 32, kFusedX = 16, kFusedBand = 32;
+void upload_fused_tables(const float *b1, const float *b2, const float *c2, const float *c1, const float *sc);
+cudaError_t launch_fused_step(int kind, const ShotDev *shots, const TileRef *xb, int nxb, const BandRef *zb, int nzb,
+                              const TileRef *in, int nin, const ModelDev &M, const StepConst &C, int it, int flags,
+                              float dtg, bool chain, cudaStream_t st);
+// closure sums of the six rows next to both ends of an axis of n samples (stride sn) on `lines` lines (stride sl)
+void launch_closures(const float *f, float *out, int lines, int ld, int n, long long sl, long long sn, cudaStream_t st);
 // top / bottom band kernel (rows clear of the x bands), zband_rows(split)
 // rows per unit; split as for the x bands
 int zband_rows(bool split);

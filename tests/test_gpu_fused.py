@@ -1,0 +1,109 @@
+"""The fused step (one launch per step over band and interior units, chained by
+programmatic dependent launch) against the oracle and the tile kernel.
+
+Grids sit at the edges of its units: the smallest it takes (40 rows, 16
+columns), one cell either side of a full interior window (32 x 16 from row 4
+and column 6), partial last windows and band units, z windows that end flush.
+Every result restates the reference's FP32 operations, so traces, snapshots
+and gradients must equal the oracle's bit for bit.
+"""
+import numpy as np
+import pytest
+
+import oracle as O
+import fwi2d_b200 as F
+from tests import cases as K
+from tests.test_gpu_parity import run_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+def fused_shape():
+    return F.load().fwi2d_tile_shape_count() - 1
+
+
+@pytest.mark.parametrize("kind,mt,bc", [
+    (O.KIND_ELASTIC, 0, (1, 2, 2, 2)),
+    (O.KIND_ELASTIC, 1, (2, 2, 2, 2)),
+    (O.KIND_ELASTIC, 0, (1, 1, 1, 1)),
+    (O.KIND_VTI, 0, (1, 2, 2, 2)),
+    (O.KIND_VTI, 1, (2, 1, 2, 1)),
+])
+@pytest.mark.parametrize("grid", [(16, 40), (17, 41), (28, 42), (29, 43), (44, 74), (45, 75), (61, 107), (120, 200)])
+def test_fused_vs_oracle(kind, mt, bc, grid):
+    nx, nz = grid
+    d, nt = 0.01, 150
+    mc = K.converted(kind, K.model_case(kind, nx, nz, d, seed=3))
+    sl, rl = K.geometry(nx, nz, d, nr=14)
+    # sources and receivers in the bands, on their seams and in the interior windows
+    sl = (np.array([0.05, 0.3 * nx * d, (nx - 7.2) * d], np.float32), np.array([0.02, 0.055, 0.36], np.float32))
+    rz = np.array([0.02, 0.045, 0.055, 0.065, 0.2, 0.35, (nz - 7.3) * d, (nz - 6.2) * d, (nz - 2.4) * d], np.float32)
+    rl = (np.linspace(1.2 * d, (nx - 2.3) * d, 27).astype(np.float32), np.tile(rz, 3))
+    pd = K.par_dict(nt=nt, dt=1e-3, bc=bc, mt=mt, taper=(0, 6, 5, 6))
+    ns = len(sl[0])
+    src = np.repeat(K.sources(3 if mt else 2, nt, 1e-3, f0=25.0, t0=0.03), ns, axis=1)
+    port = O.Port(32)
+    par = O.make_par(**pd, ns=ns, nr=len(rl[0]))
+    rcv_o, full_o = K.oracle_forward(port, kind, mc, src, par, nx, nz, d, sl, rl, mt=mt)
+    adj = np.ascontiguousarray(rcv_o[:, :, ::-1])
+    g_o = np.zeros((5 if kind == O.KIND_VTI else 3, nx, nz), np.float32)
+    srcb = np.zeros((3 if mt else 2, ns, nt), np.float32)
+    port.propagate(kind, 1, mc, adj, srcb, par, nx, nz, d, d, 0.0, 0.0, rl, sl, inj_type=0, full=full_o, grad=g_o)
+    rcv_g, g_g, snaps = run_gpu(kind, mc, src, pd, nx, nz, d, sl, rl, adj_src=adj, mt=mt, shape=fused_shape())
+    step = max(1, nt // 5)
+    want = np.stack([full_o[k] for k in range(0, nt, step)])
+    print("fused kind %d mt %d bc %s grid %s: traces %.4f snapshots %.4f gradient %.4f equal" % (
+        kind, mt, bc, grid, np.mean(rcv_g == rcv_o), np.mean(snaps == want), np.mean(g_g == g_o[:3])))
+    assert np.abs(g_o).max() > 0
+    assert np.array_equal(rcv_g, rcv_o)
+    assert np.array_equal(snaps, want)
+    assert np.array_equal(g_g, g_o[:3])
+
+
+def _gradient(kind, shape, prec, every, compensated, nx=150, nz=75, nt=97):
+    d = 0.01
+    base = O.KIND_ELASTIC if kind == O.KIND_AE else kind
+    mc = K.converted(base, K.model_case(base, nx, nz, d, seed=5))
+    rng = np.random.default_rng(9)
+    oz = 0.0
+    pd = K.par_dict(nt=nt, dt=1e-3, taper=(0, 6, 6, 6))
+    if kind == O.KIND_AE:
+        pd.update(nza=20, acoustic_source=1)
+        oz = 19 * d
+    shots, src, obs = [], [], []
+    for x0, w, n in ((0, 150, nt), (3, 61, nt), (70, 77, nt)) if every else ((0, 150, nt), (3, 61, nt - 31), (70, 77, nt - 10)):
+        rx = ((x0 + np.linspace(2.2, w - 3.3, 11)) * d).astype(np.float32)
+        sx, sz = [(x0 + 0.5 * w) * d], [0.06]
+        rz = np.full(11, 0.04, np.float32)
+        kw = {}
+        if kind == O.KIND_AE:
+            kw = dict(water_src_x=sx, water_src_z=[0.05], water_rcv_x=rx, water_rcv_z=np.full(11, 0.03, np.float32))
+        shots.append(F.ShotSpec(x0, w, n, sx, [sz[0] + oz], rx, rz + np.float32(oz), **kw))
+        ns = 1 if kind == O.KIND_AE else 2
+        src.append(K.sources(ns, n, 1e-3, f0=25.0, t0=0.03))
+        obs.append(rng.normal(size=(3 if kind == O.KIND_AE else 2, 11, n)).astype(np.float32))
+    P = F.Propagator(0)
+    P.set_model(kind, mc, d, d, 0.0, oz)
+    P.set_shots(F.make_params(**pd, tile_shape=shape, snapshot_precision=prec, checkpoint_every=every,
+                              compensated=compensated), shots)
+    out = [P.fwi_gradient(mc, src, obs) for _ in range(2)]
+    rcv = P.forward(src, store=False)
+    P.close()
+    return out, rcv
+
+
+@pytest.mark.parametrize("kind", [O.KIND_ELASTIC, O.KIND_VTI, O.KIND_AE])
+@pytest.mark.parametrize("prec,every,compensated", [(0, 0, 0), (2, 0, 1), (1, 20, 0), (0, 7, 1)])
+def test_fused_plan_equals_tile_plan(kind, prec, every, compensated):
+    """Uneven windows and records, 16-bit snapshots, replayed segments and
+    compensated accumulation: the chain of overlapping launches is broken by
+    other kernels there, and must still see every earlier write."""
+    if kind == O.KIND_AE and every:
+        pytest.skip("checkpoint-and-recompute is not available for the acoustic-elastic propagator")
+    a, ra = _gradient(kind, fused_shape(), prec, every, compensated)
+    b, rb = _gradient(kind, 3, prec, every, compensated)
+    for (ga, fa), (gb, fb) in zip(a, b):
+        assert np.abs(gb).max() > 0
+        assert fa == fb and np.array_equal(ga, gb)
+    for x, y in zip(ra, rb):
+        assert np.array_equal(x, y)

@@ -174,7 +174,7 @@ __global__ void k_grad_flush(const ShotDev *__restrict__ shots, int ncompg, int 
     }
 }
 
-// 1/rho for the corrected division of the fused step (fused.cu div_by); 0 where
+// 1/rho for the corrected division of the fused step (fused.cu div_pairs); 0 where
 // rho lies outside the range its proof covers
 __global__ void k_reciprocal(const float *__restrict__ rho, float *__restrict__ out, long long n)
 {
@@ -280,7 +280,7 @@ struct Plan {
     int tshape = 0, TZ = 32, TX = 16;   // tile shape of the tile kernel's units
     bool march = false;            // interior rows on the marching kernel
     bool framed = false;           // interior on the tile kernel's interior path, frame on the band kernels
-    bool fused = false;            // one launch per step over bands and interior (fused.cu)
+    bool fused = false;            // the whole time loop in one launch over bands and interior (fused.cu)
     bool band_split = false;       // frame on the band kernels that split a cell's components over two warps
     int ishape = 0;                // framed: tile shape of the interior tiles
     int nth = 0, lx = 0;           // marching: threads (z window) per unit, rows per unit
@@ -364,6 +364,7 @@ struct Plan {
     // device status word of the bounded waits (launch_take_timeout after each
     // pass) and its pinned host copy, read after the pass has finished
     DevBuf d_status;
+    DevBuf d_count;                // fused plans: arrivals of the launch's CTAs
     int *h_status = nullptr;
     ~Plan()
     {
@@ -545,7 +546,7 @@ static bool band_split_for(int nshots, int nz)
     return (long long)nshots * 2 * ((nz + 31) / 32) <= kSplitMaxBandWindows;
 }
 
-// The last shape is the fused step: one launch for bands and interior.
+// The last shape is the fused time loop: bands and interior, all steps, in one launch.
 static int fused_shape() { return elastic_tile_count() + kNumMarch + kNumFramed; }
 static int shape_count() { return fused_shape() + 1; }
 static bool is_march_shape(int s) { return s >= elastic_tile_count() && s < elastic_tile_count() + kNumMarch; }
@@ -557,7 +558,9 @@ static int framed_tile_shape(int s) { return kFramedShapes[s - elastic_tile_coun
 struct ShotUnits {
     bool march = false;            // marching plan: x-band tiles, bands, marching units
     bool framed = false;           // framed tile plan: x-band tiles, bands, interior tiles
-    bool fused = false;            // the same units for the fused step, whose interior windows are not flush
+    bool fused = false;            // fused plan: band units (nxband x bands first) and interior windows
+    int nxband = 0;
+    std::vector<int> xzo;          // fused: z starts of the x-band units, plus nz
     int nx = 0, nz = 0;
     int TX = 0, TZ = 0, tiles_x = 0, tiles_z = 0;
     int lx = 0, nseg = 0, nwin = 0;
@@ -573,10 +576,14 @@ struct ShotUnits {
     int unit_of(int x, int z) const
     {
         if (!march && !framed && !fused) return owner_tile(z, nz, TZ) * tiles_x + owner_tile(x, nx, TX);
+        if (fused && (x < kBand || x >= nx - kBand)) {
+            const int k = (int)(std::upper_bound(xzo.begin(), xzo.end(), z) - xzo.begin()) - 1;
+            return x < kBand ? k : k + nxband / 2;
+        }
         if (x < kBand) return owner_tile(z, nz, TZ);
         if (x >= nx - kBand) return tiles_z + owner_tile(z, nz, TZ);
         const int nt = (int)tiles.size();
-        if (z < kBand || z >= nz - kBand) return nt + 2 * ((x - kBand) / zrows) + (z < kBand ? 0 : 1);
+        if (z < kBand || z >= nz - kBand) return nt + nxband + 2 * ((x - kBand) / zrows) + (z < kBand ? 0 : 1);
         if (fused)
             return nt + (int)bands.size() + ((z - kFusedZ0) / kFusedZ) * itiles_x + (x - kBand) / kFusedX;
         if (framed) {
@@ -592,7 +599,7 @@ struct ShotUnits {
     // (band and marching units)
     bool row_sorted(int u) const
     {
-        return u >= (int)tiles.size() && u < (int)(tiles.size() + bands.size() + marches.size());
+        return u >= (int)tiles.size() + nxband && u < (int)(tiles.size() + bands.size() + marches.size());
     }
     struct RowUnit {
         int unit, xb, xe, roff;
@@ -600,7 +607,8 @@ struct ShotUnits {
     std::vector<RowUnit> row_units() const
     {
         std::vector<RowUnit> r;
-        for (const BandRef &b : bands) r.push_back({b.unit, b.xb, b.xe, b.roff});
+        for (const BandRef &b : bands)
+            if (b.side < 2) r.push_back({b.unit, b.xb, b.xe, b.roff});
         for (const MarchRef &m : marches) r.push_back({m.unit, m.xb, m.xe, m.roff});
         return r;
     }
@@ -672,7 +680,24 @@ static ShotUnits make_units(int shape, int shot, int nx, int nz, bool band_split
             }
         return U;
     }
-    for (int side = 0; side < 2; side++)
+    if (fused) {
+        // x bands in equal parts, so that the last ones hold the closure's samples of the corners
+        const int nw = (nz + kFusedBand - 1) / kFusedBand;
+        for (int k = 0; k <= nw; k++) U.xzo.push_back((int)((long long)k * nz / nw));
+        U.nxband = 2 * nw;
+        for (int side = 2; side < 4; side++)
+            for (int k = 0; k < nw; k++) {
+                BandRef b;
+                b.shot = shot;
+                b.unit = (int)U.bands.size();
+                b.xb = U.xzo[k];
+                b.xe = U.xzo[k + 1];
+                b.side = side;
+                b.roff = 0;
+                U.bands.push_back(b);
+            }
+    }
+    for (int side = 0; side < 2 && !fused; side++)
         for (int tzi = 0; tzi < U.tiles_z; tzi++) {
             TileRef r;
             r.shot = shot;
@@ -908,6 +933,11 @@ static StepConst make_const(const fwi2d_params &p, float dx, float dz)
     const float h0 = sbp_tables().h0;
     C.dt = p.dt;
     C.dt2 = p.dt * p.dt;
+    C.idt64 = 1.0 / (double)p.dt;
+    C.idx64 = 1.0 / (double)dx;
+    C.idz64 = 1.0 / (double)dz;
+    C.id2x64 = 1.0 / (double)(dx * dx);
+    C.id2z64 = 1.0 / (double)(dz * dz);
     C.dx = dx;
     C.dz = dz;
     C.d2x = dx * dx;
@@ -1549,6 +1579,7 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
     upload_init_cells(*P, ctx->st);
     P->d_grad_full.alloc((size_t)P->ncompg * M.nx * M.ldz * sizeof(float));
     P->d_status.alloc(sizeof(int));
+    if (P->fused) P->d_count.alloc(sizeof(unsigned));
     CK(cudaMemsetAsync(P->d_status.p, 0, sizeof(int), ctx->st));
     CK(cudaMallocHost((void **)&P->h_status, sizeof(int)));
     *P->h_status = 0;
@@ -1569,7 +1600,9 @@ static void check_timeout(fwi2d_ctx *ctx)
     CK(cudaMemsetAsync(P.d_status.p, 0, sizeof(int), ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     P.snapshots_valid = false;
-    throw Error(FWI2D_ERR_TIMEOUT, "a bounded device wait of the marching kernel reached its limit (row " +
+    throw Error(FWI2D_ERR_TIMEOUT, std::string("a bounded device wait of the ") +
+                                       (P.fused ? "fused time loop reached its limit (step " :
+                                                  "marching kernel reached its limit (row ") +
                                        std::to_string(v - 1) + "); the results of this pass are not trusted");
 }
 
@@ -1585,11 +1618,10 @@ static void queue_timeout_check(fwi2d_ctx *ctx, Plan &P)
 // One time step of every shot.  Tile-only plans: one launch.  Marching
 // plans: the marching kernel on `st` while the tile kernel computes the
 // boundary bands on the context's side stream; the two branches write
-// disjoint cells and join before the next step.  Fused plans: one launch,
-// with `chain` (the previous operation on `st` was this plan's previous step)
-// overlapping that one.  Returns the number of launches.
+// disjoint cells and join before the next step.  Returns the number of
+// launches.
 static int launch_step(fwi2d_ctx *ctx, const Plan &P, const ShotDev *shots, const ModelDev &md, int it, int flags,
-                       cudaStream_t st, const Plan::Wave *wave = nullptr, bool chain = false)
+                       cudaStream_t st, const Plan::Wave *wave = nullptr)
 {
     // the units of the wave's shots (the kernels index the shot tables by the
     // units' own shot numbers)
@@ -1604,8 +1636,9 @@ static int launch_step(fwi2d_ctx *ctx, const Plan &P, const ShotDev *shots, cons
         launch_ae_fluid_step(P.tshape, wshots, P.d_wtiles.as<TileRef>() + R.w0, R.w1 - R.w0, P.wdev(), P.Cw, it,
                              flags & STEP_EXTRACT, st);
         if (P.fused)
-            CK(launch_fused_step(P.kind, shots, tiles, ntiles, P.d_bands.as<BandRef>() + R.b0, R.b1 - R.b0,
-                                 P.d_itiles.as<TileRef>() + R.i0, R.i1 - R.i0, md, P.C, it, flags, P.dtg, false, st));
+            CK(launch_fused(P.kind, shots, P.d_bands.as<BandRef>() + R.b0, R.b1 - R.b0,
+                            P.d_itiles.as<TileRef>() + R.i0, R.i1 - R.i0, md, P.C, it, it + 1, flags, P.dtg,
+                            P.d_count.as<unsigned>(), P.d_status.as<int>(), st));
         else
             launch_ae_elastic_step(P.tshape, shots, tiles, ntiles, md, P.C, it, flags, P.dtg, st);
         launch_ae_couple(shots + R.s0, wshots + R.s0, R.s1 - R.s0, P.nx_max, md, P.C, it, flags, P.dtg, P.Kw, P.val0,
@@ -1614,11 +1647,6 @@ static int launch_step(fwi2d_ctx *ctx, const Plan &P, const ShotDev *shots, cons
     }
     if (P.kind == KIND_ACOUSTIC) {
         launch_acoustic_step(P.tshape, shots, tiles, ntiles, md, P.C, it, flags, P.dtg, st);
-        return 1;
-    }
-    if (P.fused) {
-        CK(launch_fused_step(P.kind, shots, tiles, ntiles, P.d_bands.as<BandRef>() + R.b0, R.b1 - R.b0,
-                             P.d_itiles.as<TileRef>() + R.i0, R.i1 - R.i0, md, P.C, it, flags, P.dtg, chain, st));
         return 1;
     }
     if (!P.march && !P.framed) {
@@ -1647,6 +1675,24 @@ static int launch_step(fwi2d_ctx *ctx, const Plan &P, const ShotDev *shots, cons
     return n;
 }
 
+// The time steps [it0, it1) of every shot: step by step, or in one launch of
+// the fused time loop.  Returns the number of launches.
+static long long launch_steps(fwi2d_ctx *ctx, const Plan &P, const ShotDev *shots, const ModelDev &md, int it0, int it1,
+                              int flags, cudaStream_t st, const Plan::Wave *wave = nullptr)
+{
+    if (it1 <= it0) return 0;
+    if (P.fused && !P.ae) {
+        const Plan::Wave &R = wave ? *wave : P.all;
+        CK(launch_fused(P.kind, shots, P.d_bands.as<BandRef>() + R.b0, R.b1 - R.b0, P.d_itiles.as<TileRef>() + R.i0,
+                        R.i1 - R.i0, md, P.C, it0, it1, flags, P.dtg, P.d_count.as<unsigned>(), P.d_status.as<int>(),
+                        st));
+        return 1;
+    }
+    long long n = 0;
+    for (int it = it0; it < it1; it++) n += launch_step(ctx, P, shots, md, it, flags, st, wave);
+    return n;
+}
+
 // Time `steps` forward steps of the current plan from launch it0 (fields
 // zeroed, no output), in milliseconds per step.  Shots whose records end
 // before a launch return from it, as in a full pass.
@@ -1666,8 +1712,7 @@ static float time_forward_steps(fwi2d_ctx *ctx, int steps, int it0 = 0)
     CK(cudaEventCreate(&a));
     CK(cudaEventCreate(&b));
     CK(cudaEventRecord(a, ctx->st));
-    for (int it = it0; it < it0 + nsteps; it++)
-        launch_step(ctx, P, shots, md, it, STEP_EXTRACT, ctx->st, nullptr, it > it0);
+    for (int it = it0; it < it0 + nsteps; it++) launch_step(ctx, P, shots, md, it, STEP_EXTRACT, ctx->st);
     CK(cudaEventRecord(b, ctx->st));
     CK(cudaEventSynchronize(b));
     float ms = 0.f;
@@ -1726,7 +1771,7 @@ static float time_adjoint_steps(fwi2d_ctx *ctx, int steps)
     CK(cudaEventCreate(&a));
     CK(cudaEventCreate(&b));
     CK(cudaEventRecord(a, ctx->st));
-    for (int k = 0; k < steps; k++) launch_step(ctx, P, shots, md, it, STEP_GRAD, ctx->st, nullptr, k > 0);
+    for (int k = 0; k < steps; k++) launch_step(ctx, P, shots, md, it, STEP_GRAD, ctx->st);
     CK(cudaEventRecord(b, ctx->st));
     CK(cudaEventSynchronize(b));
     float ms = 0.f;
@@ -1825,7 +1870,10 @@ static void set_shots(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, const
 {
     REQ(par != nullptr && shots != nullptr && nshots > 0, "no shots");
     fwi2d_params p = *par;
-    if (p.tile_shape < 0 && ctx->M.kind >= 0) {
+    bool fused = ctx->M.kind == KIND_ELASTIC || ctx->M.kind == KIND_VTI;
+    for (int i = 0; i < nshots && fused; i++) fused = shape_fits(fused_shape(), shots[i].nx, ctx->M.nz);
+    // the fused time loop is the fastest shape wherever it fits: nothing to time
+    if (p.tile_shape < 0 && ctx->M.kind >= 0 && !fused) {
         static std::vector<std::pair<std::string, int>> cache;
         const bool grad = p.sub > 0;
         std::string key = tune_build_key(ctx->device) + "/" + std::to_string(ctx->M.kind) + "/" +
@@ -1932,6 +1980,23 @@ static int grad_flush(const Plan &P, const Plan::Wave &R, int count, bool final,
     return 1;
 }
 
+// The adjoint steps [it0, it1), with the window flushes of compensated
+// accumulation; done: adjoint launches of the pass before these.
+static long long adjoint_steps(fwi2d_ctx *ctx, const Plan &P, const ShotDev *shots, const ModelDev &md, int it0, int it1,
+                               int done, cudaStream_t st, const Plan::Wave &R)
+{
+    if (!P.par.compensated) return launch_steps(ctx, P, shots, md, it0, it1, STEP_GRAD, st, &R);
+    long long n = 0;
+    for (int it = it0; it < it1;) {
+        const int to = std::min(it1, it + kCompWindow - done % kCompWindow);
+        n += launch_steps(ctx, P, shots, md, it, to, STEP_GRAD, st, &R);
+        done += to - it;
+        n += grad_flush(P, R, done, false, st);
+        it = to;
+    }
+    return n;
+}
+
 // Checkpoint-and-recompute time loops (all shots share nt, sub = 1).
 // Forward: receivers and 16-bit snapshot scales as usual, no snapshot store;
 // before launch cuts[k] - 1 (k >= 1) both field buffers of every shot are
@@ -1952,16 +2017,15 @@ static long long capture_checkpointed(fwi2d_ctx *ctx, Plan &P, bool adj, cudaStr
         const ShotDev *shots = P.d_shots_f.as<ShotDev>();
         int flags = STEP_EXTRACT;
         if (P.par.snapshot_precision != FWI2D_SNAP_FP32) flags |= STEP_AMAX;
-        int kn = 1;
-        for (int it = 0; it < nt - 1; it++) {
-            bool chain = it > 0;
-            if (kn < nseg && it == P.cuts[kn] - 1) {
+        int from = 0;
+        for (int kn = 1; kn <= nseg; kn++) {
+            const int to = kn < nseg ? P.cuts[kn] - 1 : nt - 1;
+            n += launch_steps(ctx, P, shots, md, from, to, flags, cst);
+            if (kn < nseg) {
                 launch_checkpoint(shots, nshots, ncomp, kn - 1, false, cst);
                 n++;
-                kn++;
-                chain = false;
             }
-            n += launch_step(ctx, P, shots, md, it, flags, cst, nullptr, chain);
+            from = to;
         }
         launch_finalize(shots, nshots, P.C, ncomp, STEP_EXTRACT, cst);
         return n + 1;
@@ -1985,18 +2049,13 @@ static long long capture_checkpointed(fwi2d_ctx *ctx, Plan &P, bool adj, cudaStr
         }
         n++;
         const int t0 = k == 0 ? 0 : P.cuts[k] - 1, t1 = P.cuts[k + 1];
-        for (int it = t0; it < t1; it++) n += launch_step(ctx, P, rs, md, it, STEP_STORE, cst, nullptr, it > t0);
+        n += launch_steps(ctx, P, rs, md, t0, t1, STEP_STORE, cst);
         launch_finalize(rs, nshots, P.C, ncomp, STEP_STORE, cst, t1);
         n++;
         const int lo = k == nseg - 1 ? 0 : nt - 1 - P.cuts[k + 1] + a;
         const int hi = k == 0 ? nt - 2 : nt - 2 - P.cuts[k] + a;
-        bool chain = false;
-        for (int it = lo; it <= hi; it++) {
-            n += launch_step(ctx, P, as, md, it, STEP_GRAD, cst, nullptr, chain);
-            const int flushed = grad_flush(P, P.all, ++nadj, false, cst);
-            n += flushed;
-            chain = flushed == 0;
-        }
+        n += adjoint_steps(ctx, P, as, md, lo, hi + 1, nadj, cst, P.all);
+        nadj += hi + 1 - lo;
         last_adj = as;
     }
     if (P.kind == KIND_ACOUSTIC) {
@@ -2063,13 +2122,8 @@ static void capture(fwi2d_ctx *ctx, Plan &P, int mode, int w = 0)
     if (P.ckpt > 0 && (store || adj)) {
         n += capture_checkpointed(ctx, P, adj, cst);
     } else {
-        bool chain = false;
-        for (int it = 0; it < R.nt_max - 1; it++) {
-            n += launch_step(ctx, P, shots, md, it, flags, cst, &R, chain);
-            const int flushed = adj ? grad_flush(P, R, it + 1, false, cst) : 0;
-            n += flushed;
-            chain = flushed == 0;
-        }
+        if (adj) n += adjoint_steps(ctx, P, shots, md, 0, R.nt_max - 1, 0, cst, R);
+        else n += launch_steps(ctx, P, shots, md, 0, R.nt_max - 1, flags, cst, &R);
         if (!adj) {
             launch_finalize(shots + R.s0, nshots, P.C, ncomp, STEP_EXTRACT | (store ? STEP_STORE : 0), cst);
             n++;
@@ -2881,6 +2935,7 @@ int fwi2d_plan_info(fwi2d_ctx *ctx, long long *lf, long long *la, int *shape, lo
     REQ(ctx, "null context");
     Plan &P = need_plan(ctx);
     const long long per = (P.march || P.framed || P.ae) ? 3 : 1;
+    const bool loop = P.fused && !P.ae;   // one launch per run of steps
     const long long nseg = P.ckpt > 0 ? (long long)P.cuts.size() - 1 : 0;
     const long long acf = P.kind == KIND_ACOUSTIC ? 1 : 0;
     // per wave -- forward: init, steps, last sample (+ checkpoint copies);
@@ -2890,9 +2945,13 @@ int fwi2d_plan_info(fwi2d_ctx *ctx, long long *lf, long long *la, int *shape, lo
     long long f = 0, a = 0;
     for (const auto &W : P.waves) {
         const long long steps = W.nt_max - 1;
-        f += steps * per + 2 + (P.ae ? 1 : 0) + (nseg > 0 ? nseg - 1 : 0);
         const long long flushes = P.par.compensated && P.par.sub > 0 ? steps / kCompWindow + 1 : 0;
-        a += steps * per + 1 + acf + (W.s1 - W.s0) + (nseg > 0 ? (steps + nseg - 1) * per + 2 * nseg : 0) + flushes;
+        const long long runs = std::max<long long>(nseg, 1);
+        const long long fsteps = loop ? runs : steps * per;
+        const long long asteps = loop ? (flushes ? std::max(flushes, runs) : runs) : steps * per;
+        const long long replay = loop ? nseg : (steps + nseg - 1) * per;
+        f += fsteps + 2 + (P.ae ? 1 : 0) + (nseg > 0 ? nseg - 1 : 0);
+        a += asteps + 1 + acf + (W.s1 - W.s0) + (nseg > 0 ? replay + 2 * nseg : 0) + flushes;
     }
     if (lf) *lf = f;
     if (la) *la = a;

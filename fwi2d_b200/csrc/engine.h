@@ -92,6 +92,8 @@ struct ModelDev {
 // reference computes it (float arithmetic unless noted).
 struct StepConst {
     float dt, dt2;               // dt, dt*dt
+    double idx64, idz64, idt64;  // 1/dx, 1/dz, 1/dt and 1/(dx*dx), 1/(dz*dz) of the
+    double id2x64, id2z64;       // single-precision values (fused.cu div64)
     float inv_d2x, inv_d2z;      // 1/(dx*dx), 1/(dz*dz)       (Dxx_var/Dzz_var a/d2)
     float adx, adz;              // 1/dx, 1/dz                 (mult_Dx/mult_Dz a/d)
     float sdx, sdz;              // (float)(1.0/(double)d)     (Dx/Dz interior scale)
@@ -128,6 +130,8 @@ struct MarchRef {
 
 // Work unit of the top / bottom band kernel: rows [xb, xe) of one shot's
 // top (side 0: z < 6) or bottom (side 1: z >= nz-6) band; roff as MarchRef.
+// Fused plans also hold their left (side 2) and right (side 3) bands this
+// way, with the z range [xb, xe) and no row records.
 struct BandRef {
     int shot, unit;
     int xb, xe;

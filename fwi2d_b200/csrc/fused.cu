@@ -1,21 +1,27 @@
-// One launch per time step for elastic, VTI and acoustic-elastic grids.
+// The whole time loop of a plan in one launch, for elastic, VTI and
+// acoustic-elastic grids.
 //
-// A launch advances every shot of a plan by one step.  Its CTAs (256 threads)
-// take three kinds of work units, the boundary units first:
-//   x-band     32 z cells of the 6 columns next to the left or right edge;
-//   z-band     32 columns of the 6 rows next to the top or bottom edge;
+// A cooperative launch of resident CTAs (256 threads) advances every shot by
+// the steps [it0, it1).  Each CTA keeps the same work units for all of them:
+//   x-band     up to 28 z cells of the 6 columns next to the left or right edge;
+//   z-band     up to 28 columns of the 6 rows next to the top or bottom edge;
 //   interior   a window of 32 (z) x 16 (x) cells clear of the bands.
 // Each unit performs the whole step of the reference time loop
 // (src/cpp/we_op.cpp:667-871 elastic, :1640-1840 VTI, :2240-2530 the elastic
 // grid of the acoustic-elastic propagator) with receivers, snapshots or the
 // imaging condition, in the reference's single-precision operation order.
 //
-// Consecutive steps are chained by programmatic dependent launch: a CTA of
-// step n+1 that finds a free slot while step n runs stages everything step n
-// does not write (model, boundary closures, snapshots of the imaging
-// condition) in shared memory before it waits for step n (griddepcontrol.wait).
-// Fields and gradients are read after the wait and through L2 (.cg): a line of
-// theirs may lie in L1 from before the wait.
+// Between steps the CTAs meet at a counter in global memory.  What a launch
+// per step costs, and this form does not: B200's SMs start each launch with a
+// cold instruction cache (measured on one 81 x 61 shot: about 18 cycles per
+// instruction of straight-line code, 12-20 thousand cycles through a band
+// unit), the launch gap, and the tail of CTAs.  A CTA stages what no step
+// writes (model, closures, snapshots of the imaging condition) before it waits
+// for the others, and keeps it in shared memory from step to step when it has
+// one unit only.
+//
+// Everything a step writes is read through L2 (.cg), written by the SM that
+// owns the cell and read by its neighbours after the counter.
 #include <cuda_runtime.h>
 #include "engine.h"
 #include "sbp.cuh"
@@ -32,10 +38,8 @@ constexpr int kFs = kFz + 8;                     // row stride of every staged a
 constexpr int kFt = 256;                         // threads: a z-pair of the interior window each
 constexpr int kFu = (kFx + 8) * kFs, kFw = (kFx + 4) * kFs, kFo = kFx * kFz;
 constexpr int kFb = 10;                          // band units: samples staged along the normal
+constexpr int kBt = kFusedBand + 8;              // and along the edge
 static_assert(kFt == kFz / 2 * kFx, "one z-pair per thread");
-
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // 16-byte asynchronous copy through L2; zeros when !ok (nothing is read then)
 __device__ __forceinline__ void cp16(float *dst, const float *src, bool ok)
@@ -61,24 +65,29 @@ __device__ __forceinline__ float2 dif2(float2 a, float2 b) { return fma2(b, kMin
 // lane by lane, for operands whose lanes do not sit in one register pair
 __device__ __forceinline__ float2 mulx(float ax, float ay, float2 b) { return make_float2(ax * b.x, ay * b.y); }
 
-// x / b rounded to nearest for r = 1/b rounded to nearest: two correction
-// steps of Markstein's division (IBM J. Res. Dev. 34, 1990); the first makes the
-// quotient faithful, the second rounds it correctly.  Exact while neither the
-// quotient nor the remainder leaves the normal range: |x| in [2^-100, 2^100]
-// and b in [2^-20, 2^20]; other operands take the divide (r = 0 marks such a b).
-constexpr float kDivLo = 7.888609052210118e-31f, kDivHi = 1.2676506002282294e30f;
-__device__ __forceinline__ float div_by(float x, float b, float r)
-{
-    const float a = fabsf(x);
-    if (a >= kDivLo && a <= kDivHi && r > 0.f) {
-        float q = x * r;
-        q = fmaf(fmaf(-q, b, x), r, q);
-        return fmaf(fmaf(-q, b, x), r, q);
-    }
-    return x / b;
-}
+// x / b rounded to nearest single precision from inv, 1/b in double precision
+// with a relative error below 2^-51: the quotient of two 24-bit significands
+// lies at least 2^-49 (relative) away from every midpoint of two neighbouring
+// single-precision numbers, so the double product rounds to the same number.
+// No branch, any magnitude, signed zeros included.
+__device__ __forceinline__ float div64(float x, double inv) { return (float)((double)x * inv); }
 
-// both components of a z-pair over the pair's densities
+// Both components of a z-pair over the pair's densities b, with r = 1/b rounded
+// to single precision: two correction steps of Markstein's division (IBM J.
+// Res. Dev. 34, 1990); the first makes the quotient faithful, the second
+// rounds it correctly.  Exact while neither the quotient nor the remainder
+// leaves the normal range: |x| in [2^-100, 2^100] and b in [2^-20, 2^20]
+// (r = 0 marks other b).  Other operands (the field's first, tiny values) take
+// the double product.
+constexpr float kDivLo = 7.888609052210118e-31f, kDivHi = 1.2676506002282294e30f;
+__device__ __forceinline__ double inverse64(float b, float r)
+{
+    if (!(r > 0.f)) return 1.0 / (double)b;
+    // two Newton steps from the 24 good bits of r
+    double q = (double)r;
+    q = fma(q, fma(-(double)b, q, 1.0), q);
+    return fma(q, fma(-(double)b, q, 1.0), q);
+}
 __device__ __forceinline__ void div_pairs(float2 &x0, float2 &x1, float2 b, float2 r)
 {
     const float hi = fmaxf(fmaxf(fabsf(x0.x), fabsf(x0.y)), fmaxf(fabsf(x1.x), fabsf(x1.y)));
@@ -90,11 +99,10 @@ __device__ __forceinline__ void div_pairs(float2 &x0, float2 &x1, float2 b, floa
         q1 = fma2(fma2(q1, nb, x1), r, q1);
         x0 = fma2(fma2(q0, nb, x0), r, q0);
         x1 = fma2(fma2(q1, nb, x1), r, q1);
-    } else if (hi == 0.f && fminf(b.x, b.y) > 0.f) {
-        return;   // 0 / b for both components: the zeros keep their signs
-    } else {
-        x0 = make_float2(x0.x / b.x, x0.y / b.y);
-        x1 = make_float2(x1.x / b.x, x1.y / b.y);
+    } else if (!(hi == 0.f && fminf(b.x, b.y) > 0.f)) {
+        const double ix = inverse64(b.x, r.x), iy = inverse64(b.y, r.y);
+        x0 = make_float2(div64(x0.x, ix), div64(x0.y, iy));
+        x1 = make_float2(div64(x1.x, ix), div64(x1.y, iy));
     }
 }
 
@@ -160,38 +168,74 @@ struct InLayout {
     static constexpr int FLOATS = RED + 8;
 };
 
-// Bands: [10 normal samples][40 tangential samples] per array, then the
-// closure coefficients of the owned rows, [6][8][32].
-template <bool VTI, bool GRAD>
+// Bands: [10 normal samples, counted from the edge][36 tangential samples] per
+// array (row stride kFs), then the closure coefficients of the owned rows,
+// [6][8][28], and for x bands those along z next to the corners, [2][6][8][6].
+// D, DS, DT: the strain sum (VTI and acoustic-elastic: two arrays) and the two
+// shear strains.
+template <bool VTI, bool GRAD, bool AE>
 struct BandLayout {
-    static constexpr int A = kFb * kFs, CL = 6 * 8 * 32;
-    static constexpr int U0 = 0, U1 = A, MU = 2 * A, Q = 3 * A, T0 = 4 * A, CZ = 5 * A, BX = 6 * A, T1 = 7 * A;
-    static constexpr int LB = 8 * A, LC = LB + (VTI ? A : 0), LA = LC + (VTI ? A : 0);
+    static constexpr int A = kFb * kFs, CL = 6 * 8 * kFusedBand;
+    static constexpr int UN = 0, UT = A, MU = 2 * A, Q = 3 * A, D = 4 * A, DS = 5 * A, DT = 6 * A;
+    static constexpr int D1 = 7 * A, LB = D1 + (VTI || AE ? A : 0), LC = LB + (VTI ? A : 0), LA = LC + (VTI ? A : 0);
     static constexpr int F0 = LA + (VTI ? A : 0), F1 = F0 + (GRAD ? A : 0), C0 = F1 + (GRAD ? A : 0);
     static constexpr int C1 = C0 + CL;                     // VTI x bands: closure of (1+2eps)2mu
-    static constexpr int RED = C1 + (VTI ? CL : 0);
+    static constexpr int ZC = C1 + (VTI ? CL : 0);
+    static constexpr int RED = ZC + 2 * 6 * 8 * 6;
     static constexpr int FLOATS = RED + 8;
 };
 
 template <bool VTI, bool GRAD, bool AE>
 constexpr size_t fused_bytes()
 {
-    return sizeof(float) * (InLayout<VTI, GRAD, AE>::FLOATS > BandLayout<VTI, GRAD>::FLOATS
+    return sizeof(float) * (InLayout<VTI, GRAD, AE>::FLOATS > BandLayout<VTI, GRAD, AE>::FLOATS
                                 ? InLayout<VTI, GRAD, AE>::FLOATS
-                                : BandLayout<VTI, GRAD>::FLOATS);
+                                : BandLayout<VTI, GRAD, AE>::FLOATS);
 }
 
 struct FusedArgs {
     const ShotDev *shots;
-    const TileRef *xb;
-    const BandRef *zb;
+    const BandRef *bands;   // x bands (side 2, 3), then z bands (side 0, 1)
     const TileRef *in;
-    int nxb, nzb;
+    int nband, nunit;       // band units, all units
     ModelDev M;
     StepConst C;
-    int it, flags;
+    int it0, it1, flags;
     float dtg;
+    unsigned *count;        // arrivals of this launch's steps, zero at its start
+    int *status;            // step + 1 of a wait that gave up
 };
+
+// ---- the meeting point of a launch's CTAs -------------------------------------
+__device__ __forceinline__ void arrive(const FusedArgs &A)
+{
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(A.count) : "memory");
+}
+__device__ __forceinline__ bool reached(const FusedArgs &A, unsigned target)
+{
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(A.count) : "memory");
+    return v >= target;
+}
+// Waits until every CTA has finished the steps before `it`.  The launch is
+// cooperative, so all of them are resident.  Bounded twice: past StepConst::spin
+// polls the step is reported, past kHardPolls more the CTA leaves (false).
+constexpr int kHardPolls = 1 << 22;
+__device__ __forceinline__ bool meet(const FusedArgs &A, int it)
+{
+    int lost = 0;
+    if (threadIdx.x == 0 && it > A.it0) {
+        const unsigned target = (unsigned)(it - A.it0) * gridDim.x;
+        bool ok = false;
+        for (int k = 0; k < A.C.spin && !ok; k++) ok = reached(A, target);
+        if (!ok) {
+            atomicCAS(A.status, 0, it + 1);
+            for (int k = 0; k < kHardPolls && !ok; k++) ok = reached(A, target);
+            lost = !ok;
+        }
+    }
+    return !__syncthreads_or(lost);
+}
 
 // max |next| of a CTA for the scale of the next 16-bit snapshot
 __device__ __forceinline__ void block_amax(float m, float *red, unsigned *dst)
@@ -229,15 +273,19 @@ __device__ __forceinline__ float density_term(float g, double wdt, int k, int la
 
 // ---------------------------------------------------------------------------
 // Interior window.  Thread t owns the z-pair 2 (t & 15) of column t >> 4.
-// Measured on B200, see launch_fused_step.
+// Measured on B200, see launch_fused.
 // ---------------------------------------------------------------------------
+// first: the CTA's first unit of this step (it waits for the others there);
+// keep: the unit's model arrays are in shared memory from the last step.
+// Returns false when the wait gave up.
 template <bool VTI, bool GRAD, bool AE>
-__device__ __forceinline__ void fused_interior(const FusedArgs &A, const TileRef tr, float *sm)
+__device__ __forceinline__ bool fused_interior(const FusedArgs &A, const TileRef tr, const int it, const bool first,
+                                               const bool keep, float *sm)
 {
     using L = InLayout<VTI, GRAD, AE>;
     const ModelDev &M = A.M;
     const StepConst &C = A.C;
-    const int t = threadIdx.x, it = A.it;
+    const int t = threadIdx.x;
     const ShotDev *__restrict__ Sp = A.shots + tr.shot;
     const int nt = Sp->nt, nx = Sp->nx, ldz = Sp->ldz;
     const int nxz = nx * ldz;
@@ -255,12 +303,14 @@ __device__ __forceinline__ void fused_interior(const FusedArgs &A, const TileRef
         const bool ok = gx < nx && gz < ldz;
         const long long o = mofs + (ok ? (long long)gx * ldz + gz : 0);
         const int s = xr * kFs + xq;
-        cp16(sm + L::MU + s, M.p1 + o, ok);
-        cp16(sm + L::Q + s, (VTI ? M.fxx : M.p0) + o, ok);
-        if (VTI) {
-            cp16(sm + L::LB + s, M.lbis + o, ok);
-            cp16(sm + L::LC + s, M.c13 + o, ok);
-            cp16(sm + L::LA + s, M.p0 + o, ok);
+        if (!keep) {
+            cp16(sm + L::MU + s, M.p1 + o, ok);
+            cp16(sm + L::Q + s, (VTI ? M.fxx : M.p0) + o, ok);
+            if (VTI) {
+                cp16(sm + L::LB + s, M.lbis + o, ok);
+                cp16(sm + L::LC + s, M.c13 + o, ok);
+                cp16(sm + L::LA + s, M.p0 + o, ok);
+            }
         }
         if (GRAD && do_grad) {
             const long long so = (long long)itf * Sp->snap_slot + (ok ? (long long)gx * ldz + gz : 0);
@@ -278,7 +328,7 @@ __device__ __forceinline__ void fused_interior(const FusedArgs &A, const TileRef
     const bool ook = ogx < nx && ogz < ldz;
     const long long oc = ook ? (long long)ogx * ldz + ogz : 0;
     const int os = (t >> 7) * kFo + orow * kFz + oq;
-    cp16(sm + L::RHO + os, ((t >> 7) ? M.irho : M.p2) + mofs + oc, ook);
+    if (!keep) cp16(sm + L::RHO + os, ((t >> 7) ? M.irho : M.p2) + mofs + oc, ook);
     if (GRAD && do_grad) {
         const long long oo = oc + (t >> 7 ? nxz : 0);
         auto own_snap = [&](int dst, int k, bool have) {
@@ -292,7 +342,7 @@ __device__ __forceinline__ void fused_interior(const FusedArgs &A, const TileRef
         };
         own_snap(L::FP0, itf + 1, itf + 1 <= last);
         own_snap(L::FM0, itf - 1, itf > 0);
-        if (VTI) {
+        if (VTI && !keep) {
             cp16(sm + L::E + os, ((t >> 7) ? M.gv2 : M.eps) + mofs + oc, ook);
             if (t < 128) cp16(sm + L::E + 2 * kFo + os, M.gv3 + mofs + oc, ook);
         }
@@ -311,11 +361,13 @@ __device__ __forceinline__ void fused_interior(const FusedArgs &A, const TileRef
     const float *curr = Sp->u[(it + 1) & 1];
     float *pn = Sp->u[it & 1];   // prev in, next out
 
-    pdl_wait();
-    pdl_launch();
+    if (first && !meet(A, it)) {
+        cp_wait();
+        return false;
+    }
     if (it >= nt - 1) {
         cp_wait();
-        return;
+        return true;
     }
 
     // ---- fields and, in the adjoint, the gradient
@@ -566,56 +618,65 @@ __device__ __forceinline__ void fused_interior(const FusedArgs &A, const TileRef
         if (own1) m = fmaxf(m, fmaxf(fabsf(n0.y), fabsf(n1.y)));
         block_amax(m, sm + L::RED, Sp->snap_amax + (it + 1) / C.sub);
     }
+    return true;
 }
 
 // ---------------------------------------------------------------------------
-// Band unit: 32 cells along the edge (tangential, lanes) x 6 rows next to it
-// (normal, warps 0-5).  XB: left / right edge, normal = x; else top / bottom,
-// normal = z.  The arithmetic is the tile kernel's general path through the
-// same sbp.cuh routines, except that the coefficient sums of the second
-// derivative's closure, which depend on the model only, come ready from
-// k_closures: 8 products instead of 8 x 16 operations and a division each.
+// Band unit: up to 28 cells along the edge (tangential, lanes 2-29) x 6 rows
+// next to it (warps 0-5).  XB: left / right edge, the normal is x; else top /
+// bottom, the normal is z.  In the components and axes along (t) and across
+// (n) the edge the operators of all four sides are the same; samples along the
+// normal are counted from the edge, which turns the sign (sg) of the far
+// side's first normal derivatives and leaves every rounding as it was
+// (s -= B b is s += (-B) b).  A row is uniform across a warp, so that the
+// closures' rows do not diverge.  The coefficient sums of the second
+// derivative's closure depend on the model only and come ready from
+// k_closures: 8 products and quotients instead of 8 x 16 operations.
 // ---------------------------------------------------------------------------
 template <bool XB, bool VTI, bool GRAD, bool AE>
-__device__ __forceinline__ void fused_band(const FusedArgs &A, const ShotDev *__restrict__ Sp, int far, int t0, int own0,
-                                           int own1, int unit, int roff, float *sm)
+__device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br, const int it, const bool first,
+                                           const bool keep, float *sm)
 {
-    using L = BandLayout<VTI, GRAD>;
+    using L = BandLayout<VTI, GRAD, AE>;
     const ModelDev &M = A.M;
     const StepConst &C = A.C;
-    const int t = threadIdx.x, it = A.it, lane = t & 31, warp = t >> 5;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const ShotDev *__restrict__ Sp = A.shots + br.shot;
     const int nt = Sp->nt, nx = Sp->nx, nz = Sp->nz, ldz = Sp->ldz;
     const int nxz = nx * ldz;
-    const int nn = XB ? nx : nz;                       // samples along the normal
-    const int nb = far ? nn - kFb : 0;                 // first staged normal sample
+    const bool far = br.side & 1;
+    const int t0 = br.xb, t1 = br.xe;                  // owned cells along the edge
+    const int nn = XB ? nx : nz;
     const int prec = C.snap_prec;
     const long long mofs = (long long)Sp->x0 * ldz;
     const int itf = GRAD ? (nt - 1 - (it + 1)) / C.sub : 0;
     const bool do_grad = GRAD && it < nt - 1 && ((nt - 1 - (it + 1)) % C.sub == 0) && (!AE || itf != 0);
     const int last = nt / C.sub;
-    constexpr int sx = XB ? kFs : 1, sz = XB ? 1 : kFs;   // shared-memory strides along x and z
-    // the unit's tangential range along the grid (z bands: columns clear of the x bands)
-    const int tlo = XB ? 0 : 2, thi = XB ? nz : own1 + 4;
+    const float sg = far ? -1.f : 1.f;
+    // along the edge: samples that exist (z bands: within the columns clear of the x bands and their halo)
+    const int glo = XB ? 0 : t0 - 4, ghi = XB ? nz : t1 + 4;
 
     // sample i of a staged array: its shared index, its cell, and whether it exists
     auto sample = [&](int i, int &s, int &o) {
         int c, tt;
-        if (XB) { c = i / kFs; tt = i - c * kFs; }
+        if (XB) { c = i / kBt; tt = i - c * kBt; }
         else { tt = i / kFb; c = i - tt * kFb; }
-        const int g = t0 - 4 + tt;
+        const int g = t0 - 4 + tt, gn = far ? nn - 1 - c : c;
         s = c * kFs + tt;
-        o = XB ? (nb + c) * ldz + g : g * ldz + nb + c;
-        return g >= tlo && g < thi;
+        o = XB ? gn * ldz + g : g * ldz + gn;
+        return g >= glo && g < ghi;
     };
-    for (int i = t; i < kFb * kFs; i += kFt) {
+    for (int i = t; i < kFb * kBt; i += kFt) {
         int s, o;
         const bool in = sample(i, s, o);
-        sm[L::MU + s] = in ? M.p1[mofs + o] : 0.f;
-        sm[L::Q + s] = in ? (VTI ? M.fxx : M.p0)[mofs + o] : 0.f;
-        if (VTI) {
-            sm[L::LB + s] = in ? M.lbis[mofs + o] : 0.f;
-            sm[L::LC + s] = in ? M.c13[mofs + o] : 0.f;
-            sm[L::LA + s] = in ? M.p0[mofs + o] : 0.f;
+        if (!keep) {
+            sm[L::MU + s] = in ? M.p1[mofs + o] : 0.f;
+            sm[L::Q + s] = in ? (VTI ? M.fxx : M.p0)[mofs + o] : 0.f;
+            if (VTI) {
+                sm[L::LB + s] = in ? M.lbis[mofs + o] : 0.f;
+                sm[L::LC + s] = in ? M.c13[mofs + o] : 0.f;
+                sm[L::LA + s] = in ? M.p0[mofs + o] : 0.f;
+            }
         }
         if (GRAD && do_grad) {
             const long long so = (long long)itf * Sp->snap_slot + o;
@@ -624,28 +685,32 @@ __device__ __forceinline__ void fused_band(const FusedArgs &A, const ShotDev *__
             sm[L::F1 + s] = in ? snap_load(Sp->snap, so + nxz, prec, inv) : 0.f;
         }
     }
-    // closure coefficients [far][row][sample][tangential] of this unit's cells
-    {
-        const int ld = XB ? ldz : M.nx, base = (XB ? 0 : Sp->x0) + t0 + lane;
-        const bool in = XB ? t0 + lane < nz : t0 + lane < own1;
-        for (int k = warp; k < 48; k += kFt / 32) {
-            const long long o = (long long)(far * 48 + k) * ld + base;
-            sm[L::C0 + k * 32 + lane] = in ? (XB ? Sp->xclos : M.zclos)[o] : 0.f;
-            if (VTI && XB) sm[L::C1 + k * 32 + lane] = in ? Sp->xclos[(long long)96 * ldz + o] : 0.f;
+    if (!keep) {
+        // closure coefficients [row][sample][tangential] of the owned cells
+        const int ld = XB ? ldz : M.nx, base = (XB ? 0 : Sp->x0) + t0;
+        for (int i = t; i < L::CL; i += kFt) {
+            const int k = i / kFusedBand, q = i - k * kFusedBand;
+            const bool in = t0 + q < t1;
+            const long long o = (long long)((far ? 48 : 0) + k) * ld + base + q;
+            sm[L::C0 + i] = in ? (XB ? Sp->xclos : M.zclos)[o] : 0.f;
+            if (VTI && XB) sm[L::C1 + i] = in ? Sp->xclos[(long long)96 * ldz + o] : 0.f;
         }
+        if (XB)   // along z next to the corners: [top, bottom][row][sample][column]
+            for (int i = t; i < 2 * 48 * 6; i += kFt) {
+                const int k = i / 6, c = i - 6 * k;
+                sm[L::ZC + i] = M.zclos[(long long)k * M.nx + Sp->x0 + (far ? nx - 1 - c : c)];
+            }
     }
 
-    // this thread's cell: normal row k, tangential t0 + lane
-    const int k = warp, c = (far ? kFb - 6 : 0) + k, r = far ? 5 - k : k;
-    const int gn = nb + c, gt = t0 + lane;
+    // this thread's cell: row `warp` from the edge, tangential t0 + lane - 2
+    const int gt = t0 + lane - 2, gn = far ? nn - 1 - warp : warp;
     const int gx = XB ? gn : gt, gz = XB ? gt : gn;
-    const bool owned = warp < 6 && gt >= own0 && gt < own1;
-    const int cell = gx * ldz + gz;
+    const bool owned = warp < 6 && lane >= 2 && gt < t1;
+    const int cell = owned ? gx * ldz + gz : 0;
     const long long mcell = mofs + cell;
-    float rho = 1.f, irho = 0.f, tzv = 0.f, txv = 0.f, fp0 = 0.f, fp1 = 0.f, fm0 = 0.f, fm1 = 0.f;
+    float rho = 1.f, tzv = 0.f, txv = 0.f, fp0 = 0.f, fp1 = 0.f, fm0 = 0.f, fm1 = 0.f;
     if (owned) {
         rho = M.p2[mcell];
-        irho = M.irho[mcell];
         tzv = Sp->tz[gz];
         txv = Sp->tx[gx];
         if (GRAD && do_grad) {
@@ -663,18 +728,36 @@ __device__ __forceinline__ void fused_band(const FusedArgs &A, const ShotDev *__
             }
         }
     }
+    const double irho = 1.0 / (double)rho;
+    const bool edge = owned && (gz == 0 || gz == nz - 1 || gx == 0 || gx == nx - 1);
+    // entries of this unit: x bands its own list, z bands one record per column
+    int e0, e1, r0, r1, rstep;
+    if (XB) {
+        e0 = Sp->inj_off[br.unit];
+        e1 = Sp->inj_off[br.unit + 1];
+        r0 = Sp->ext_off[br.unit] + t;
+        r1 = Sp->ext_off[br.unit + 1];
+        rstep = kFt;
+    } else {
+        MarchRow R = {};
+        if (lane >= 2 && gt < t1) R = Sp->mrow[br.roff + gt - t0];
+        e0 = R.e0;
+        e1 = R.e1;
+        r0 = R.r0;
+        r1 = warp == 0 ? R.r1 : R.r0;
+        rstep = 1;
+    }
     const float *curr = Sp->u[(it + 1) & 1];
     float *pn = Sp->u[it & 1];
 
-    pdl_wait();
-    pdl_launch();
-    if (it >= nt - 1) return;
+    if (first && !meet(A, it)) return false;
+    if (it >= nt - 1) return true;
 
-    for (int i = t; i < kFb * kFs; i += kFt) {
+    for (int i = t; i < kFb * kBt; i += kFt) {
         int s, o;
         const bool in = sample(i, s, o);
-        sm[L::U0 + s] = in ? __ldcg(curr + o) : 0.f;
-        sm[L::U1 + s] = in ? __ldcg(curr + nxz + o) : 0.f;
+        sm[L::UN + s] = in ? __ldcg(curr + o + (XB ? 0 : nxz)) : 0.f;
+        sm[L::UT + s] = in ? __ldcg(curr + o + (XB ? nxz : 0)) : 0.f;
     }
     float p0 = 0.f, p1 = 0.f, g0 = 0.f, g1 = 0.f, g2 = 0.f;
     if (owned) {
@@ -688,154 +771,175 @@ __device__ __forceinline__ void fused_band(const FusedArgs &A, const ShotDev *__
     }
     __syncthreads();
 
-    const float *U0 = sm + L::U0, *U1 = sm + L::U1, *MU = sm + L::MU, *Q = sm + L::Q;
-    float *T0 = sm + L::T0, *T1 = sm + L::T1, *CZ = sm + L::CZ, *BX = sm + L::BX;
-    // ---- first derivatives on the 8 rows next to the edge, 2 cells beyond the unit along it
-    for (int i = t; i < 8 * 36; i += kFt) {
-        const int q = i / 36, tt = 2 + i - q * 36, cc = (far ? 2 : 0) + q;
-        const int g = t0 - 4 + tt, n = nb + cc;
-        // along z a closure reads up to 5 samples from its edge: evaluate where the window holds them
-        bool ok = g >= tlo && g < thi;
-        if (XB) ok = ok && ((g >= 4 && g < nz - 4) || (g < 4 ? t0 <= 4 : t0 + kFz + 4 >= nz));
-        else ok = ok && g >= 4 && g < own1 + 2;
-        if (!ok) continue;
-        const int s = cc * kFs + tt;
-        const int x = XB ? n : g, z = XB ? g : n;
-        const float ux_x = d1(U0 + s, sx, x, nx, C.dx, C.sdx);
-        const float uz_z = d1(U1 + s, sz, z, nz, C.dz, C.sdz);
-        BX[s] = d1(U1 + s, sx, x, nx, C.dx, C.sdx);
-        CZ[s] = d1(U0 + s, sz, z, nz, C.dz, C.sdz);
-        if (VTI) {
-            const float lb = sm[L::LB + s], c13 = sm[L::LC + s], lam = sm[L::LA + s];
-            T0[s] = lb * ux_x + c13 * uz_z;
-            T1[s] = lam * uz_z + c13 * ux_x;
-        } else if (AE) {
-            T0[s] = ux_x;
-            T1[s] = uz_z;
-        } else {
-            T0[s] = ux_x + uz_z;
+    const float ssn = XB ? C.sdx : C.sdz, sst = XB ? C.sdz : C.sdx, adn = XB ? C.adx : C.adz, adt = XB ? C.adz : C.adx;
+    const double idn = XB ? C.idx64 : C.idz64, idt = XB ? C.idz64 : C.idx64;
+    const double idn2 = XB ? C.id2x64 : C.id2z64;
+    const float inv_d2t = XB ? C.inv_d2z : C.inv_d2x;
+    const int i = warp * kFs + lane + 2;      // this thread's sample
+    // x bands: z closures along the edge; zo / zs: the end's sample relative to this one and the way in
+    const int zr = XB ? (gz < nz - 1 - gz ? gz : nz - 1 - gz) : 6;
+    const bool zfar = XB && gz >= nz - 1 - gz;
+    const int zo = XB ? (zfar ? nz - 1 - gz : -gz) : 0, zs = zfar ? -1 : 1;
+
+    // first derivatives at sample i of array p (row `warp`)
+    auto dern = [&](int p) {
+        const float *u = sm + p + i;
+        if (warp >= 4)
+            return sg * (ssn * (kC1[0] * (u[kFs] - u[-kFs]) + kC1[1] * (u[2 * kFs] - u[-2 * kFs])));
+        const float *b = sm + p + lane + 2;
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 6; k++) s += kB1[warp][k] * b[k * kFs];
+        return div64(sg * s, idn);
+    };
+    // sum of the closure row along the edge (x bands near the corners), without the division
+    auto zsum = [&](const float *u) {
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 6; k++) s += ((zfar ? -1.f : 1.f) * kB1[zr][k]) * u[zo + k * zs];
+        return s;
+    };
+    auto dert = [&](int p) {
+        const float *u = sm + p + i;
+        if (XB && zr < 4) return div64(zsum(u), idt);
+        return sst * (kC1[0] * (u[1] - u[-1]) + kC1[1] * (u[2] - u[-2]));
+    };
+    // first derivatives of products of arrays p and q
+    auto mdern = [&](int p, int q) {
+        const float *u = sm + p + i, *v = sm + q + i;
+        if (warp >= 4)
+            return sg * (adn * (kC1[0] * (u[kFs] * v[kFs] - u[-kFs] * v[-kFs]) +
+                                kC1[1] * (u[2 * kFs] * v[2 * kFs] - u[-2 * kFs] * v[-2 * kFs])));
+        const float *b = sm + p + lane + 2, *c = sm + q + lane + 2;
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 6; k++) s += kB1[warp][k] * b[k * kFs] * c[k * kFs];
+        return adn * (sg * s);
+    };
+    auto mdert = [&](int p, int q) {
+        const float *u = sm + p + i, *v = sm + q + i;
+        if (XB && zr < 4) {
+            float s = 0.f;
+#pragma unroll
+            for (int k = 0; k < 6; k++)
+                s += ((zfar ? -1.f : 1.f) * kB1[zr][k]) * u[zo + k * zs] * v[zo + k * zs];
+            return adt * s;
         }
+        return adt * (kC1[0] * (u[1] * v[1] - u[-1] * v[-1]) + kC1[1] * (u[2] * v[2] - u[-2] * v[-2]));
+    };
+
+    // ---- first derivatives on the 8 rows next to the edge, 2 cells beyond the unit along it.
+    // Near a corner the closure's samples have to lie in the staged window: other points are never used.
+    float en = 0.f, et = 0.f, es = 0.f, eq = 0.f;   // d_n un, d_t ut, d_n ut, d_t un
+    if (gt >= glo && gt < ghi) {
+        en = dern(L::UN);
+        es = dern(L::UT);
+        if (!XB || zr >= 4 || (zfar ? nz - 1 - t0 + 4 < kBt : t0 - 4 <= 0)) {
+            et = dert(L::UT);
+            eq = dert(L::UN);
+        }
+        if (VTI) {
+            const float lb = sm[L::LB + i], lc = sm[L::LC + i], la = sm[L::LA + i];
+            sm[L::D + i] = (XB ? lb : la) * en + lc * et;
+            sm[L::D1 + i] = (XB ? la : lb) * et + lc * en;
+        } else if (AE) {
+            sm[L::D + i] = en;
+            sm[L::D1 + i] = et;
+        } else {
+            sm[L::D + i] = en + et;
+        }
+        sm[L::DS + i] = es;
+        sm[L::DT + i] = eq;
     }
     __syncthreads();
 
     // receivers of this unit (forward)
     if (!GRAD && (A.flags & F_EXTRACT)) {
-        int r0 = 0, r1 = 0, step = 1;
-        if (XB) {
-            r0 = Sp->ext_off[unit] + t;
-            r1 = Sp->ext_off[unit + 1];
-            step = kFt;
-        } else if (t < own1 - own0) {
-            const MarchRow Rr = Sp->mrow[roff + t];
-            r0 = Rr.r0;
-            r1 = Rr.r1;
-        }
-        for (int e = r0; e < r1; e += step) {
+        for (int e = r0; e < r1; e += rstep) {
             const ExtEntry &E = Sp->ext[e];
-            const float *U = E.comp == 0 ? U0 : U1;
-            const int base = XB ? (E.gx0 - nb) * kFs + E.gz0 - t0 + 4 : (E.gz0 - nb) * kFs + E.gx0 - t0 + 4;
+            const bool nc = XB ? E.comp == 0 : E.comp == 1;
+            const int gn0 = XB ? E.gx0 : E.gz0, gt0 = XB ? E.gz0 : E.gx0;
+            const float *U = sm + (nc ? L::UN : L::UT) + (far ? nn - 1 - gn0 : gn0) * kFs + gt0 - t0 + 4;
+            const int sn = far ? -kFs : kFs;
             float o = 0.f;
 #pragma unroll
             for (int a = 0; a < 3; a++)
 #pragma unroll
-                for (int b = 0; b < 3; b++) o += E.w[a * 3 + b] * U[base + a * sx + b * sz];
+                for (int b = 0; b < 3; b++) o += E.w[a * 3 + b] * U[XB ? a * sn + b : b * sn + a];
             Sp->rcv[(long long)it * Sp->nrcv + E.row] = o;
         }
     }
 
     float amax = 0.f;
     if (owned) {
-        const int i = c * kFs + lane + 4;
-        const float a00 = U0[i], b00 = U1[i], mu = MU[i];
-        // second derivatives: along the normal the closure rows, along the edge the
-        // interior form (x bands: the closure again near the corners)
-        const float dn2 = XB ? C.d2x : C.d2z, idn2 = XB ? C.inv_d2x : C.inv_d2z;   // inv_d2 is 1/d2 rounded
-        const int en = (far ? kFb - 1 : 0) * kFs + lane + 4, dn = far ? -kFs : kFs;
-        const float *CL = sm + L::C0 + r * 256 + lane, *CQ = sm + (VTI && XB ? L::C1 : L::C0) + r * 256 + lane;
-        float n0 = 0.f, n1 = 0.f;
-        if (XB) {
-            // ux: x closure of 2 mu (VTI: (1+2eps)2mu), then z with mu; uz: z with 2 mu, then x closure of mu
+        const float un = sm[L::UN + i], ut = sm[L::UT + i], mu = sm[L::MU + i];
+        float pn_ = XB ? p0 : p1, pt_ = XB ? p1 : p0;   // previous values
+        // second derivatives: the closure rows across the edge, the interior form along it
+        // (x bands: the closure again near the corners); acc += val u / d^2, sample by sample
+        const float *CL = sm + L::C0 + warp * 8 * kFusedBand + lane - 2;
+        const float *CQ = sm + (VTI && XB ? L::C1 : L::C0) + warp * 8 * kFusedBand + lane - 2;
+        const float *UN = sm + L::UN + lane + 2, *UT = sm + L::UT + lane + 2;
+        float an = 0.f, at = 0.f;
 #pragma unroll
-            for (int j = 0; j < 8; j++)
-                n0 += div_by((VTI ? CQ[j * 32] : 2.f * CL[j * 32]) * U0[en + j * dn], dn2, idn2);
-            if (gz >= 6 && gz < nz - 6) {
-                const Brk b = brackets(MU + i, 1);
-                n1 = d2i(n1, twice(b), U1 + i, 1, C.inv_d2z);
-                n0 = d2i(n0, b, U0 + i, 1, C.inv_d2z);
-            } else {
-                const bool bot = gz >= 6;
-                const int rz = bot ? nz - 1 - gz : gz, d = bot ? -1 : 1;
-                const int ez = c * kFs + (bot ? nz - 1 : 0) - t0 + 4;
-                const float *zc = M.zclos + (long long)(bot ? 48 : 0) * M.nx + (long long)rz * 8 * M.nx + Sp->x0 + gx;
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const float v = zc[(long long)j * M.nx];
-                    n1 += div_by((2.f * v) * U1[ez + j * d], C.d2z, C.inv_d2z);
-                    n0 += div_by(v * U0[ez + j * d], C.d2z, C.inv_d2z);
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 8; j++) n1 += div_by(CL[j * 32] * U1[en + j * dn], dn2, idn2);
-        } else {
-            const Brk b = brackets(MU + i, 1);
-            if (VTI) n0 = d2i(n0, brackets(Q + i, 1), U0 + i, 1, C.inv_d2x);
-            else n0 = d2i(n0, twice(b), U0 + i, 1, C.inv_d2x);
-#pragma unroll
+        for (int j = 0; j < 8; j++)
+            an += div64((VTI && XB ? CQ[j * kFusedBand] : 2.f * CL[j * kFusedBand]) * UN[j * kFs], idn2);
+        if (XB && zr < 6) {
+            const float *zc = sm + L::ZC + (zfar ? 288 : 0) + zr * 48 + warp;
+            const float *vn = sm + L::UN + i + zo, *vt = sm + L::UT + i + zo;
+#pragma unroll 2
             for (int j = 0; j < 8; j++) {
-                const float v = CL[j * 32];
-                n1 += div_by((2.f * v) * U1[en + j * dn], dn2, idn2);
-                n0 += div_by(v * U0[en + j * dn], dn2, idn2);
+                const float v = zc[j * 6];
+                at += div64((2.f * v) * vt[j * zs], C.id2z64);
+                an += div64(v * vn[j * zs], C.id2z64);
             }
-            n1 = d2i(n1, b, U1 + i, 1, C.inv_d2x);
+        } else {
+            const Brk b = brackets(sm + L::MU + i, 1);
+            if (VTI && !XB) at = d2i(at, brackets(sm + L::Q + i, 1), sm + L::UT + i, 1, inv_d2t);
+            else at = d2i(at, twice(b), sm + L::UT + i, 1, inv_d2t);
+            an = d2i(an, b, sm + L::UN + i, 1, inv_d2t);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) at += div64(CL[j * kFusedBand] * UT[j * kFs], idn2);
+        // mixed terms
+        if (VTI) {
+            an += dern(L::D);
+            at += dert(L::D1);
+        } else {
+            an += mdern(L::D, L::Q);
+            at += mdert(AE ? L::D1 : L::D, L::Q);
         }
         if (AE) {
-            n0 += md1(T0 + i, Q + i, sx, gx, nx, C.adx);
-            n1 += md1(T1 + i, Q + i, sz, gz, nz, C.adz);
-            n0 += md1(T1 + i, Q + i, sx, gx, nx, C.adx);
-            n1 += md1(T0 + i, Q + i, sz, gz, nz, C.adz);
-        } else if (!VTI) {
-            n0 += md1(T0 + i, Q + i, sx, gx, nx, C.adx);
-            n1 += md1(T0 + i, Q + i, sz, gz, nz, C.adz);
-        } else {
-            n0 += d1(T0 + i, sx, gx, nx, C.dx, C.sdx);
-            n1 += d1(T1 + i, sz, gz, nz, C.dz, C.sdz);
+            an += mdern(L::D1, L::Q);
+            at += mdert(L::D, L::Q);
         }
-        n1 += md1(CZ + i, MU + i, sx, gx, nx, C.adx);
-        n0 += md1(BX + i, MU + i, sz, gz, nz, C.adz);
-
-        // sources of this cell, in the reference's order
-        int e0, e1;
         if (XB) {
-            e0 = Sp->inj_off[unit];
-            e1 = Sp->inj_off[unit + 1];
+            at += mdern(L::DT, L::MU);
+            an += mdert(L::DS, L::MU);
         } else {
-            const MarchRow Rr = Sp->mrow[roff + gt - own0];
-            e0 = Rr.e0;
-            e1 = Rr.e1;
+            an += mdert(L::DS, L::MU);
+            at += mdern(L::DT, L::MU);
         }
+        // sources of this cell, in the reference's order
         if (e0 < e1) {
             const float *srcrow = Sp->src + (long long)it * Sp->nsrc;
             for (int e = e0; e < e1; e++) {
                 const InjEntry &E = Sp->inj[e];
                 if (E.gx != gx || E.gz != gz) continue;
                 const float v = E.mt ? (E.wa * srcrow[E.ia] - E.wb * srcrow[E.ib]) : E.wa * srcrow[E.ia];
-                if (E.comp == 0) n0 += v;
-                else n1 += v;
+                if (XB ? E.comp == 0 : E.comp == 1) an += v;
+                else at += v;
             }
         }
         if (it > 0) {
-            p0 = p0 * tzv * txv;
-            p1 = p1 * tzv * txv;
+            pn_ = pn_ * tzv * txv;
+            pt_ = pt_ * tzv * txv;
         }
 
         // SAT closures (spatial_operators.hpp:160-822), in the reference's side order
         // (the fluid interface of the acoustic-elastic propagator, its top edge, last)
-        const bool edge = gz == 0 || gz == nz - 1 || gx == 0 || gx == nx - 1;
         if (edge) {
-            const float lam = VTI ? sm[L::LA + i] : Q[i];
-            const float c13 = VTI ? sm[L::LC + i] : lam;
-            const float fxx = VTI ? Q[i] : 2 * mu;
-            const float lamx = VTI ? sm[L::LB + i] : lam;
+            const float lam = VTI ? sm[L::LA + i] : sm[L::Q + i], c13 = VTI ? sm[L::LC + i] : lam;
+            const float fxx = VTI ? sm[L::Q + i] : 2 * mu, lamx = VTI ? sm[L::LB + i] : lam;
             const float imp_s = 0.5f * sqrtf(mu * rho);
             const float imp_p = 0.5f * sqrtf((lam + 2 * mu) * rho);
             const float imp_px = VTI ? 0.5f * sqrtf((1 + 2 * M.eps[mcell]) * (lam + 2 * mu) * rho) : imp_p;
@@ -843,36 +947,68 @@ __device__ __forceinline__ void fused_band(const FusedArgs &A, const ShotDev *__
             for (int q = 0; q < 4; q++) {
                 const int side = AE ? (q + 1) & 3 : q;
                 const int bc = side == 0 ? C.bc[0] : side == 1 ? C.bc[1] : side == 2 ? C.bc[2] : C.bc[3];
-                if (bc != 1 && bc != 2) continue;
-                const bool ab = bc == 2;
-                if (side < 2) {
-                    if (gz != (side == 0 ? 0 : nz - 1)) continue;
-                    const int in = side == 0 ? sz : -sz;
-                    const float sg = side == 0 ? -1.f : 1.f;
-                    float tt = (sg * mu) * tsum(U1 + i, sx, gx, nx) / C.dx + mu * nsum(U0 + i, in) / C.dz;
-                    if (ab) tt = tt - imp_s * p0 / C.dt;
-                    n0 = n0 - C.sat_z * tt;
-                    tt = (sg * c13) * tsum(U0 + i, sx, gx, nx) / C.dx + (2 * mu) * nsum(U1 + i, in) / C.dz;
-                    if (ab) tt = tt - imp_p * p1 / C.dt;
-                    n1 = n1 - C.sat_z * tt;
-                    n1 = n1 - C.nsat_z * lam * ndsum(U1 + i, in);
-                } else if (XB) {
-                    if (gx != (side == 2 ? 0 : nx - 1)) continue;
-                    const int in = side == 2 ? sx : -sx;
-                    const float sg = side == 2 ? -1.f : 1.f;
-                    float tt = (sg * c13) * tsum(U1 + i, sz, gz, nz) / C.dz + fxx * nsum(U0 + i, in) / C.dx;
-                    if (ab) tt = tt - imp_px * p0 / C.dt;
-                    n0 = n0 - C.sat_x * tt;
-                    n0 = n0 - C.nsat_x * lamx * ndsum(U0 + i, in);
-                    tt = (sg * mu) * tsum(U0 + i, sz, gz, nz) / C.dz + mu * nsum(U1 + i, in) / C.dx;
-                    if (ab) tt = tt - imp_s * p1 / C.dt;
-                    n1 = n1 - C.sat_x * tt;
+                const bool zside = side < 2;
+                if ((bc != 1 && bc != 2) || (zside ? gz : gx) != (side & 1 ? (zside ? nz : nx) - 1 : 0)) continue;
+                const bool mine = XB ? !zside : zside;   // the band's own edge, or the other one at a corner
+                // u across the side, u along it; derivative sums along the side (tsum) and into the domain
+                const float *v = sm + (mine ? L::UN : L::UT) + i, *w = sm + (mine ? L::UT : L::UN) + i;
+                const int in = mine ? kFs : zs;          // samples count from the edge / the corner
+                const float s2 = side & 1 ? 1.f : -1.f;
+                float sv, sw;   // tsum of v and w along the side
+                if (mine) {
+                    if (XB && zr < 4) {
+                        sv = zsum(v);
+                        sw = zsum(w);
+                    } else {
+                        sv = 0.f + kC1[0] * (v[1] - v[-1]);
+                        sv += kC1[1] * (v[2] - v[-2]);
+                        sw = 0.f + kC1[0] * (w[1] - w[-1]);
+                        sw += kC1[1] * (w[2] - w[-2]);
+                    }
+                } else {
+                    // along the band's normal, at row `warp`
+                    if (warp >= 4) {
+                        sv = 0.f + kC1[0] * (v[kFs] - v[-kFs]);
+                        sv += kC1[1] * (v[2 * kFs] - v[-2 * kFs]);
+                        sw = 0.f + kC1[0] * (w[kFs] - w[-kFs]);
+                        sw += kC1[1] * (w[2 * kFs] - w[-2 * kFs]);
+                    } else {
+                        sv = sw = 0.f;
+#pragma unroll
+                        for (int k = 0; k < 6; k++) {
+                            sv += kB1[warp][k] * v[(k - warp) * kFs];
+                            sw += kB1[warp][k] * w[(k - warp) * kFs];
+                        }
+                    }
+                    sv = sg * sv;
+                    sw = sg * sw;
                 }
+                float nv = 0.f, nw = 0.f, nd = 0.f;   // S.v, S.w and -(D v)_0 (sbp.cuh nsum, ndsum)
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    nv += kSC[k] * v[k * in];
+                    nw += kSC[k] * w[k * in];
+                }
+#pragma unroll
+                for (int k = 0; k < 6; k++) nd -= kB1[0][k] * v[k * in];
+                const double ia = mine ? idt : idn, ic = mine ? idn : idt;   // 1 / spacing along and across the side
+                const float sat = zside ? C.sat_z : C.sat_x;
+                float along = mine ? at : an, across = mine ? an : at;
+                float tt = div64((s2 * mu) * sv, ia) + div64(mu * nw, ic);
+                if (bc == 2) tt = tt - div64(imp_s * (mine ? pt_ : pn_), C.idt64);
+                along = along - sat * tt;
+                tt = div64((s2 * c13) * sw, ia) + div64((zside ? 2 * mu : fxx) * nv, ic);
+                if (bc == 2) tt = tt - div64((zside ? imp_p : imp_px) * (mine ? pn_ : pt_), C.idt64);
+                across = across - sat * tt;
+                across = across - (zside ? C.nsat_z : C.nsat_x) * (zside ? lam : lamx) * nd;
+                an = mine ? across : along;
+                at = mine ? along : across;
             }
         }
 
-        n0 = div_by(C.dt2 * n0, rho, irho) + 2 * a00 - p0;
-        n1 = div_by(C.dt2 * n1, rho, irho) + 2 * b00 - p1;
+        an = div64(C.dt2 * an, irho) + 2 * un - pn_;
+        at = div64(C.dt2 * at, irho) + 2 * ut - pt_;
+        float n0 = XB ? an : at, n1 = XB ? at : an;
         if (edge) {
             const int per = 2 * nx + 2 * nz;
             int kk;
@@ -880,11 +1016,11 @@ __device__ __forceinline__ void fused_band(const FusedArgs &A, const ShotDev *__
             else if (gz == nz - 1) kk = nx + gx;
             else if (gx == 0) kk = 2 * nx + gz;
             else kk = 2 * nx + nz + gz;
-            n0 = n0 / Sp->den[kk];
-            n1 = n1 / Sp->den[per + kk];
+            n0 = div64(n0, 1.0 / (double)Sp->den[kk]);
+            n1 = div64(n1, 1.0 / (double)Sp->den[per + kk]);
         }
         n0 = n0 * tzv * txv;
-        if (AE && gz == 0) Sp->halo_save[gx] = p1;   // interface row: coupled and tapered by ae_couple
+        if (AE && gz == 0) Sp->halo_save[gx] = XB ? pt_ : pn_;   // interface row: coupled and tapered by ae_couple
         else n1 = n1 * tzv * txv;
         pn[cell] = n0;
         pn[nxz + cell] = n1;
@@ -893,16 +1029,16 @@ __device__ __forceinline__ void fused_band(const FusedArgs &A, const ShotDev *__
             const int slot = it / C.sub;
             const float sc = prec == SNAP_FP32 ? 1.f : snap_scale(Sp->snap_amax, slot);
             const long long o = (long long)slot * Sp->snap_slot + cell;
-            snap_store(Sp->snap, o, prec, a00, sc);
-            snap_store(Sp->snap, o + nxz, prec, b00, sc);
+            snap_store(Sp->snap, o, prec, XB ? un : ut, sc);
+            snap_store(Sp->snap, o + nxz, prec, XB ? ut : un, sc);
         }
 
         if (GRAD && do_grad) {
-            const float *F0 = sm + L::F0, *F1 = sm + L::F1;
-            const float ax0 = d1(U0 + i, sx, gx, nx, C.dx, C.sdx), az1 = d1(U1 + i, sz, gz, nz, C.dz, C.sdz);
-            const float q0 = d1(F0 + i, sx, gx, nx, C.dx, C.sdx), q1 = d1(F1 + i, sz, gz, nz, C.dz, C.sdz);
-            const float q2 = d1(F1 + i, sx, gx, nx, C.dx, C.sdx), q3 = d1(F0 + i, sz, gz, nz, C.dz, C.sdz);
-            const float az0 = CZ[i], ax1 = BX[i];
+            // strains of the adjoint field (this thread's own) and of the snapshot
+            const float ax0 = XB ? en : et, az1 = XB ? et : en, ax1 = XB ? es : eq, az0 = XB ? eq : es;
+            const int FN = XB ? L::F0 : L::F1, FT = XB ? L::F1 : L::F0;
+            const float qn = dern(FN), qt = dert(FT), qs = dern(FT), qq = dert(FN);
+            const float q0 = XB ? qn : qt, q1 = XB ? qt : qn, q2 = XB ? qs : qq, q3 = XB ? qq : qs;
             float dl = 0.f, dm;
             if (!VTI) {
                 dm = (az0 + ax1) * (q2 + q3) + 2 * ax0 * q0 + 2 * az1 * q1;
@@ -928,11 +1064,13 @@ __device__ __forceinline__ void fused_band(const FusedArgs &A, const ShotDev *__
             G[nxz] = g1;
             // interface row: the density term needs the coupled uz (ae_couple)
             if (!AE || gz != 0)
-                G[2 * (long long)nxz] = density_term(g2, wdt, itf, last, n0, n1, F0[i], F1[i], fp0, fp1, fm0, fm1);
+                G[2 * (long long)nxz] = density_term(g2, wdt, itf, last, n0, n1, sm[L::F0 + i], sm[L::F1 + i], fp0, fp1,
+                                                     fm0, fm1);
         }
     }
     if (!GRAD && (A.flags & F_AMAX) && (it + 1) % C.sub == 0)
         block_amax(amax, sm + L::RED, Sp->snap_amax + (it + 1) / C.sub);
+    return true;
 }
 
 #ifndef FUSED_FWD_BLOCKS
@@ -943,18 +1081,30 @@ __device__ __forceinline__ void fused_band(const FusedArgs &A, const ShotDev *__
 #endif
 template <bool VTI, bool GRAD, bool AE>
 __global__ void __launch_bounds__(kFt, VTI && GRAD ? 3 : (GRAD ? FUSED_GRAD_BLOCKS : FUSED_FWD_BLOCKS))
-fused_step(const __grid_constant__ FusedArgs A)
+fused_steps(const __grid_constant__ FusedArgs A)
 {
     extern __shared__ __align__(16) float sm[];
-    const int b = blockIdx.x;
-    if (b < A.nxb) {
-        const TileRef tr = A.xb[b];
-        fused_band<true, VTI, GRAD, AE>(A, A.shots + tr.shot, tr.ox0 != 0, tr.wz0, tr.oz0, tr.oz1, tr.unit, 0, sm);
-    } else if (b < A.nxb + A.nzb) {
-        const BandRef br = A.zb[b - A.nxb];
-        fused_band<false, VTI, GRAD, AE>(A, A.shots + br.shot, br.side, br.xb, br.xb, br.xe, br.unit, br.roff, sm);
-    } else {
-        fused_interior<VTI, GRAD, AE>(A, A.in[b - A.nxb - A.nzb], sm);
+    // slots blockIdx.x, + gridDim.x, ... of the units rotated so that, with fewer
+    // than two units per CTA, the band units (the longest) get a CTA of their own
+    const int off = A.nunit < 2 * (int)gridDim.x ? max(0, A.nunit - (int)gridDim.x) : 0;
+    const bool one = blockIdx.x + gridDim.x >= A.nunit;   // this CTA's only unit
+    for (int it = A.it0; it < A.it1; it++) {
+        const bool keep = one && it > A.it0;
+        for (int slot = blockIdx.x; slot < A.nunit; slot += gridDim.x) {
+            const bool first = slot == blockIdx.x;
+            const int u = slot >= off ? slot - off : slot - off + A.nunit;
+            bool ok;
+            if (u >= A.nband) {
+                ok = fused_interior<VTI, GRAD, AE>(A, A.in[u - A.nband], it, first, keep, sm);
+            } else {
+                const BandRef br = A.bands[u];
+                if (br.side >= 2) ok = fused_band<true, VTI, GRAD, AE>(A, br, it, first, keep, sm);
+                else ok = fused_band<false, VTI, GRAD, AE>(A, br, it, first, keep, sm);
+            }
+            if (!ok) return;
+            __syncthreads();   // the next unit's staging, and this step's writes before the arrival
+        }
+        if (threadIdx.x == 0 && it + 1 < A.it1) arrive(A);
     }
 }
 
@@ -996,48 +1146,54 @@ void upload_fused_tables(const float *b1, const float *b2, const float *c2, cons
 }
 
 template <bool VTI, bool GRAD, bool AE>
-static cudaError_t launch_fused_t(const FusedArgs &A, int nin, bool chain, cudaStream_t st)
+static cudaError_t launch_fused_t(const FusedArgs &A, cudaStream_t st)
 {
     constexpr size_t bytes = fused_bytes<VTI, GRAD, AE>();
-    // a kernel attribute of the current device; cheap, and set before every launch so that no state is shared
-    cudaError_t e = cudaFuncSetAttribute(fused_step<VTI, GRAD, AE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    auto kernel = fused_steps<VTI, GRAD, AE>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    int dev = 0, sms = 0, per = 0;
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kFt, bytes);
+    if (e == cudaSuccess) e = cudaMemsetAsync(A.count, 0, sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
+    const long long room = (long long)sms * per;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(A.nxb + A.nzb + nin);
+    cfg.gridDim = dim3((unsigned)(A.nunit < room ? A.nunit : room));
     cfg.blockDim = dim3(kFt);
     cfg.dynamicSmemBytes = bytes;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[0].id = cudaLaunchAttributeCooperative;   // all CTAs resident: they wait for one another
+    at[0].val.cooperative = 1;
     cfg.attrs = at;
-    cfg.numAttrs = chain ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, fused_step<VTI, GRAD, AE>, A);
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, A);
 }
 
-cudaError_t launch_fused_step(int kind, const ShotDev *shots, const TileRef *xb, int nxb, const BandRef *zb, int nzb,
-                              const TileRef *in, int nin, const ModelDev &M, const StepConst &C, int it, int flags,
-                              float dtg, bool chain, cudaStream_t st)
+cudaError_t launch_fused(int kind, const ShotDev *shots, const BandRef *bands, int nband, const TileRef *in, int nin,
+                         const ModelDev &M, const StepConst &C, int it0, int it1, int flags, float dtg, unsigned *count,
+                         int *status, cudaStream_t st)
 {
-    if (nxb + nzb + nin <= 0) return cudaSuccess;
+    if (nband + nin <= 0 || it1 <= it0) return cudaSuccess;
     FusedArgs A;
     A.shots = shots;
-    A.xb = xb;
-    A.zb = zb;
+    A.bands = bands;
     A.in = in;
-    A.nxb = nxb;
-    A.nzb = nzb;
+    A.nband = nband;
+    A.nunit = nband + nin;
     A.M = M;
     A.C = C;
-    A.it = it;
+    A.it0 = it0;
+    A.it1 = it1;
     A.flags = flags;
     A.dtg = dtg;
+    A.count = count;
+    A.status = status;
     const bool g = (flags & F_GRAD) != 0;
-    if (kind == KIND_VTI)
-        return g ? launch_fused_t<true, true, false>(A, nin, chain, st) : launch_fused_t<true, false, false>(A, nin, chain, st);
-    if (kind == KIND_AE)
-        return g ? launch_fused_t<false, true, true>(A, nin, chain, st) : launch_fused_t<false, false, true>(A, nin, chain, st);
-    return g ? launch_fused_t<false, true, false>(A, nin, chain, st) : launch_fused_t<false, false, false>(A, nin, chain, st);
+    if (kind == KIND_VTI) return g ? launch_fused_t<true, true, false>(A, st) : launch_fused_t<true, false, false>(A, st);
+    if (kind == KIND_AE) return g ? launch_fused_t<false, true, true>(A, st) : launch_fused_t<false, false, true>(A, st);
+    return g ? launch_fused_t<false, true, false>(A, st) : launch_fused_t<false, false, false>(A, st);
 }
 
 }  // namespace fwi2d

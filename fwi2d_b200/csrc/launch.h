@@ -24,15 +24,17 @@ void launch_elastic_step(int shape, bool vti, const ShotDev *shots, const TileRe
 bool march_threads_ok(int nth);
 void launch_elastic_march(bool vti, const ShotDev *shots, const MarchRef *units, int nunits, int nth,
                           const ModelDev &M, const StepConst &C, int it, int flags, float dtg, cudaStream_t st);
-// fused.cu: one launch per step over x-band, z-band and interior units; chain:
-// the launch may start beside the previous launch of the stream, which must be
-// a fused step too.  Interior windows of kFusedZ x kFusedX cells start at
-// z = 4 + kFusedZ k (rows of 16-byte multiples) and x = 6 + kFusedX k.
-constexpr int kFusedZ = 32, kFusedX = 16, kFusedBand = 32;
+// fused.cu: the steps [it0, it1) in one cooperative launch over x-band, z-band
+// and interior units.  Interior windows of kFusedZ x kFusedX cells start at
+// z = 4 + kFusedZ k (rows of 16-byte multiples) and x = 6 + kFusedX k; band
+// units have up to kFusedBand cells along their edge.  count: one word of
+// device memory of the plan's own; status: receives step + 1 of a wait that
+// gave up.
+constexpr int kFusedZ = 32, kFusedX = 16, kFusedBand = 28;
 void upload_fused_tables(const float *b1, const float *b2, const float *c2, const float *c1, const float *sc);
-cudaError_t launch_fused_step(int kind, const ShotDev *shots, const TileRef *xb, int nxb, const BandRef *zb, int nzb,
-                              const TileRef *in, int nin, const ModelDev &M, const StepConst &C, int it, int flags,
-                              float dtg, bool chain, cudaStream_t st);
+cudaError_t launch_fused(int kind, const ShotDev *shots, const BandRef *bands, int nband, const TileRef *in, int nin,
+                         const ModelDev &M, const StepConst &C, int it0, int it1, int flags, float dtg, unsigned *count,
+                         int *status, cudaStream_t st);
 // closure sums of the six rows next to both ends of an axis of n samples (stride sn) on `lines` lines (stride sl)
 void launch_closures(const float *f, float *out, int lines, int ld, int n, long long sl, long long sn, cudaStream_t st);
 // top / bottom band kernel (rows clear of the x bands), zband_rows(split)

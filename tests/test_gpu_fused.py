@@ -1,5 +1,5 @@
-"""The fused step (one launch per step over band and interior units, chained by
-programmatic dependent launch) against the oracle and the tile kernel.
+"""The fused time loop (all steps of a pass in one launch of resident CTAs that
+meet between steps) against the oracle and the tile kernel.
 
 Grids sit at the edges of its units: the smallest it takes (40 rows, 16
 columns), one cell either side of a full interior window (32 x 16 from row 4
@@ -96,8 +96,7 @@ def _gradient(kind, shape, prec, every, compensated, nx=150, nz=75, nt=97):
 @pytest.mark.parametrize("prec,every,compensated", [(0, 0, 0), (2, 0, 1), (1, 20, 0), (0, 7, 1)])
 def test_fused_plan_equals_tile_plan(kind, prec, every, compensated):
     """Uneven windows and records, 16-bit snapshots, replayed segments and
-    compensated accumulation: the chain of overlapping launches is broken by
-    other kernels there, and must still see every earlier write."""
+    compensated accumulation: the loop is cut into several launches there."""
     if kind == O.KIND_AE and every:
         pytest.skip("checkpoint-and-recompute is not available for the acoustic-elastic propagator")
     a, ra = _gradient(kind, fused_shape(), prec, every, compensated)
@@ -107,3 +106,30 @@ def test_fused_plan_equals_tile_plan(kind, prec, every, compensated):
         assert fa == fb and np.array_equal(ga, gb)
     for x, y in zip(ra, rb):
         assert np.array_equal(x, y)
+
+
+def test_fused_wait_limit_returns_timeout(monkeypatch):
+    """A meeting of the CTAs that reaches its poll limit (0 here, so at once; the
+    second bound is the ordinary one and nothing is left waiting) is reported,
+    and the context stays usable."""
+    kind, nx, nz, d, nt = O.KIND_ELASTIC, 60, 50, 0.01, 60
+    mc = K.converted(kind, K.model_case(kind, nx, nz, d, seed=11))
+    sl, rl = K.geometry(nx, nz, d, nr=8)
+    pd = K.par_dict(nt=nt, dt=1e-3)
+    src = [K.sources(2, nt, 1e-3)]
+    P = F.Propagator(0)
+    P.set_model(kind, mc, d, d)
+    shot = F.ShotSpec(0, nx, nt, sl[0], sl[1], rl[0], rl[1])
+    monkeypatch.setenv("FWI2D_SPIN_LIMIT", "0")
+    P.set_shots(F.make_params(**pd, tile_shape=fused_shape()), [shot])
+    with pytest.raises(F.Fwi2dError, match="reached its limit"):
+        P.forward(src, store=True)
+    with pytest.raises(F.Fwi2dError):
+        P.adjoint([np.zeros((2, 8, nt), np.float32)])
+    monkeypatch.delenv("FWI2D_SPIN_LIMIT")
+    out = []
+    for shape in (fused_shape(), 3):
+        P.set_shots(F.make_params(**pd, tile_shape=shape), [shot])
+        out.append(P.forward(src, store=False)[0])
+    P.close()
+    assert np.array_equal(out[0], out[1])

@@ -46,7 +46,7 @@ struct MarchRow {
     int pad;
 };
 
-struct ShotDev {
+struct alignas(16) ShotDev {
     int nx, nz, ldz;      // shot grid (nz == model nz)
     int x0;               // first model column of this shot's grid
     int nt;               // time samples of this shot
@@ -111,7 +111,7 @@ struct StepConst {
 
 // Work unit of the tile kernel: a TX x TZ window of one shot grid starting
 // at (wx0, wz0) that writes the cells of [ox0, ox1) x [oz0, oz1).
-struct TileRef {
+struct alignas(16) TileRef {
     int shot, unit;
     int wx0, ox0, ox1;
     int wz0, oz0, oz1;

@@ -49,6 +49,8 @@ __device__ __forceinline__ void cp16(float *dst, const float *src, bool ok)
                  : "memory");
 }
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_wait_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 // ---- packed arithmetic beyond sbp.cuh ---------------------------------------
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
@@ -181,9 +183,15 @@ struct BandLayout {
     static constexpr int F0 = LA + (VTI ? A : 0), F1 = F0 + (GRAD ? A : 0), C0 = F1 + (GRAD ? A : 0);
     static constexpr int C1 = C0 + CL;                     // VTI x bands: closure of (1+2eps)2mu
     static constexpr int ZC = C1 + (VTI ? CL : 0);
-    static constexpr int RED = ZC + 2 * 6 * 8 * 6;
+    // per thread, set once per unit: doubles 1/rho and 1/den (two components), then the floats of Slot
+    static constexpr int SD = ZC + 2 * 6 * 8 * 6;
+    static constexpr int SF = SD + 3 * 2 * kFt;
+    static constexpr int SAT = SF + 8 * kFt;               // [own side, corner][along, across, normal][32]
+    static constexpr int RED = SAT + 6 * 32;
     static constexpr int FLOATS = RED + 8;
+    static_assert(SD % 2 == 0, "doubles");
 };
+enum Slot { SL_TZX = 0, SL_TX, SL_IMP, SL_IMPC, SL_E0, SL_E1, SL_R0, SL_R1 };
 
 template <bool VTI, bool GRAD, bool AE>
 constexpr size_t fused_bytes()
@@ -272,124 +280,137 @@ __device__ __forceinline__ float density_term(float g, double wdt, int k, int la
 }
 
 // ---------------------------------------------------------------------------
-// Interior window.  Thread t owns the z-pair 2 (t & 15) of column t >> 4.
-// Measured on B200, see launch_fused.
+// Interior window.  Thread t owns the z-pair 2 (t & 15) of column t >> 4.  The
+// loads come in two groups: what the first half of the work reads (fields with
+// their halo, coefficients: Lead) and what the second half reads (previous
+// field, density, snapshots, gradient: Own).  While a window is in its second
+// half, the Lead group of the CTA's next window is on its way into the arrays
+// that the first half has left, and while it is in its first half its own Own
+// group is: a CTA's loads overlap its arithmetic without a second buffer.
+// keep: the model arrays are in shared memory from the last step.
 // ---------------------------------------------------------------------------
-// first: the CTA's first unit of this step (it waits for the others there);
-// keep: the unit's model arrays are in shared memory from the last step.
-// Returns false when the wait gave up.
+struct Imaging {
+    int itf, last;
+    bool on;
+};
+template <bool GRAD, bool AE>
+__device__ __forceinline__ Imaging imaging(const ShotDev &S, const StepConst &C, int it)
+{
+    Imaging g;
+    g.itf = GRAD ? (S.nt - 1 - (it + 1)) / C.sub : 0;
+    g.last = S.nt / C.sub;
+    g.on = GRAD && it < S.nt - 1 && (S.nt - 1 - (it + 1)) % C.sub == 0 && (!AE || g.itf != 0);
+    return g;
+}
+
 template <bool VTI, bool GRAD, bool AE>
-__device__ __forceinline__ bool fused_interior(const FusedArgs &A, const TileRef tr, const int it, const bool first,
-                                               const bool keep, float *sm)
+__device__ __forceinline__ void lead_model(const FusedArgs &A, const ShotDev &S, const TileRef &tr, float *sm)
 {
     using L = InLayout<VTI, GRAD, AE>;
-    const ModelDev &M = A.M;
-    const StepConst &C = A.C;
-    const int t = threadIdx.x;
-    const ShotDev *__restrict__ Sp = A.shots + tr.shot;
-    const int nt = Sp->nt, nx = Sp->nx, ldz = Sp->ldz;
-    const int nxz = nx * ldz;
-    const int prec = C.snap_prec;
-    const long long mofs = (long long)Sp->x0 * ldz;   // the model has the shots' pitch
-    const int itf = GRAD ? (nt - 1 - (it + 1)) / C.sub : 0;
-    const bool do_grad = GRAD && it < nt - 1 && ((nt - 1 - (it + 1)) % C.sub == 0) && (!AE || itf != 0);
-    const int last = nt / C.sub;
-    const int xr = t / 10, xq = 4 * (t - 10 * xr);    // staged row and sample of this thread's copies
-    const int orow = (t >> 3) & 15, oq = 4 * (t & 7); // the same for the own-cell arrays (two per pass)
+    const int t = threadIdx.x, xr = t / 10, xq = 4 * (t - 10 * xr);
+    if (t >= (kFx + 4) * 10) return;
+    const int gx = tr.wx0 - 2 + xr, gz = tr.wz0 - 4 + xq;
+    const bool ok = gx < S.nx && gz < S.ldz;
+    const long long o = (long long)S.x0 * S.ldz + (ok ? (long long)gx * S.ldz + gz : 0);   // the model has the shots' pitch
+    const int s = xr * kFs + xq;
+    cp16(sm + L::MU + s, A.M.p1 + o, ok);
+    cp16(sm + L::Q + s, (VTI ? A.M.fxx : A.M.p0) + o, ok);
+    if (VTI) {
+        cp16(sm + L::LB + s, A.M.lbis + o, ok);
+        cp16(sm + L::LC + s, A.M.c13 + o, ok);
+        cp16(sm + L::LA + s, A.M.p0 + o, ok);
+    }
+}
 
-    // ---- what no step writes: coefficients, densities, snapshots
+template <bool VTI, bool GRAD, bool AE>
+__device__ __forceinline__ void lead_fields(const ShotDev &S, const TileRef &tr, int it, float *sm)
+{
+    using L = InLayout<VTI, GRAD, AE>;
+    const int t = threadIdx.x, xr = t / 10, xq = 4 * (t - 10 * xr);
+    if (t >= (kFx + 8) * 10) return;
+    const int x = tr.wx0 - 4 + xr, z = tr.wz0 - 4 + xq;
+    const bool ok = x < S.nx && z < S.ldz;
+    const long long o = ok ? (long long)x * S.ldz + z : 0;
+    const float *curr = S.u[(it + 1) & 1];
+    cp16(sm + L::U0 + xr * kFs + xq, curr + o, ok);
+    cp16(sm + L::U1 + xr * kFs + xq, curr + (long long)S.nx * S.ldz + o, ok);
+}
+
+// density and its reciprocal; snapshots of the imaging condition (no step of this launch writes them)
+template <bool VTI, bool GRAD, bool AE>
+__device__ __forceinline__ void own_model(const FusedArgs &A, const ShotDev &S, const TileRef &tr, int it, bool keep,
+                                          float *sm)
+{
+    using L = InLayout<VTI, GRAD, AE>;
+    const int t = threadIdx.x, h = t >> 7, row = (t >> 3) & 15, q = 4 * (t & 7);
+    const int gx = tr.wx0 + row, gz = tr.wz0 + q;
+    const bool ok = gx < S.nx && gz < S.ldz;
+    const long long nxz = (long long)S.nx * S.ldz, c = ok ? (long long)gx * S.ldz + gz : 0;
+    const long long m = (long long)S.x0 * S.ldz + c;
+    const int s = h * kFo + row * kFz + q;
+    if (!keep) cp16(sm + L::RHO + s, (h ? A.M.irho : A.M.p2) + m, ok);
+    const Imaging g = imaging<GRAD, AE>(S, A.C, it);
+    if (!GRAD || !g.on) return;
+    if (VTI && !keep) {
+        cp16(sm + L::E + s, (h ? A.M.gv2 : A.M.eps) + m, ok);
+        if (t < 128) cp16(sm + L::E + 2 * kFo + s, A.M.gv3 + m, ok);
+    }
+    const int prec = A.C.snap_prec;
+    auto snap = [&](int dst, int k, long long off, bool have) {
+        const long long so = (long long)k * S.snap_slot + off;
+        if (prec == SNAP_FP32 || !have) {
+            cp16(sm + dst, (const float *)S.snap + (have ? so : 0), have);
+        } else {
+            const float inv = 1.f / snap_scale(S.snap_amax, k);
+            *reinterpret_cast<float4 *>(sm + dst) = snap_load4(S.snap, so, prec, inv);
+        }
+    };
+    snap(L::FP0 + s, g.itf + 1, c + h * nxz, ok && g.itf + 1 <= g.last);
+    snap(L::FM0 + s, g.itf - 1, c + h * nxz, ok && g.itf > 0);
+    const int xr = t / 10, xq = 4 * (t - 10 * xr);
     if (t < (kFx + 4) * 10) {
-        const int gx = tr.wx0 - 2 + xr, gz = tr.wz0 - 4 + xq;
-        const bool ok = gx < nx && gz < ldz;
-        const long long o = mofs + (ok ? (long long)gx * ldz + gz : 0);
-        const int s = xr * kFs + xq;
-        if (!keep) {
-            cp16(sm + L::MU + s, M.p1 + o, ok);
-            cp16(sm + L::Q + s, (VTI ? M.fxx : M.p0) + o, ok);
-            if (VTI) {
-                cp16(sm + L::LB + s, M.lbis + o, ok);
-                cp16(sm + L::LC + s, M.c13 + o, ok);
-                cp16(sm + L::LA + s, M.p0 + o, ok);
-            }
-        }
-        if (GRAD && do_grad) {
-            const long long so = (long long)itf * Sp->snap_slot + (ok ? (long long)gx * ldz + gz : 0);
-            if (prec == SNAP_FP32) {
-                cp16(sm + L::F0 + s, (const float *)Sp->snap + so, ok);
-                cp16(sm + L::F1 + s, (const float *)Sp->snap + so + nxz, ok);
-            } else if (ok) {
-                const float inv = 1.f / snap_scale(Sp->snap_amax, itf);
-                *reinterpret_cast<float4 *>(sm + L::F0 + s) = snap_load4(Sp->snap, so, prec, inv);
-                *reinterpret_cast<float4 *>(sm + L::F1 + s) = snap_load4(Sp->snap, so + nxz, prec, inv);
-            }
-        }
+        const int x = tr.wx0 - 2 + xr, z = tr.wz0 - 4 + xq;
+        const bool in = x < S.nx && z < S.ldz;
+        const long long o = in ? (long long)x * S.ldz + z : 0;
+        snap(L::F0 + xr * kFs + xq, g.itf, o, in);
+        snap(L::F1 + xr * kFs + xq, g.itf, o + nxz, in);
     }
-    const int ogx = tr.wx0 + orow, ogz = tr.wz0 + oq;
-    const bool ook = ogx < nx && ogz < ldz;
-    const long long oc = ook ? (long long)ogx * ldz + ogz : 0;
-    const int os = (t >> 7) * kFo + orow * kFz + oq;
-    if (!keep) cp16(sm + L::RHO + os, ((t >> 7) ? M.irho : M.p2) + mofs + oc, ook);
-    if (GRAD && do_grad) {
-        const long long oo = oc + (t >> 7 ? nxz : 0);
-        auto own_snap = [&](int dst, int k, bool have) {
-            const long long so = (long long)k * Sp->snap_slot + oo;
-            if (prec == SNAP_FP32 || !have) {
-                cp16(sm + dst + os, (const float *)Sp->snap + (have ? so : 0), ook && have);
-            } else if (ook) {
-                const float inv = 1.f / snap_scale(Sp->snap_amax, k);
-                *reinterpret_cast<float4 *>(sm + dst + os) = snap_load4(Sp->snap, so, prec, inv);
-            }
-        };
-        own_snap(L::FP0, itf + 1, itf + 1 <= last);
-        own_snap(L::FM0, itf - 1, itf > 0);
-        if (VTI && !keep) {
-            cp16(sm + L::E + os, ((t >> 7) ? M.gv2 : M.eps) + mofs + oc, ook);
-            if (t < 128) cp16(sm + L::E + 2 * kFo + os, M.gv3 + mofs + oc, ook);
-        }
+}
+
+template <bool VTI, bool GRAD, bool AE>
+__device__ __forceinline__ void own_fields(const FusedArgs &A, const ShotDev &S, const TileRef &tr, int it, float *sm)
+{
+    using L = InLayout<VTI, GRAD, AE>;
+    const int t = threadIdx.x, h = t >> 7, row = (t >> 3) & 15, q = 4 * (t & 7);
+    const int gx = tr.wx0 + row, gz = tr.wz0 + q;
+    const bool ok = gx < S.nx && gz < S.ldz;
+    const long long nxz = (long long)S.nx * S.ldz, c = ok ? (long long)gx * S.ldz + gz : 0;
+    const int s = h * kFo + row * kFz + q;
+    cp16(sm + L::PV0 + s, S.u[it & 1] + h * nxz + c, ok);
+    if (GRAD && imaging<GRAD, AE>(S, A.C, it).on) {
+        cp16(sm + L::G0 + s, S.grad + h * nxz + c, ok);
+        if (t < 128) cp16(sm + L::G0 + 2 * kFo + s, S.grad + 2 * nxz + c, ok);
     }
+}
+
+// The window's step, its Lead group present; mid() runs between its halves.
+template <bool VTI, bool GRAD, bool AE, class Mid>
+__device__ __forceinline__ void window_step(const FusedArgs &A, const ShotDev &S, const TileRef &tr, const int it, float *sm,
+                                            Mid mid)
+{
+    using L = InLayout<VTI, GRAD, AE>;
+    const StepConst &C = A.C;
+    const int t = threadIdx.x, nxz = S.nx * S.ldz, ldz = S.ldz, prec = C.snap_prec;
+    const Imaging im = imaging<GRAD, AE>(S, C, it);
+    const int itf = im.itf, last = im.last;
+    const bool do_grad = im.on;
     const int tx = t >> 4, pz = 2 * (t & 15);
     const int gx = tr.wx0 + tx, gz = tr.wz0 + pz;
     const bool ownx = gx >= tr.ox0 && gx < tr.ox1;
     const bool own0 = ownx && gz >= tr.oz0 && gz < tr.oz1, own1 = ownx && gz + 1 >= tr.oz0 && gz + 1 < tr.oz1;
-    float2 tzv = make_float2(0.f, 0.f);
-    float txv = 0.f;
-    if (own0 || own1) {
-        tzv = *reinterpret_cast<const float2 *>(Sp->tz + gz);
-        txv = Sp->tx[gx];
-    }
-    const int e0 = Sp->inj_off[tr.unit], e1 = Sp->inj_off[tr.unit + 1];
-    const float *curr = Sp->u[(it + 1) & 1];
-    float *pn = Sp->u[it & 1];   // prev in, next out
-
-    if (first && !meet(A, it)) {
-        cp_wait();
-        return false;
-    }
-    if (it >= nt - 1) {
-        cp_wait();
-        return true;
-    }
-
-    // ---- fields and, in the adjoint, the gradient
-    if (t < (kFx + 8) * 10) {
-        const int x = tr.wx0 - 4 + xr, z = tr.wz0 - 4 + xq;
-        const bool ok = x < nx && z < ldz;
-        const long long o = ok ? (long long)x * ldz + z : 0;
-        const int s = xr * kFs + xq;
-        cp16(sm + L::U0 + s, curr + o, ok);
-        cp16(sm + L::U1 + s, curr + nxz + o, ok);
-    }
-    cp16(sm + L::PV0 + os, pn + (t >> 7 ? nxz : 0) + oc, ook);
-    if (GRAD && do_grad) {
-        cp16(sm + L::G0 + os, Sp->grad + (t >> 7 ? nxz : 0) + oc, ook);
-        if (t < 128) cp16(sm + L::G0 + 2 * kFo + os, Sp->grad + 2 * (long long)nxz + oc, ook);
-    }
-    cp_wait();
-    __syncthreads();
-
     const float *U0 = sm + L::U0 + 2 * kFs, *U1 = sm + L::U1 + 2 * kFs;   // indexed as the 2-halo arrays
     const float *MU = sm + L::MU, *Q = sm + L::Q;
-    float *P = sm + L::P, *R = sm + L::R, *S = sm + L::S, *P1 = sm + L::P1;
+    float *P = sm + L::P, *R = sm + L::R, *T = sm + L::S, *P1 = sm + L::P1;
 
     // products of the mixed terms at one pair from its strains
     auto mixed = [&](int i, float2 exx, float2 ezz) {
@@ -420,7 +441,7 @@ __device__ __forceinline__ bool fused_interior(const FusedArgs &A, const TileRef
         if (side)
             *reinterpret_cast<float2 *>(R + i) = mul2(der_z(ld2(U0, i - 2), ld2(U0, i), ld2(U0, i + 2), C.sdz), m);
         else
-            *reinterpret_cast<float2 *>(S + i) =
+            *reinterpret_cast<float2 *>(T + i) =
                 mul2(der_x(ld2(U1, i - 2 * kFs), ld2(U1, i - kFs), ld2(U1, i + kFs), ld2(U1, i + 2 * kFs), C.sdx), m);
     }
 
@@ -435,7 +456,7 @@ __device__ __forceinline__ bool fused_interior(const FusedArgs &A, const TileRef
         const float2 m00 = ld2(MU, i);
         exx = der_x(am2, am1, ap1, ap2, C.sdx);
         ezx = der_x(bm2, bm1, bp1, bp2, C.sdx);
-        *reinterpret_cast<float2 *>(S + i) = mul2(ezx, m00);
+        *reinterpret_cast<float2 *>(T + i) = mul2(ezx, m00);
         const Brk2 bx = brackets2(ld2(MU, i - 2 * kFs), ld2(MU, i - kFs), m00, ld2(MU, i + kFs), ld2(MU, i + 2 * kFs));
         if (VTI) {
             const Brk2 bq = brackets2(ld2(Q, i - 2 * kFs), ld2(Q, i - kFs), ld2(Q, i), ld2(Q, i + kFs), ld2(Q, i + 2 * kFs));
@@ -457,7 +478,24 @@ __device__ __forceinline__ bool fused_interior(const FusedArgs &A, const TileRef
         n1 = add2(mul2(bc2(C.inv_d2z), sum_z(twice2(bz), blo, b00, bhi)), n1);
         n0 = add2(n0, mul2(bc2(C.inv_d2z), sum_z(bz, alo, a00, ahi)));
     }
+    // receivers (forward): one thread per receiver of this window
+    if (!GRAD && (A.flags & F_EXTRACT)) {
+        const int r0 = S.ext_off[tr.unit], r1 = S.ext_off[tr.unit + 1];
+        for (int e = r0 + t; e < r1; e += kFt) {
+            const ExtEntry &E = S.ext[e];
+            const float *U = sm + (E.comp == 0 ? L::U0 : L::U1) + (E.gx0 - tr.wx0 + 4) * kFs + (E.gz0 - tr.wz0 + 4);
+            float o = 0.f;
+#pragma unroll
+            for (int a = 0; a < 3; a++)
+#pragma unroll
+                for (int b = 0; b < 3; b++) o += E.w[a * 3 + b] * U[a * kFs + b];
+            S.rcv[(long long)it * S.nrcv + E.row] = o;
+        }
+    }
+    const float2 a00 = ld2(U0, i), b00 = ld2(U1, i);
+    cp_wait();
     __syncthreads();
+    mid();   // U, the coefficients and their loads' addresses are free for the next window
 
     // ---- mixed terms
     auto along_x = [&](const float *p, float s) {
@@ -471,15 +509,15 @@ __device__ __forceinline__ bool fused_interior(const FusedArgs &A, const TileRef
         n1 = add2(n1, along_z(P, C.adz));
     }
     n1 = add2(n1, along_x(R, C.adx));
-    n0 = add2(n0, along_z(S, C.adz));
+    n0 = add2(n0, along_z(T, C.adz));
 
-    const float2 a00 = ld2(U0, i), b00 = ld2(U1, i);
     const int cell = gx * ldz + gz;
     // sources, cell by cell in the reference's order
+    const int e0 = S.inj_off[tr.unit], e1 = S.inj_off[tr.unit + 1];
     if (e0 < e1) {
-        const float *srcrow = Sp->src + (long long)it * Sp->nsrc;
+        const float *srcrow = S.src + (long long)it * S.nsrc;
         for (int e = e0; e < e1; e++) {
-            const InjEntry &E = Sp->inj[e];
+            const InjEntry &E = S.inj[e];
             if (E.gx == gx && (E.gz == gz || E.gz == gz + 1)) {
                 const float v = E.mt ? (E.wa * srcrow[E.ia] - E.wb * srcrow[E.ib]) : E.wa * srcrow[E.ia];
                 if (E.comp == 0) {
@@ -492,19 +530,12 @@ __device__ __forceinline__ bool fused_interior(const FusedArgs &A, const TileRef
             }
         }
     }
-    // receivers (forward): one thread per receiver of this window
-    if (!GRAD && (A.flags & F_EXTRACT)) {
-        const int r0 = Sp->ext_off[tr.unit], r1 = Sp->ext_off[tr.unit + 1];
-        for (int e = r0 + t; e < r1; e += kFt) {
-            const ExtEntry &E = Sp->ext[e];
-            const float *U = sm + (E.comp == 0 ? L::U0 : L::U1) + (E.gx0 - tr.wx0 + 4) * kFs + (E.gz0 - tr.wz0 + 4);
-            float o = 0.f;
-#pragma unroll
-            for (int a = 0; a < 3; a++)
-#pragma unroll
-                for (int b = 0; b < 3; b++) o += E.w[a * 3 + b] * U[a * kFs + b];
-            Sp->rcv[(long long)it * Sp->nrcv + E.row] = o;
-        }
+    float *pn = S.u[it & 1];   // prev in, next out
+    float2 tzv = make_float2(0.f, 0.f);
+    float txv = 0.f;
+    if (own0 || own1) {
+        tzv = *reinterpret_cast<const float2 *>(S.tz + gz);
+        txv = S.tx[gx];
     }
     // leapfrog: dt^2 n / rho + 2 curr - prev, tapered; prev takes its second taper here
     const int oi = tx * kFz + pz;
@@ -534,19 +565,19 @@ __device__ __forceinline__ bool fused_interior(const FusedArgs &A, const TileRef
     }
     if (!GRAD && (A.flags & F_STORE) && it % C.sub == 0) {
         const int slot = it / C.sub;
-        const long long o = (long long)slot * Sp->snap_slot + cell;
+        const long long o = (long long)slot * S.snap_slot + cell;
         if (prec == SNAP_FP32 && own0 && own1) {
-            *reinterpret_cast<float2 *>((float *)Sp->snap + o) = a00;
-            *reinterpret_cast<float2 *>((float *)Sp->snap + o + nxz) = b00;
+            *reinterpret_cast<float2 *>((float *)S.snap + o) = a00;
+            *reinterpret_cast<float2 *>((float *)S.snap + o + nxz) = b00;
         } else {
-            const float sc = prec == SNAP_FP32 ? 1.f : snap_scale(Sp->snap_amax, slot);
+            const float sc = prec == SNAP_FP32 ? 1.f : snap_scale(S.snap_amax, slot);
             if (own0) {
-                snap_store(Sp->snap, o, prec, a00.x, sc);
-                snap_store(Sp->snap, o + nxz, prec, b00.x, sc);
+                snap_store(S.snap, o, prec, a00.x, sc);
+                snap_store(S.snap, o + nxz, prec, b00.x, sc);
             }
             if (own1) {
-                snap_store(Sp->snap, o + 1, prec, a00.y, sc);
-                snap_store(Sp->snap, o + nxz + 1, prec, b00.y, sc);
+                snap_store(S.snap, o + 1, prec, a00.y, sc);
+                snap_store(S.snap, o + nxz + 1, prec, b00.y, sc);
             }
         }
     }
@@ -573,7 +604,7 @@ __device__ __forceinline__ bool fused_interior(const FusedArgs &A, const TileRef
                       mul2(v3, cross));
         }
         float2 g0 = ld2(sm + L::G0, oi), g1 = ld2(sm + L::G0 + kFo, oi), g2 = ld2(sm + L::G0 + 2 * kFo, oi);
-        const float gw = Sp->gwt[itf];
+        const float gw = S.gwt[itf];
         const double wdt = (double)gw * 1.0 / (double)A.dtg;
         if (itf > 0) {
             const float2 gd = bc2(gw * A.dtg);
@@ -597,7 +628,7 @@ __device__ __forceinline__ bool fused_interior(const FusedArgs &A, const TileRef
         const float2 fm0 = ld2(sm + L::FM0, oi), fm1 = ld2(sm + L::FM0 + kFo, oi);
         g2.x = density_term(g2.x, wdt, itf, last, n0.x, n1.x, f0.x, f1.x, fp0.x, fp1.x, fm0.x, fm1.x);
         g2.y = density_term(g2.y, wdt, itf, last, n0.y, n1.y, f0.y, f1.y, fp0.y, fp1.y, fm0.y, fm1.y);
-        float *G = Sp->grad + cell;
+        float *G = S.grad + cell;
         if (own0 && own1) {
             *reinterpret_cast<float2 *>(G) = g0;
             *reinterpret_cast<float2 *>(G + nxz) = g1;
@@ -616,9 +647,8 @@ __device__ __forceinline__ bool fused_interior(const FusedArgs &A, const TileRef
         float m = 0.f;
         if (own0) m = fmaxf(fabsf(n0.x), fabsf(n1.x));
         if (own1) m = fmaxf(m, fmaxf(fabsf(n0.y), fabsf(n1.y)));
-        block_amax(m, sm + L::RED, Sp->snap_amax + (it + 1) / C.sub);
+        block_amax(m, sm + L::RED, S.snap_amax + (it + 1) / C.sub);
     }
-    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -632,6 +662,10 @@ __device__ __forceinline__ bool fused_interior(const FusedArgs &A, const TileRef
 // closures' rows do not diverge.  The coefficient sums of the second
 // derivative's closure depend on the model only and come ready from
 // k_closures: 8 products and quotients instead of 8 x 16 operations.
+// One such CTA sets the time of a step on small plans, and its time is one
+// warp's chain of instructions: so the SAT terms of the edge row, which need
+// the fields only, are formed by warps 6 and 7 beside the rows' derivatives,
+// and whatever depends on the model alone is set up once per unit (keep).
 // ---------------------------------------------------------------------------
 template <bool XB, bool VTI, bool GRAD, bool AE>
 __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br, const int it, const bool first,
@@ -656,36 +690,52 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
     // along the edge: samples that exist (z bands: within the columns clear of the x bands and their halo)
     const int glo = XB ? 0 : t0 - 4, ghi = XB ? nz : t1 + 4;
 
-    // sample i of a staged array: its shared index, its cell, and whether it exists
-    auto sample = [&](int i, int &s, int &o) {
+    // the two staged samples of this thread: shared index, cell, and whether they exist
+    int s_[2], o_[2];
+    bool in_[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int i = t + h * kFt;
         int c, tt;
         if (XB) { c = i / kBt; tt = i - c * kBt; }
         else { tt = i / kFb; c = i - tt * kFb; }
         const int g = t0 - 4 + tt, gn = far ? nn - 1 - c : c;
-        s = c * kFs + tt;
-        o = XB ? gn * ldz + g : g * ldz + gn;
-        return g >= glo && g < ghi;
-    };
-    for (int i = t; i < kFb * kBt; i += kFt) {
-        int s, o;
-        const bool in = sample(i, s, o);
-        if (!keep) {
-            sm[L::MU + s] = in ? M.p1[mofs + o] : 0.f;
-            sm[L::Q + s] = in ? (VTI ? M.fxx : M.p0)[mofs + o] : 0.f;
-            if (VTI) {
-                sm[L::LB + s] = in ? M.lbis[mofs + o] : 0.f;
-                sm[L::LC + s] = in ? M.c13[mofs + o] : 0.f;
-                sm[L::LA + s] = in ? M.p0[mofs + o] : 0.f;
-            }
-        }
-        if (GRAD && do_grad) {
-            const long long so = (long long)itf * Sp->snap_slot + o;
-            const float inv = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, itf);
-            sm[L::F0 + s] = in ? snap_load(Sp->snap, so, prec, inv) : 0.f;
-            sm[L::F1 + s] = in ? snap_load(Sp->snap, so + nxz, prec, inv) : 0.f;
-        }
+        const bool slot = i < kFb * kBt;
+        in_[h] = slot && g >= glo && g < ghi;
+        s_[h] = slot ? c * kFs + tt : -1;
+        o_[h] = in_[h] ? (XB ? gn * ldz + g : g * ldz + gn) : 0;
     }
+    static_assert(kFb * kBt <= 2 * kFt, "two samples per thread");
+    auto stage = [&](int dst, const float *src) {
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+            if (s_[h] >= 0) sm[dst + s_[h]] = in_[h] ? src[o_[h]] : 0.f;
+    };
+
+    // this thread's cell: row `warp` from the edge, tangential t0 + lane - 2; warps 6
+    // and 7 take the edge row (its SAT terms along and across the edge)
+    const int row = warp < 6 ? warp : 0;
+    const int gt = t0 + lane - 2, gn = far ? nn - 1 - row : row;
+    const int gx = XB ? gn : gt, gz = XB ? gt : gn;
+    const bool mine = lane >= 2 && gt < t1, owned = mine && warp < 6;
+    const int cell = mine ? gx * ldz + gz : 0;
+    const long long mcell = mofs + cell;
+    // x bands: the corner cells' rows along the top or bottom edge, one per lane of warps 6 and 7
+    const bool top_here = XB && t0 == 0, bot_here = XB && t1 == nz;
+    const bool cside = warp >= 6 && lane < 6 && (top_here || bot_here);
+    const int cgx = far ? nx - 1 - lane : lane, cgz = top_here ? 0 : nz - 1;
+    const int ccell = cside ? cgx * ldz + cgz : 0;
+    double *SD = reinterpret_cast<double *>(sm + L::SD) + t;
+    float *SF = sm + L::SF + t;
+
     if (!keep) {
+        stage(L::MU, M.p1 + mofs);
+        stage(L::Q, (VTI ? M.fxx : M.p0) + mofs);
+        if (VTI) {
+            stage(L::LB, M.lbis + mofs);
+            stage(L::LC, M.c13 + mofs);
+            stage(L::LA, M.p0 + mofs);
+        }
         // closure coefficients [row][sample][tangential] of the owned cells
         const int ld = XB ? ldz : M.nx, base = (XB ? 0 : Sp->x0) + t0;
         for (int i = t; i < L::CL; i += kFt) {
@@ -700,74 +750,110 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
                 const int k = i / 6, c = i - 6 * k;
                 sm[L::ZC + i] = M.zclos[(long long)k * M.nx + Sp->x0 + (far ? nx - 1 - c : c)];
             }
-    }
-
-    // this thread's cell: row `warp` from the edge, tangential t0 + lane - 2
-    const int gt = t0 + lane - 2, gn = far ? nn - 1 - warp : warp;
-    const int gx = XB ? gn : gt, gz = XB ? gt : gn;
-    const bool owned = warp < 6 && lane >= 2 && gt < t1;
-    const int cell = owned ? gx * ldz + gz : 0;
-    const long long mcell = mofs + cell;
-    float rho = 1.f, tzv = 0.f, txv = 0.f, fp0 = 0.f, fp1 = 0.f, fm0 = 0.f, fm1 = 0.f;
-    if (owned) {
-        rho = M.p2[mcell];
-        tzv = Sp->tz[gz];
-        txv = Sp->tx[gx];
-        if (GRAD && do_grad) {
-            if (itf + 1 <= last) {
-                const float inv = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, itf + 1);
-                const long long o = (long long)(itf + 1) * Sp->snap_slot + cell;
-                fp0 = snap_load(Sp->snap, o, prec, inv);
-                fp1 = snap_load(Sp->snap, o + nxz, prec, inv);
+        // impedance of a side's SAT at model cell m: warp 6 the shear one, warp 7 the compressional one
+        auto impedance = [&](long long m, bool zside) {
+            const float mu = M.p1[m], rho = M.p2[m];
+            if (warp == 6) return 0.5f * sqrtf(mu * rho);
+            const float l2m = M.p0[m] + 2 * mu;
+            return VTI && !zside ? 0.5f * sqrtf((1 + 2 * M.eps[m]) * l2m * rho) : 0.5f * sqrtf(l2m * rho);
+        };
+        float tzv = 0.f, txv = 0.f;
+        int e0 = 0, e1 = 0, r0 = 0, r1 = 0;
+        if (mine) {
+            SD[0] = 1.0 / (double)M.p2[mcell];
+            if (warp >= 6) SF[SL_IMP * kFt] = impedance(mcell, !XB);
+            if (gz == 0 || gz == nz - 1 || gx == 0 || gx == nx - 1) {
+                const int per = 2 * nx + 2 * nz;
+                const int kk = gz == 0 ? gx : gz == nz - 1 ? nx + gx : gx == 0 ? 2 * nx + gz : 2 * nx + nz + gz;
+                SD[kFt] = 1.0 / (double)Sp->den[kk];
+                SD[2 * kFt] = 1.0 / (double)Sp->den[per + kk];
             }
-            if (itf > 0) {
-                const float inv = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, itf - 1);
-                const long long o = (long long)(itf - 1) * Sp->snap_slot + cell;
-                fm0 = snap_load(Sp->snap, o, prec, inv);
-                fm1 = snap_load(Sp->snap, o + nxz, prec, inv);
+            tzv = Sp->tz[gz];
+            txv = Sp->tx[gx];
+            if (!XB) {
+                const MarchRow R = Sp->mrow[br.roff + gt - t0];
+                e0 = R.e0;
+                e1 = R.e1;
+                r0 = R.r0;
+                r1 = warp == 0 ? R.r1 : R.r0;
             }
         }
+        if (XB) {
+            e0 = Sp->inj_off[br.unit];
+            e1 = Sp->inj_off[br.unit + 1];
+            r0 = Sp->ext_off[br.unit] + t;
+            r1 = Sp->ext_off[br.unit + 1];
+        }
+        if (cside) SF[SL_IMPC * kFt] = impedance(mofs + ccell, true);
+        SF[SL_TZX * kFt] = tzv;
+        SF[SL_TX * kFt] = txv;
+        SF[SL_E0 * kFt] = __int_as_float(e0);
+        SF[SL_E1 * kFt] = __int_as_float(e1);
+        SF[SL_R0 * kFt] = __int_as_float(r0);
+        SF[SL_R1 * kFt] = __int_as_float(r1);
     }
-    const double irho = 1.0 / (double)rho;
+    float fp0 = 0.f, fp1 = 0.f, fm0 = 0.f, fm1 = 0.f;
+    if (GRAD && do_grad) {
+        // loads first: they come from HBM
+        const long long so = (long long)itf * Sp->snap_slot;
+        float a_[2], b_[2];
+        const float inv = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, itf);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            a_[h] = in_[h] ? snap_load(Sp->snap, so + o_[h], prec, inv) : 0.f;
+            b_[h] = in_[h] ? snap_load(Sp->snap, so + o_[h] + nxz, prec, inv) : 0.f;
+        }
+        if (owned && itf + 1 <= last) {
+            const float ip = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, itf + 1);
+            fp0 = snap_load(Sp->snap, so + Sp->snap_slot + cell, prec, ip);
+            fp1 = snap_load(Sp->snap, so + Sp->snap_slot + cell + nxz, prec, ip);
+        }
+        if (owned && itf > 0) {
+            const float im = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, itf - 1);
+            fm0 = snap_load(Sp->snap, so - Sp->snap_slot + cell, prec, im);
+            fm1 = snap_load(Sp->snap, so - Sp->snap_slot + cell + nxz, prec, im);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+            if (s_[h] >= 0) {
+                sm[L::F0 + s_[h]] = a_[h];
+                sm[L::F1 + s_[h]] = b_[h];
+            }
+    }
     const bool edge = owned && (gz == 0 || gz == nz - 1 || gx == 0 || gx == nx - 1);
-    // entries of this unit: x bands its own list, z bands one record per column
-    int e0, e1, r0, r1, rstep;
-    if (XB) {
-        e0 = Sp->inj_off[br.unit];
-        e1 = Sp->inj_off[br.unit + 1];
-        r0 = Sp->ext_off[br.unit] + t;
-        r1 = Sp->ext_off[br.unit + 1];
-        rstep = kFt;
-    } else {
-        MarchRow R = {};
-        if (lane >= 2 && gt < t1) R = Sp->mrow[br.roff + gt - t0];
-        e0 = R.e0;
-        e1 = R.e1;
-        r0 = R.r0;
-        r1 = warp == 0 ? R.r1 : R.r0;
-        rstep = 1;
-    }
     const float *curr = Sp->u[(it + 1) & 1];
     float *pn = Sp->u[it & 1];
 
     if (first && !meet(A, it)) return false;
     if (it >= nt - 1) return true;
 
-    for (int i = t; i < kFb * kBt; i += kFt) {
-        int s, o;
-        const bool in = sample(i, s, o);
-        sm[L::UN + s] = in ? __ldcg(curr + o + (XB ? 0 : nxz)) : 0.f;
-        sm[L::UT + s] = in ? __ldcg(curr + o + (XB ? nxz : 0)) : 0.f;
-    }
-    float p0 = 0.f, p1 = 0.f, g0 = 0.f, g1 = 0.f, g2 = 0.f;
-    if (owned) {
-        p0 = __ldcg(pn + cell);
-        p1 = __ldcg(pn + nxz + cell);
-        if (GRAD && do_grad) {
+    float p0 = 0.f, p1 = 0.f, g0 = 0.f, g1 = 0.f, g2 = 0.f, c0 = 0.f, c1 = 0.f;
+    {
+        float a_[2], b_[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            a_[h] = in_[h] ? __ldcg(curr + o_[h] + (XB ? 0 : nxz)) : 0.f;
+            b_[h] = in_[h] ? __ldcg(curr + o_[h] + (XB ? nxz : 0)) : 0.f;
+        }
+        if (mine) {
+            p0 = __ldcg(pn + cell);
+            p1 = __ldcg(pn + nxz + cell);
+        }
+        if (cside) {
+            c0 = __ldcg(pn + ccell);
+            c1 = __ldcg(pn + nxz + ccell);
+        }
+        if (GRAD && do_grad && owned) {
             g0 = __ldcg(Sp->grad + cell);
             g1 = __ldcg(Sp->grad + nxz + cell);
             g2 = __ldcg(Sp->grad + 2 * (long long)nxz + cell);
         }
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+            if (s_[h] >= 0) {
+                sm[L::UN + s_[h]] = a_[h];
+                sm[L::UT + s_[h]] = b_[h];
+            }
     }
     __syncthreads();
 
@@ -855,7 +941,8 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
 
     // receivers of this unit (forward)
     if (!GRAD && (A.flags & F_EXTRACT)) {
-        for (int e = r0; e < r1; e += rstep) {
+        const int r1 = __float_as_int(SF[SL_R1 * kFt]);
+        for (int e = __float_as_int(SF[SL_R0 * kFt]); e < r1; e += XB ? kFt : 1) {
             const ExtEntry &E = Sp->ext[e];
             const bool nc = XB ? E.comp == 0 : E.comp == 1;
             const int gn0 = XB ? E.gx0 : E.gz0, gt0 = XB ? E.gz0 : E.gx0;
@@ -870,16 +957,91 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
         }
     }
 
-    float amax = 0.f;
+    const float tzv = SF[SL_TZX * kFt], txv = SF[SL_TX * kFt];
+    if (it > 0) {
+        p0 = p0 * tzv * txv;
+        p1 = p1 * tzv * txv;
+    }
+    float pn_ = XB ? p0 : p1, pt_ = XB ? p1 : p0;   // previous values
+    if (warp >= 6) {
+        // SAT terms (spatial_operators.hpp:160-822) of one side at one cell, scaled as they are subtracted:
+        // warp 6 the term of the component along the side, warp 7 that of the component across it and its
+        // normal-derivative term.  v: the component across, w: along; at: the cell's sample; row k of the band;
+        // own: the side is the band's edge, else the top or bottom edge at a corner.
+        auto sat_terms = [&](bool own, int side, int at, int k, float prev, float imp, float *out) {
+            const int bc = side == 0 ? C.bc[0] : side == 1 ? C.bc[1] : side == 2 ? C.bc[2] : C.bc[3];
+            const bool zside = side < 2, ab = bc == 2;
+            const float *v = sm + (own ? L::UN : L::UT) + at, *w = sm + (own ? L::UT : L::UN) + at;
+            const float *q = warp == 6 ? v : w;   // the derivative along the side is that of the other component
+            const int in = own ? kFs : (side & 1 ? -1 : 1);
+            const double ia = own ? idt : idn, ic = own ? idn : idt;
+            const float mu = sm[L::MU + at], lam = VTI ? sm[L::LA + at] : sm[L::Q + at];
+            float s = 0.f;
+            if (own) {
+                const int g = XB ? t0 - 4 + at : 6;   // position along z (edge row: `at` is the tangential sample)
+                if (XB && (g < 4 || g >= nz - 4)) {
+                    const bool f = g >= 4;
+                    const int r = f ? nz - 1 - g : g, o = f ? r : -r, d = f ? -1 : 1;
+                    const float e = f ? -1.f : 1.f;
+#pragma unroll
+                    for (int j = 0; j < 6; j++) s += (e * kB1[r][j]) * q[o + j * d];
+                } else {
+                    s += kC1[0] * (q[1] - q[-1]);
+                    s += kC1[1] * (q[2] - q[-2]);
+                }
+            } else {
+                if (k >= 4) {
+                    s += kC1[0] * (q[kFs] - q[-kFs]);
+                    s += kC1[1] * (q[2 * kFs] - q[-2 * kFs]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 6; j++) s += kB1[k][j] * q[(j - k) * kFs];
+                }
+                s = sg * s;
+            }
+            const float s2 = side & 1 ? 1.f : -1.f, sat = zside ? C.sat_z : C.sat_x;
+            const float *u = warp == 6 ? w : v;   // the component itself: one-sided derivative into the domain
+            float nv = 0.f, nd = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; j++) nv += kSC[j] * u[j * in];
+#pragma unroll
+            for (int j = 0; j < 6; j++) nd -= kB1[0][j] * u[j * in];
+            const float c13 = VTI ? sm[L::LC + at] : lam, fxx = VTI ? sm[L::Q + at] : 2 * mu;
+            const float ca = warp == 6 ? mu : c13, cn = warp == 6 ? mu : (zside ? 2 * mu : fxx);
+            float tt = div64((s2 * ca) * s, ia) + div64(cn * nv, ic);
+            if (ab) tt = tt - div64(imp * prev, C.idt64);
+            if (warp == 6) {
+                out[0] = sat * tt;
+            } else {
+                out[32] = sat * tt;
+                out[64] = (zside ? C.nsat_z : C.nsat_x) * (zside || !VTI ? lam : sm[L::LB + at]) * nd;
+            }
+        };
+        if (mine) {
+            const int bc = br.side == 0 ? C.bc[0] : br.side == 1 ? C.bc[1] : br.side == 2 ? C.bc[2] : C.bc[3];
+            if (bc == 1 || bc == 2)
+                sat_terms(true, br.side, lane + 2, 0, warp == 6 ? pt_ : pn_, SF[SL_IMP * kFt], sm + L::SAT + lane);
+        }
+        if (cside) {
+            const float ctz = Sp->tz[cgz], ctx = Sp->tx[cgx];
+            float c = warp == 6 ? c0 : c1;   // along the top or bottom edge: ux, across: uz
+            if (it > 0) c = c * ctz * ctx;
+            const int bc = top_here ? C.bc[0] : C.bc[1];
+            if (bc == 1 || bc == 2)
+                sat_terms(false, top_here ? 0 : 1, lane * kFs + cgz - t0 + 4, lane, c, SF[SL_IMPC * kFt],
+                          sm + L::SAT + 96 + lane);
+        }
+    }
+
+    float amax = 0.f, an = 0.f, at = 0.f, un = 0.f, ut = 0.f;
     if (owned) {
-        const float un = sm[L::UN + i], ut = sm[L::UT + i], mu = sm[L::MU + i];
-        float pn_ = XB ? p0 : p1, pt_ = XB ? p1 : p0;   // previous values
+        un = sm[L::UN + i];
+        ut = sm[L::UT + i];
         // second derivatives: the closure rows across the edge, the interior form along it
         // (x bands: the closure again near the corners); acc += val u / d^2, sample by sample
         const float *CL = sm + L::C0 + warp * 8 * kFusedBand + lane - 2;
         const float *CQ = sm + (VTI && XB ? L::C1 : L::C0) + warp * 8 * kFusedBand + lane - 2;
         const float *UN = sm + L::UN + lane + 2, *UT = sm + L::UT + lane + 2;
-        float an = 0.f, at = 0.f;
 #pragma unroll
         for (int j = 0; j < 8; j++)
             an += div64((VTI && XB ? CQ[j * kFusedBand] : 2.f * CL[j * kFusedBand]) * UN[j * kFs], idn2);
@@ -920,9 +1082,11 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
             at += mdern(L::DT, L::MU);
         }
         // sources of this cell, in the reference's order
-        if (e0 < e1) {
+        const int e1 = __float_as_int(SF[SL_E1 * kFt]);
+        int e = __float_as_int(SF[SL_E0 * kFt]);
+        if (e < e1) {
             const float *srcrow = Sp->src + (long long)it * Sp->nsrc;
-            for (int e = e0; e < e1; e++) {
+            for (; e < e1; e++) {
                 const InjEntry &E = Sp->inj[e];
                 if (E.gx != gx || E.gz != gz) continue;
                 const float v = E.mt ? (E.wa * srcrow[E.ia] - E.wb * srcrow[E.ib]) : E.wa * srcrow[E.ia];
@@ -930,94 +1094,40 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
                 else at += v;
             }
         }
-        if (it > 0) {
-            pn_ = pn_ * tzv * txv;
-            pt_ = pt_ * tzv * txv;
-        }
+    }
+    __syncthreads();   // the SAT terms of warps 6 and 7
 
-        // SAT closures (spatial_operators.hpp:160-822), in the reference's side order
-        // (the fluid interface of the acoustic-elastic propagator, its top edge, last)
-        if (edge) {
-            const float lam = VTI ? sm[L::LA + i] : sm[L::Q + i], c13 = VTI ? sm[L::LC + i] : lam;
-            const float fxx = VTI ? sm[L::Q + i] : 2 * mu, lamx = VTI ? sm[L::LB + i] : lam;
-            const float imp_s = 0.5f * sqrtf(mu * rho);
-            const float imp_p = 0.5f * sqrtf((lam + 2 * mu) * rho);
-            const float imp_px = VTI ? 0.5f * sqrtf((1 + 2 * M.eps[mcell]) * (lam + 2 * mu) * rho) : imp_p;
-#pragma unroll 1
-            for (int q = 0; q < 4; q++) {
-                const int side = AE ? (q + 1) & 3 : q;
-                const int bc = side == 0 ? C.bc[0] : side == 1 ? C.bc[1] : side == 2 ? C.bc[2] : C.bc[3];
-                const bool zside = side < 2;
-                if ((bc != 1 && bc != 2) || (zside ? gz : gx) != (side & 1 ? (zside ? nz : nx) - 1 : 0)) continue;
-                const bool mine = XB ? !zside : zside;   // the band's own edge, or the other one at a corner
-                // u across the side, u along it; derivative sums along the side (tsum) and into the domain
-                const float *v = sm + (mine ? L::UN : L::UT) + i, *w = sm + (mine ? L::UT : L::UN) + i;
-                const int in = mine ? kFs : zs;          // samples count from the edge / the corner
-                const float s2 = side & 1 ? 1.f : -1.f;
-                float sv, sw;   // tsum of v and w along the side
-                if (mine) {
-                    if (XB && zr < 4) {
-                        sv = zsum(v);
-                        sw = zsum(w);
-                    } else {
-                        sv = 0.f + kC1[0] * (v[1] - v[-1]);
-                        sv += kC1[1] * (v[2] - v[-2]);
-                        sw = 0.f + kC1[0] * (w[1] - w[-1]);
-                        sw += kC1[1] * (w[2] - w[-2]);
-                    }
-                } else {
-                    // along the band's normal, at row `warp`
-                    if (warp >= 4) {
-                        sv = 0.f + kC1[0] * (v[kFs] - v[-kFs]);
-                        sv += kC1[1] * (v[2 * kFs] - v[-2 * kFs]);
-                        sw = 0.f + kC1[0] * (w[kFs] - w[-kFs]);
-                        sw += kC1[1] * (w[2 * kFs] - w[-2 * kFs]);
-                    } else {
-                        sv = sw = 0.f;
-#pragma unroll
-                        for (int k = 0; k < 6; k++) {
-                            sv += kB1[warp][k] * v[(k - warp) * kFs];
-                            sw += kB1[warp][k] * w[(k - warp) * kFs];
-                        }
-                    }
-                    sv = sg * sv;
-                    sw = sg * sw;
-                }
-                float nv = 0.f, nw = 0.f, nd = 0.f;   // S.v, S.w and -(D v)_0 (sbp.cuh nsum, ndsum)
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    nv += kSC[k] * v[k * in];
-                    nw += kSC[k] * w[k * in];
-                }
-#pragma unroll
-                for (int k = 0; k < 6; k++) nd -= kB1[0][k] * v[k * in];
-                const double ia = mine ? idt : idn, ic = mine ? idn : idt;   // 1 / spacing along and across the side
-                const float sat = zside ? C.sat_z : C.sat_x;
-                float along = mine ? at : an, across = mine ? an : at;
-                float tt = div64((s2 * mu) * sv, ia) + div64(mu * nw, ic);
-                if (bc == 2) tt = tt - div64(imp_s * (mine ? pt_ : pn_), C.idt64);
-                along = along - sat * tt;
-                tt = div64((s2 * c13) * sw, ia) + div64((zside ? 2 * mu : fxx) * nv, ic);
-                if (bc == 2) tt = tt - div64((zside ? imp_p : imp_px) * (mine ? pn_ : pt_), C.idt64);
-                across = across - sat * tt;
-                across = across - (zside ? C.nsat_z : C.nsat_x) * (zside ? lam : lamx) * nd;
-                an = mine ? across : along;
-                at = mine ? along : across;
+    if (owned) {
+        // subtracted in the reference's side order: top, bottom, left, right (the fluid
+        // interface of the acoustic-elastic propagator, its top edge, last)
+        auto corner = [&](int side) {
+            const int bc = side == 0 ? C.bc[0] : C.bc[1];
+            if (bc != 1 && bc != 2) return;
+            const float *q = sm + L::SAT + 96 + warp;
+            an = an - q[0];
+            at = at - q[32];
+            at = at - q[64];
+        };
+        if (XB && !AE && gz == 0) corner(0);
+        if (XB && gz == nz - 1) corner(1);
+        if (warp == 0) {
+            const int bc = br.side == 0 ? C.bc[0] : br.side == 1 ? C.bc[1] : br.side == 2 ? C.bc[2] : C.bc[3];
+            if (bc == 1 || bc == 2) {
+                const float *q = sm + L::SAT + lane;
+                at = at - q[0];
+                an = an - q[32];
+                an = an - q[64];
             }
         }
+        if (XB && AE && gz == 0) corner(0);
 
+        const double irho = SD[0];
         an = div64(C.dt2 * an, irho) + 2 * un - pn_;
         at = div64(C.dt2 * at, irho) + 2 * ut - pt_;
         float n0 = XB ? an : at, n1 = XB ? at : an;
         if (edge) {
-            const int per = 2 * nx + 2 * nz;
-            int kk;
-            if (gz == 0) kk = gx;
-            else if (gz == nz - 1) kk = nx + gx;
-            else if (gx == 0) kk = 2 * nx + gz;
-            else kk = 2 * nx + nz + gz;
-            n0 = div64(n0, 1.0 / (double)Sp->den[kk]);
-            n1 = div64(n1, 1.0 / (double)Sp->den[per + kk]);
+            n0 = div64(n0, SD[kFt]);
+            n1 = div64(n1, SD[2 * kFt]);
         }
         n0 = n0 * tzv * txv;
         if (AE && gz == 0) Sp->halo_save[gx] = XB ? pt_ : pn_;   // interface row: coupled and tapered by ae_couple
@@ -1079,30 +1189,102 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
 #ifndef FUSED_GRAD_BLOCKS
 #define FUSED_GRAD_BLOCKS 4
 #endif
+// Table entries of the windows to come, copied ahead: the next window's shot and
+// the tile after it (whose address needs nothing that is still on its way).
+__device__ __forceinline__ void fetch16(void *dst, const void *src, int bytes, int lane0)
+{
+    const int q = (int)threadIdx.x - lane0;
+    if (q >= 0 && q < bytes / 16) cp16((float *)dst + 4 * q, (const float *)src + 4 * q, true);
+}
+
 template <bool VTI, bool GRAD, bool AE>
 __global__ void __launch_bounds__(kFt, VTI && GRAD ? 3 : (GRAD ? FUSED_GRAD_BLOCKS : FUSED_FWD_BLOCKS))
 fused_steps(const __grid_constant__ FusedArgs A)
 {
     extern __shared__ __align__(16) float sm[];
-    // slots blockIdx.x, + gridDim.x, ... of the units rotated so that, with fewer
-    // than two units per CTA, the band units (the longest) get a CTA of their own
-    const int off = A.nunit < 2 * (int)gridDim.x ? max(0, A.nunit - (int)gridDim.x) : 0;
-    const bool one = blockIdx.x + gridDim.x >= A.nunit;   // this CTA's only unit
+    static_assert(sizeof(ShotDev) % 16 == 0 && sizeof(TileRef) % 16 == 0, "copied in 16-byte pieces");
+    __shared__ __align__(16) ShotDev S_[2];
+    __shared__ __align__(16) TileRef T_[4];
+    const int G = gridDim.x;
+    // slots blockIdx.x, + G, ... of the units (band units first) rotated so that, with
+    // fewer than two units per CTA, the band units (the longest) get a CTA of their own
+    const int off = A.nunit < 2 * G ? max(0, A.nunit - G) : 0;
+    auto unit = [&](int m) {
+        const int slot = blockIdx.x + m * G;
+        return slot >= off ? slot - off : slot - off + A.nunit;
+    };
+    const int n = (A.nunit - (int)blockIdx.x + G - 1) / G;   // this CTA's units
+    const bool one = n == 1;
+    // its windows are the slots [w0, w0 + nw), the others are band units
+    int w0 = 0, nw = 0;
+    for (int m = 0; m < n; m++)
+        if (unit(m) >= A.nband) {
+            if (nw == 0) w0 = m;
+            nw++;
+        }
+    auto window = [&](int q) { return A.in + (unit(w0 + q % nw) - A.nband); };
+    int q = 0;   // windows done so far
+    if (nw > 0) {
+        fetch16(&T_[0], window(0), sizeof(TileRef), 0);
+        fetch16(&T_[1], window(1), sizeof(TileRef), 32);
+        fetch16(&S_[0], A.shots + window(0)->shot, sizeof(ShotDev), 64);
+        cp_wait();
+        __syncthreads();
+    }
     for (int it = A.it0; it < A.it1; it++) {
         const bool keep = one && it > A.it0;
-        for (int slot = blockIdx.x; slot < A.nunit; slot += gridDim.x) {
-            const bool first = slot == blockIdx.x;
-            const int u = slot >= off ? slot - off : slot - off + A.nunit;
-            bool ok;
-            if (u >= A.nband) {
-                ok = fused_interior<VTI, GRAD, AE>(A, A.in[u - A.nband], it, first, keep, sm);
-            } else {
-                const BandRef br = A.bands[u];
-                if (br.side >= 2) ok = fused_band<true, VTI, GRAD, AE>(A, br, it, first, keep, sm);
-                else ok = fused_band<false, VTI, GRAD, AE>(A, br, it, first, keep, sm);
-            }
+        bool first = true;
+        for (int m = 0; m < n; m++) {
+            if (nw > 0 && m >= w0 && m < w0 + nw) continue;
+            const BandRef br = A.bands[unit(m)];
+            const bool ok = br.side >= 2 ? fused_band<true, VTI, GRAD, AE>(A, br, it, first, keep, sm)
+                                         : fused_band<false, VTI, GRAD, AE>(A, br, it, first, keep, sm);
             if (!ok) return;
-            __syncthreads();   // the next unit's staging, and this step's writes before the arrival
+            first = false;
+            __syncthreads();
+        }
+        for (int k = 0; k < nw; k++, q++) {
+            const ShotDev &S = S_[q & 1];
+            const TileRef &tr = T_[q & 3];
+            const bool active = it < S.nt - 1;
+            if (k == 0) {
+                if (active) {
+                    if (!keep) lead_model<VTI, GRAD, AE>(A, S, tr, sm);
+                    own_model<VTI, GRAD, AE>(A, S, tr, it, keep, sm);
+                }
+                if (first && !meet(A, it)) {
+                    cp_wait();
+                    return;
+                }
+                if (active) lead_fields<VTI, GRAD, AE>(S, tr, it, sm);
+                cp_commit();
+                if (active) own_fields<VTI, GRAD, AE>(A, S, tr, it, sm);
+                cp_commit();
+            }
+            cp_wait_but_one();
+            __syncthreads();   // the Lead group
+            fetch16(&T_[(q + 2) & 3], window(q + 2), sizeof(TileRef), 0);
+            fetch16(&S_[(q + 1) & 1], A.shots + T_[(q + 1) & 3].shot, sizeof(ShotDev), 32);
+            auto ahead = [&]() {
+                if (k + 1 < nw && it < S_[(q + 1) & 1].nt - 1) {
+                    lead_model<VTI, GRAD, AE>(A, S_[(q + 1) & 1], T_[(q + 1) & 3], sm);
+                    lead_fields<VTI, GRAD, AE>(S_[(q + 1) & 1], T_[(q + 1) & 3], it, sm);
+                }
+                cp_commit();
+            };
+            if (active) {
+                window_step<VTI, GRAD, AE>(A, S, tr, it, sm, ahead);
+            } else {
+                cp_wait();
+                __syncthreads();
+                ahead();
+            }
+            __syncthreads();   // the second half's arrays, and this step's writes before the arrival
+            if (k + 1 < nw && it < S_[(q + 1) & 1].nt - 1) {
+                own_model<VTI, GRAD, AE>(A, S_[(q + 1) & 1], T_[(q + 1) & 3], it, false, sm);
+                own_fields<VTI, GRAD, AE>(A, S_[(q + 1) & 1], T_[(q + 1) & 3], it, sm);
+            }
+            cp_commit();
         }
         if (threadIdx.x == 0 && it + 1 < A.it1) arrive(A);
     }

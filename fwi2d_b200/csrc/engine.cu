@@ -265,6 +265,7 @@ struct ShotPlan {
     DevBuf u0, u1, src_f, rcv_f, src_a;
     DevBuf d_inj_f, d_inj_f_off, d_inj_a, d_inj_a_off, d_ext_f, d_ext_f_off, d_ext_none_off;
     DevBuf d_mrow_f, d_mrow_a;
+    DevBuf d_brange_f, d_brange_a; // fused plans: the band cells' injection entries
     DevBuf den, tz, tx, snap, amax, grad, gwt;
     DevBuf xclos;                  // fused plans: x-closure sums of this shot's columns
     DevBuf gcomp;                  // compensated accumulation: running sum pair (hi, lo) of the gradient
@@ -365,6 +366,7 @@ struct Plan {
     // pass) and its pinned host copy, read after the pass has finished
     DevBuf d_status;
     DevBuf d_count;                // fused plans: arrivals of the launch's CTAs
+    DevBuf d_maps;                 // and the shots' tensor maps: [shot], then [shot] of the replay fields
     int *h_status = nullptr;
     ~Plan()
     {
@@ -599,7 +601,7 @@ struct ShotUnits {
     // (band and marching units)
     bool row_sorted(int u) const
     {
-        return u >= (int)tiles.size() + nxband && u < (int)(tiles.size() + bands.size() + marches.size());
+        return u >= (int)tiles.size() && u < (int)(tiles.size() + bands.size() + marches.size());
     }
     struct RowUnit {
         int unit, xb, xe, roff;
@@ -876,6 +878,26 @@ static void build_inj(const fwi2d_injector &J, int ncomp, const int *rowbase_a, 
     group_entries(U, ent, unit, row, zk, out, off, roff);
 }
 
+// Injection entries of every owned band cell of a fused plan (ShotDev::brange):
+// a band unit's entries are sorted by cell, a cell's in the reference's order
+// (component first).
+static std::vector<int4> band_ranges(const ShotUnits &U, const std::vector<InjEntry> &inj, const std::vector<int> &off)
+{
+    std::vector<int4> out(U.bands.size() * 6 * kFusedBand, int4{0, 0, 0, 0});
+    for (const BandRef &b : U.bands) {
+        const bool xb = b.side >= 2, far = b.side & 1;
+        const int n = xb ? U.nx : U.nz, e0 = off[b.unit], e1 = off[b.unit + 1];
+        for (int e = e0; e < e1; e++) {
+            const int gn = xb ? inj[e].gx : inj[e].gz, gt = xb ? inj[e].gz : inj[e].gx;
+            int4 &r = out[((size_t)b.unit * 6 + (far ? n - 1 - gn : gn)) * kFusedBand + gt - b.xb];
+            if (r.y + r.z == 0) r.x = e - e0;
+            if (inj[e].comp == 0) r.y++;
+            else r.z++;
+        }
+    }
+    return out;
+}
+
 // Receiver entries, owned by the unit of the pivot cell (the middle of the 3x3).
 static void build_ext(const fwi2d_injector &J, int ncomp, const ShotUnits &U, std::vector<ExtEntry> &out,
                       std::vector<int> &off, std::vector<int> &roff, int row0 = 0)
@@ -990,6 +1012,7 @@ static void shot_dev(const Plan &P, const ShotPlan &s, const ModelState &M, bool
         d.ext_off = s.d_ext_f_off.as<int>();
         d.n_ext = (int)s.ext_f.size();
         d.mrow = s.d_mrow_f.as<MarchRow>();
+        d.brange = s.d_brange_f.as<int4>();
     } else {
         d.src = s.src_a.as<float>();
         d.nsrc = s.nrcv_rows;
@@ -1001,6 +1024,7 @@ static void shot_dev(const Plan &P, const ShotPlan &s, const ModelState &M, bool
         d.ext_off = s.d_ext_none_off.as<int>();
         d.n_ext = 0;
         d.mrow = s.d_mrow_a.as<MarchRow>();
+        d.brange = s.d_brange_a.as<int4>();
     }
     d.den = s.den.as<float>();
     d.tz = s.tz.as<float>();
@@ -1482,6 +1506,13 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
         build_march_rows(U, S->inj_a, S->inj_a_roff, nullptr, tx, S->mrow_a);
         S->d_mrow_f.upload(S->mrow_f, ctx->st);
         S->d_mrow_a.upload(S->mrow_a, ctx->st);
+        std::vector<int4> brf, bra;
+        if (P->fused) {
+            brf = band_ranges(U, S->inj_f, S->inj_f_off);
+            bra = band_ranges(U, S->inj_a, S->inj_a_off);
+            S->d_brange_f.upload(brf, ctx->st);
+            S->d_brange_a.upload(bra, ctx->st);
+        }
         S->den.upload(den, ctx->st);
         S->tz.upload(tz, ctx->st);
         S->tx.upload(tx, ctx->st);
@@ -1531,6 +1562,23 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
         shot_dev(*P, *P->shots[s], M, true, sa[s]);
     }
     for (int s = 0; s < nshots; s++) sf[s].ckpt = P->shots[s]->ckpt.as<float>();
+    const size_t mb = fused_maps_bytes();
+    std::vector<unsigned char> maps;
+    if (P->fused) {
+        const bool replay = p.checkpoint_every > 0, f32 = p.snapshot_precision == FWI2D_SNAP_FP32;
+        maps.resize((replay ? 2 : 1) * nshots * mb);
+        for (int s = 0; s < nshots; s++) {
+            const ShotPlan &S = *P->shots[s];
+            const float *snap = f32 ? (const float *)S.snap_base : nullptr;
+            CK(fused_shot_maps(&maps[s * mb], S.nx, M.ldz, S.u0.as<float>(), S.u1.as<float>(), S.grad.as<float>(), snap,
+                               S.nbuf));
+            if (replay && S.r0.p)
+                CK(fused_shot_maps(&maps[(nshots + s) * mb], S.nx, M.ldz, S.r0.as<float>(), S.r1.as<float>(), nullptr,
+                                   nullptr, 0));
+        }
+        P->d_maps.upload(maps, ctx->st);
+        for (int s = 0; s < nshots; s++) sf[s].maps = sa[s].maps = P->d_maps.as<char>() + s * mb;
+    }
     P->d_shots_f.upload(sf, ctx->st);
     P->d_shots_a.upload(sa, ctx->st);
     if (ae) {
@@ -1568,6 +1616,8 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
                 r.snap = win;
                 ShotDev a = sa[s];
                 a.snap = win;
+                a.snap_first = (int)base;
+                if (P->fused) r.maps = P->d_maps.as<char>() + (nshots + s) * mb;
                 sr[(size_t)k * nshots + s] = r;
                 sc[(size_t)k * nshots + s] = a;
             }
@@ -1870,7 +1920,7 @@ static void set_shots(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, const
 {
     REQ(par != nullptr && shots != nullptr && nshots > 0, "no shots");
     fwi2d_params p = *par;
-    bool fused = ctx->M.kind == KIND_ELASTIC || ctx->M.kind == KIND_VTI;
+    bool fused = ctx->M.kind != KIND_ACOUSTIC;
     for (int i = 0; i < nshots && fused; i++) fused = shape_fits(fused_shape(), shots[i].nx, ctx->M.nz);
     // the fused time loop is the fastest shape wherever it fits: nothing to time
     if (p.tile_shape < 0 && ctx->M.kind >= 0 && !fused) {

@@ -57,6 +57,8 @@ struct alignas(16) ShotDev {
     int nrcv;
     const InjEntry *inj;  // grouped by work unit; march units sorted by (x, z), reference order per cell
     const int *inj_off;   // [units+1]
+    const int4 *brange;   // fused plans: per band unit and owned cell [6][kFusedBand], its entries: the first,
+                          // counted from the unit's, and the numbers of ux and of uz entries
     const ExtEntry *ext;  // grouped by the unit owning the pivot; march units sorted by pivot row
     const int *ext_off;   // [units+1]
     int n_ext;
@@ -73,8 +75,14 @@ struct alignas(16) ShotDev {
     float *halo_save;     // interface scratch (acoustic-elastic) or nullptr
     const float *gwt;     // gradient time-damping weight per snapshot index
     const float *xclos;   // fused plans: x-closure sums of mu [2 sides][6][8][ldz]; VTI: then those of fxx
+    const void *maps;     // fused plans: tensor maps of the fields, the gradient and the snapshots (ShotMap)
+    int snap_first;       // snapshot index of the snapshot maps' first slot
     float *ckpt;          // checkpoints [k][2][ncomp][nx][ldz] (checkpoint-and-recompute) or nullptr
 };
+
+// Tensor maps of a shot (fused.cu): field buffers 0 and 1 with the windows'
+// 4-cell halo and their own cells only, the gradient, FP32 snapshots likewise.
+enum ShotMap { SM_LEAD = 0, SM_OWN = 2, SM_GRAD = 4, SM_SNAP_LEAD, SM_SNAP_OWN, SM_COUNT = 8 };
 
 // Model on the full grid; shots index it at column x0 + ix.
 struct ModelDev {

@@ -22,7 +22,9 @@
 //
 // Everything a step writes is read through L2 (.cg), written by the SM that
 // owns the cell and read by its neighbours after the counter.
+#include <cuda.h>
 #include <cuda_runtime.h>
+#include <cstring>
 #include "engine.h"
 #include "sbp.cuh"
 #include "snap.cuh"
@@ -49,8 +51,51 @@ __device__ __forceinline__ void cp16(float *dst, const float *src, bool ok)
                  : "memory");
 }
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_wait_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+
+// ---- tiled bulk copies (TMA) of a window's arrays, issued by one thread -------------
+__device__ __forceinline__ unsigned saddr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void tma2(float *dst, const CUtensorMap *m, int z, int x, unsigned long long *bar)
+{
+    asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                     saddr(dst)),
+                 "l"(m), "r"(z), "r"(x), "r"(saddr(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void tma3(float *dst, const CUtensorMap *m, int z, int x, int c, unsigned long long *bar)
+{
+    asm volatile("cp.async.bulk.tensor.3d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+                     saddr(dst)),
+                 "l"(m), "r"(z), "r"(x), "r"(c), "r"(saddr(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void tma4(float *dst, const CUtensorMap *m, int z, int x, int c, int k, unsigned long long *bar)
+{
+    asm volatile("cp.async.bulk.tensor.4d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
+                     saddr(dst)),
+                 "l"(m), "r"(z), "r"(x), "r"(c), "r"(k), "r"(saddr(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void bar_init(unsigned long long *bar)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(bar)) : "memory");
+}
+__device__ __forceinline__ void bar_expect(unsigned long long *bar, unsigned bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(saddr(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool bar_done(unsigned long long *bar, unsigned parity)
+{
+    unsigned ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(ok)
+                 : "r"(saddr(bar)), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+// Fields and gradients are written by ordinary stores and read by TMA: ordered
+// by this fence on the writing side (before the arrival) and on the reading
+// side (after the meeting).
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
 // ---- packed arithmetic beyond sbp.cuh ---------------------------------------
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
@@ -175,6 +220,7 @@ struct InLayout {
 // [6][8][28], and for x bands those along z next to the corners, [2][6][8][6].
 // D, DS, DT: the strain sum (VTI and acoustic-elastic: two arrays) and the two
 // shear strains.
+constexpr int kVal = 512;
 template <bool VTI, bool GRAD, bool AE>
 struct BandLayout {
     static constexpr int A = kFb * kFs, CL = 6 * 8 * kFusedBand;
@@ -186,12 +232,15 @@ struct BandLayout {
     // per thread, set once per unit: doubles 1/rho and 1/den (two components), then the floats of Slot
     static constexpr int SD = ZC + 2 * 6 * 8 * 6;
     static constexpr int SF = SD + 3 * 2 * kFt;
-    static constexpr int SAT = SF + 8 * kFt;               // [own side, corner][along, across, normal][32]
-    static constexpr int RED = SAT + 6 * 32;
+    static constexpr int SAT = SF + 7 * kFt;               // [own side, corner][along, across, normal][32]
+    static constexpr int VAL = SAT + 6 * 32;               // this step's injected values, one per entry of the unit
+    static constexpr int RED = VAL + kVal;
     static constexpr int FLOATS = RED + 8;
     static_assert(SD % 2 == 0, "doubles");
 };
-enum Slot { SL_TZX = 0, SL_TX, SL_IMP, SL_IMPC, SL_E0, SL_E1, SL_R0, SL_R1 };
+constexpr int kCells = 6 * kFusedBand;                     // owned cells of a band unit
+// (warps 6 and 7 hold impedances where the others hold their cell's entries)
+enum Slot { SL_TZX = 0, SL_TX, SL_IMP, SL_IMPC, SL_R0, SL_R1, SL_NX, SL_E0 = SL_IMP, SL_NZ = SL_IMPC };
 
 template <bool VTI, bool GRAD, bool AE>
 constexpr size_t fused_bytes()
@@ -201,7 +250,10 @@ constexpr size_t fused_bytes()
                                 : BandLayout<VTI, GRAD, AE>::FLOATS);
 }
 
-struct FusedArgs {
+// model arrays of the windows: boxes with the 2-cell halo (mu .. lam), own cells (rho ..)
+enum ModelMap { MM_MU = 0, MM_Q, MM_LB, MM_LC, MM_LA, MM_RHO, MM_IR, MM_EPS, MM_V2, MM_V3, MM_COUNT };
+struct alignas(64) FusedArgs {
+    CUtensorMap mm[MM_COUNT];
     const ShotDev *shots;
     const BandRef *bands;   // x bands (side 2, 3), then z bands (side 0, 1)
     const TileRef *in;
@@ -279,16 +331,33 @@ __device__ __forceinline__ float density_term(float g, double wdt, int k, int la
     return (float)((double)g + wdt * (double)s);
 }
 
+// Waits for a phase of an mbarrier, bounded as `meet`; false when the copies are taken to be lost.
+__device__ __forceinline__ bool wait_bar(const FusedArgs &A, unsigned long long *bar, unsigned &parity, int it)
+{
+    bool ok = false;
+    for (int k = 0; k < A.C.spin && !ok; k++) ok = bar_done(bar, parity);
+    if (!ok) {
+        atomicCAS(A.status, 0, it + 1);
+        for (int k = 0; k < kHardPolls && !ok; k++) ok = bar_done(bar, parity);
+    }
+    parity ^= 1u;
+    return ok;
+}
+
 // ---------------------------------------------------------------------------
 // Interior window.  Thread t owns the z-pair 2 (t & 15) of column t >> 4.  The
-// loads come in two groups: what the first half of the work reads (fields with
-// their halo, coefficients: Lead) and what the second half reads (previous
-// field, density, snapshots, gradient: Own).  While a window is in its second
-// half, the Lead group of the CTA's next window is on its way into the arrays
-// that the first half has left, and while it is in its first half its own Own
-// group is: a CTA's loads overlap its arithmetic without a second buffer.
+// loads come in two groups of tiled bulk copies, issued by one thread: what the
+// first half of the work reads (fields with their halo, coefficients: Lead) and
+// what the second half reads (previous field, density, snapshots, gradient:
+// Own).  While a window is in its second half, the Lead group of the CTA's next
+// window is on its way into the arrays that the first half has left, and while
+// it is in its first half its own Own group is: a CTA's loads overlap its
+// arithmetic without a second buffer.  With a 16-byte cp.async per thread
+// instead of the bulk copies, addresses and predicates were 130 of the 420
+// instructions per cell (8 forward shots of 801 x 401).
 // keep: the model arrays are in shared memory from the last step.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ int by(int a, int sub) { return sub == 1 ? a : a / sub; }
 struct Imaging {
     int itf, last;
     bool on;
@@ -296,106 +365,119 @@ struct Imaging {
 template <bool GRAD, bool AE>
 __device__ __forceinline__ Imaging imaging(const ShotDev &S, const StepConst &C, int it)
 {
-    Imaging g;
-    g.itf = GRAD ? (S.nt - 1 - (it + 1)) / C.sub : 0;
-    g.last = S.nt / C.sub;
-    g.on = GRAD && it < S.nt - 1 && (S.nt - 1 - (it + 1)) % C.sub == 0 && (!AE || g.itf != 0);
+    Imaging g = {0, 0, false};
+    if (!GRAD) return g;
+    const int k = S.nt - 2 - it;
+    g.itf = by(k, C.sub);
+    g.last = by(S.nt, C.sub);
+    g.on = k >= 0 && g.itf * C.sub == k && (!AE || g.itf != 0);
     return g;
 }
 
+// by one thread
 template <bool VTI, bool GRAD, bool AE>
-__device__ __forceinline__ void lead_model(const FusedArgs &A, const ShotDev &S, const TileRef &tr, float *sm)
+__device__ __forceinline__ void issue_lead(const FusedArgs &A, const ShotDev &S, const TileRef &tr, int it, bool model,
+                                           bool fields, float *sm, unsigned long long *bar)
 {
     using L = InLayout<VTI, GRAD, AE>;
-    const int t = threadIdx.x, xr = t / 10, xq = 4 * (t - 10 * xr);
-    if (t >= (kFx + 4) * 10) return;
-    const int gx = tr.wx0 - 2 + xr, gz = tr.wz0 - 4 + xq;
-    const bool ok = gx < S.nx && gz < S.ldz;
-    const long long o = (long long)S.x0 * S.ldz + (ok ? (long long)gx * S.ldz + gz : 0);   // the model has the shots' pitch
-    const int s = xr * kFs + xq;
-    cp16(sm + L::MU + s, A.M.p1 + o, ok);
-    cp16(sm + L::Q + s, (VTI ? A.M.fxx : A.M.p0) + o, ok);
-    if (VTI) {
-        cp16(sm + L::LB + s, A.M.lbis + o, ok);
-        cp16(sm + L::LC + s, A.M.c13 + o, ok);
-        cp16(sm + L::LA + s, A.M.p0 + o, ok);
-    }
-}
-
-template <bool VTI, bool GRAD, bool AE>
-__device__ __forceinline__ void lead_fields(const ShotDev &S, const TileRef &tr, int it, float *sm)
-{
-    using L = InLayout<VTI, GRAD, AE>;
-    const int t = threadIdx.x, xr = t / 10, xq = 4 * (t - 10 * xr);
-    if (t >= (kFx + 8) * 10) return;
-    const int x = tr.wx0 - 4 + xr, z = tr.wz0 - 4 + xq;
-    const bool ok = x < S.nx && z < S.ldz;
-    const long long o = ok ? (long long)x * S.ldz + z : 0;
-    const float *curr = S.u[(it + 1) & 1];
-    cp16(sm + L::U0 + xr * kFs + xq, curr + o, ok);
-    cp16(sm + L::U1 + xr * kFs + xq, curr + (long long)S.nx * S.ldz + o, ok);
-}
-
-// density and its reciprocal; snapshots of the imaging condition (no step of this launch writes them)
-template <bool VTI, bool GRAD, bool AE>
-__device__ __forceinline__ void own_model(const FusedArgs &A, const ShotDev &S, const TileRef &tr, int it, bool keep,
-                                          float *sm)
-{
-    using L = InLayout<VTI, GRAD, AE>;
-    const int t = threadIdx.x, h = t >> 7, row = (t >> 3) & 15, q = 4 * (t & 7);
-    const int gx = tr.wx0 + row, gz = tr.wz0 + q;
-    const bool ok = gx < S.nx && gz < S.ldz;
-    const long long nxz = (long long)S.nx * S.ldz, c = ok ? (long long)gx * S.ldz + gz : 0;
-    const long long m = (long long)S.x0 * S.ldz + c;
-    const int s = h * kFo + row * kFz + q;
-    if (!keep) cp16(sm + L::RHO + s, (h ? A.M.irho : A.M.p2) + m, ok);
-    const Imaging g = imaging<GRAD, AE>(S, A.C, it);
-    if (!GRAD || !g.on) return;
-    if (VTI && !keep) {
-        cp16(sm + L::E + s, (h ? A.M.gv2 : A.M.eps) + m, ok);
-        if (t < 128) cp16(sm + L::E + 2 * kFo + s, A.M.gv3 + m, ok);
-    }
-    const int prec = A.C.snap_prec;
-    auto snap = [&](int dst, int k, long long off, bool have) {
-        const long long so = (long long)k * S.snap_slot + off;
-        if (prec == SNAP_FP32 || !have) {
-            cp16(sm + dst, (const float *)S.snap + (have ? so : 0), have);
-        } else {
-            const float inv = 1.f / snap_scale(S.snap_amax, k);
-            *reinterpret_cast<float4 *>(sm + dst) = snap_load4(S.snap, so, prec, inv);
+    const int z = tr.wz0 - 4, x = tr.wx0 - 2, xm = S.x0 + x;
+    if (model) {
+        tma2(sm + L::MU, &A.mm[MM_MU], z, xm, bar);
+        tma2(sm + L::Q, &A.mm[MM_Q], z, xm, bar);
+        if (VTI) {
+            tma2(sm + L::LB, &A.mm[MM_LB], z, xm, bar);
+            tma2(sm + L::LC, &A.mm[MM_LC], z, xm, bar);
+            tma2(sm + L::LA, &A.mm[MM_LA], z, xm, bar);
         }
-    };
-    snap(L::FP0 + s, g.itf + 1, c + h * nxz, ok && g.itf + 1 <= g.last);
-    snap(L::FM0 + s, g.itf - 1, c + h * nxz, ok && g.itf > 0);
-    const int xr = t / 10, xq = 4 * (t - 10 * xr);
-    if (t < (kFx + 4) * 10) {
-        const int x = tr.wx0 - 2 + xr, z = tr.wz0 - 4 + xq;
-        const bool in = x < S.nx && z < S.ldz;
-        const long long o = in ? (long long)x * S.ldz + z : 0;
-        snap(L::F0 + xr * kFs + xq, g.itf, o, in);
-        snap(L::F1 + xr * kFs + xq, g.itf, o + nxz, in);
     }
+    if (fields) tma3(sm + L::U0, (const CUtensorMap *)S.maps + SM_LEAD + ((it + 1) & 1), z, x - 2, 0, bar);
+}
+template <bool VTI>
+__device__ __forceinline__ unsigned lead_bytes(bool model)
+{
+    return 4u * (2 * kFu + (model ? (VTI ? 5 : 2) * kFw : 0));
 }
 
+// model: density and its reciprocal (VTI imaging: its coefficients); snapshots (FP32; no step of this launch writes them)
 template <bool VTI, bool GRAD, bool AE>
-__device__ __forceinline__ void own_fields(const FusedArgs &A, const ShotDev &S, const TileRef &tr, int it, float *sm)
+__device__ __forceinline__ void issue_own_static(const FusedArgs &A, const ShotDev &S, const TileRef &tr, int it, bool model,
+                                                 float *sm, unsigned long long *bar)
 {
     using L = InLayout<VTI, GRAD, AE>;
+    const CUtensorMap *sp = (const CUtensorMap *)S.maps;
+    const int z = tr.wz0, x = tr.wx0, xm = S.x0 + x;
+    const Imaging g = imaging<GRAD, AE>(S, A.C, it);
+    const bool f32 = GRAD && g.on && A.C.snap_prec == SNAP_FP32;
+    unsigned bytes = 4u * kFo * (2 + (model ? 2 : 0));
+    if (GRAD && g.on) bytes += 4u * kFo * 3;
+    if (VTI && GRAD && model) bytes += 4u * kFo * 3;
+    if (f32) bytes += 4u * (2 * kFw + kFo * ((g.itf + 1 <= g.last ? 2 : 0) + (g.itf > 0 ? 2 : 0)));
+    bar_expect(bar, bytes);
+    if (model) {
+        tma2(sm + L::RHO, &A.mm[MM_RHO], z, xm, bar);
+        tma2(sm + L::IR, &A.mm[MM_IR], z, xm, bar);
+        if (VTI && GRAD) {
+            tma2(sm + L::E, &A.mm[MM_EPS], z, xm, bar);
+            tma2(sm + L::E + kFo, &A.mm[MM_V2], z, xm, bar);
+            tma2(sm + L::E + 2 * kFo, &A.mm[MM_V3], z, xm, bar);
+        }
+    }
+    if (f32) {
+        const int k = g.itf - S.snap_first;
+        tma4(sm + L::F0, sp + SM_SNAP_LEAD, z - 4, x - 2, 0, k, bar);
+        if (g.itf + 1 <= g.last) tma4(sm + L::FP0, sp + SM_SNAP_OWN, z, x, 0, k + 1, bar);
+        if (g.itf > 0) tma4(sm + L::FM0, sp + SM_SNAP_OWN, z, x, 0, k - 1, bar);
+        // the next imaging step's new snapshot, from HBM to L2
+        if (k >= 2)
+            asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global [%0, {%1, %2, %3, %4}];" ::"l"(sp + SM_SNAP_OWN), "r"(z),
+                         "r"(x), "r"(0), "r"(k - 2)
+                         : "memory");
+    }
+}
+template <bool VTI, bool GRAD, bool AE>
+__device__ __forceinline__ void issue_own_fields(const FusedArgs &A, const ShotDev &S, const TileRef &tr, int it, float *sm,
+                                                 unsigned long long *bar)
+{
+    using L = InLayout<VTI, GRAD, AE>;
+    const CUtensorMap *sp = (const CUtensorMap *)S.maps;
+    tma3(sm + L::PV0, sp + SM_OWN + (it & 1), tr.wz0, tr.wx0, 0, bar);
+    if (GRAD && imaging<GRAD, AE>(S, A.C, it).on) tma3(sm + L::G0, sp + SM_GRAD, tr.wz0, tr.wx0, 0, bar);
+}
+
+// 16-bit snapshots of a window: converted on the way to shared memory by all threads
+template <bool VTI, bool GRAD, bool AE>
+__device__ __forceinline__ void load_snaps16(const FusedArgs &A, const ShotDev &S, const TileRef &tr, int it, float *sm)
+{
+    using L = InLayout<VTI, GRAD, AE>;
+    const int prec = A.C.snap_prec;
+    if (!GRAD || prec == SNAP_FP32) return;
+    const Imaging g = imaging<GRAD, AE>(S, A.C, it);
+    if (!g.on) return;
     const int t = threadIdx.x, h = t >> 7, row = (t >> 3) & 15, q = 4 * (t & 7);
     const int gx = tr.wx0 + row, gz = tr.wz0 + q;
-    const bool ok = gx < S.nx && gz < S.ldz;
-    const long long nxz = (long long)S.nx * S.ldz, c = ok ? (long long)gx * S.ldz + gz : 0;
+    const long long nxz = (long long)S.nx * S.ldz;
     const int s = h * kFo + row * kFz + q;
-    cp16(sm + L::PV0 + s, S.u[it & 1] + h * nxz + c, ok);
-    if (GRAD && imaging<GRAD, AE>(S, A.C, it).on) {
-        cp16(sm + L::G0 + s, S.grad + h * nxz + c, ok);
-        if (t < 128) cp16(sm + L::G0 + 2 * kFo + s, S.grad + 2 * nxz + c, ok);
+    const float inv = 1.f / snap_scale(S.snap_amax, g.itf);
+    if (gx < S.nx && gz < S.ldz) {
+        const long long c = (long long)g.itf * S.snap_slot + h * nxz + (long long)gx * S.ldz + gz;
+        if (g.itf + 1 <= g.last)
+            *reinterpret_cast<float4 *>(sm + L::FP0 + s) =
+                snap_load4(S.snap, c + S.snap_slot, prec, 1.f / snap_scale(S.snap_amax, g.itf + 1));
+        if (g.itf > 0)
+            *reinterpret_cast<float4 *>(sm + L::FM0 + s) =
+                snap_load4(S.snap, c - S.snap_slot, prec, 1.f / snap_scale(S.snap_amax, g.itf - 1));
+    }
+    const int xr = t / 10, xq = 4 * (t - 10 * xr), x = tr.wx0 - 2 + xr, z = tr.wz0 - 4 + xq;
+    if (t < (kFx + 4) * 10 && x < S.nx && z < S.ldz) {
+        const long long o = (long long)g.itf * S.snap_slot + (long long)x * S.ldz + z;
+        *reinterpret_cast<float4 *>(sm + L::F0 + xr * kFs + xq) = snap_load4(S.snap, o, prec, inv);
+        *reinterpret_cast<float4 *>(sm + L::F1 + xr * kFs + xq) = snap_load4(S.snap, o + nxz, prec, inv);
     }
 }
 
 // The window's step, its Lead group present; mid() runs between its halves.
 template <bool VTI, bool GRAD, bool AE, class Mid>
-__device__ __forceinline__ void window_step(const FusedArgs &A, const ShotDev &S, const TileRef &tr, const int it, float *sm,
+__device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S, const TileRef &tr, const int it, float *sm,
                                             Mid mid)
 {
     using L = InLayout<VTI, GRAD, AE>;
@@ -493,9 +575,7 @@ __device__ __forceinline__ void window_step(const FusedArgs &A, const ShotDev &S
         }
     }
     const float2 a00 = ld2(U0, i), b00 = ld2(U1, i);
-    cp_wait();
-    __syncthreads();
-    mid();   // U, the coefficients and their loads' addresses are free for the next window
+    if (!mid()) return false;   // the Own group is there; U and the coefficients are free for the next window
 
     // ---- mixed terms
     auto along_x = [&](const float *p, float s) {
@@ -563,8 +643,8 @@ __device__ __forceinline__ void window_step(const FusedArgs &A, const ShotDev &S
         pn[cell + 1] = n0.y;
         pn[nxz + cell + 1] = n1.y;
     }
-    if (!GRAD && (A.flags & F_STORE) && it % C.sub == 0) {
-        const int slot = it / C.sub;
+    const int slot = by(it, C.sub);
+    if (!GRAD && (A.flags & F_STORE) && slot * C.sub == it) {
         const long long o = (long long)slot * S.snap_slot + cell;
         if (prec == SNAP_FP32 && own0 && own1) {
             *reinterpret_cast<float2 *>((float *)S.snap + o) = a00;
@@ -649,6 +729,7 @@ __device__ __forceinline__ void window_step(const FusedArgs &A, const ShotDev &S
         if (own1) m = fmaxf(m, fmaxf(fabsf(n0.y), fabsf(n1.y)));
         block_amax(m, sm + L::RED, S.snap_amax + (it + 1) / C.sub);
     }
+    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -683,9 +764,9 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
     const int nn = XB ? nx : nz;
     const int prec = C.snap_prec;
     const long long mofs = (long long)Sp->x0 * ldz;
-    const int itf = GRAD ? (nt - 1 - (it + 1)) / C.sub : 0;
-    const bool do_grad = GRAD && it < nt - 1 && ((nt - 1 - (it + 1)) % C.sub == 0) && (!AE || itf != 0);
-    const int last = nt / C.sub;
+    const Imaging im = imaging<GRAD, AE>(*Sp, C, it);
+    const int itf = im.itf, last = im.last;
+    const bool do_grad = im.on;
     const float sg = far ? -1.f : 1.f;
     // along the edge: samples that exist (z bands: within the columns clear of the x bands and their halo)
     const int glo = XB ? 0 : t0 - 4, ghi = XB ? nz : t1 + 4;
@@ -758,7 +839,8 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
             return VTI && !zside ? 0.5f * sqrtf((1 + 2 * M.eps[m]) * l2m * rho) : 0.5f * sqrtf(l2m * rho);
         };
         float tzv = 0.f, txv = 0.f;
-        int e0 = 0, e1 = 0, r0 = 0, r1 = 0;
+        int4 ent = make_int4(0, 0, 0, 0);
+        int r0 = 0, r1 = 0;
         if (mine) {
             SD[0] = 1.0 / (double)M.p2[mcell];
             if (warp >= 6) SF[SL_IMP * kFt] = impedance(mcell, !XB);
@@ -770,27 +852,37 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
             }
             tzv = Sp->tz[gz];
             txv = Sp->tx[gx];
+            if (owned) ent = Sp->brange[(long long)br.unit * kCells + row * kFusedBand + lane - 2];
             if (!XB) {
                 const MarchRow R = Sp->mrow[br.roff + gt - t0];
-                e0 = R.e0;
-                e1 = R.e1;
                 r0 = R.r0;
                 r1 = warp == 0 ? R.r1 : R.r0;
             }
         }
         if (XB) {
-            e0 = Sp->inj_off[br.unit];
-            e1 = Sp->inj_off[br.unit + 1];
             r0 = Sp->ext_off[br.unit] + t;
             r1 = Sp->ext_off[br.unit + 1];
         }
         if (cside) SF[SL_IMPC * kFt] = impedance(mofs + ccell, true);
         SF[SL_TZX * kFt] = tzv;
         SF[SL_TX * kFt] = txv;
-        SF[SL_E0 * kFt] = __int_as_float(e0);
-        SF[SL_E1 * kFt] = __int_as_float(e1);
+        if (warp < 6) {
+            SF[SL_E0 * kFt] = __int_as_float(ent.x);
+            SF[SL_NX * kFt] = __int_as_float(ent.y);
+            SF[SL_NZ * kFt] = __int_as_float(ent.z);
+        }
         SF[SL_R0 * kFt] = __int_as_float(r0);
         SF[SL_R1 * kFt] = __int_as_float(r1);
+    }
+    // this step's injected values, in the entries' order, and a look ahead at the next row
+    const int inj0 = Sp->inj_off[br.unit], ninj = Sp->inj_off[br.unit + 1] - inj0;
+    if (it < nt - 1 && ninj <= kVal) {
+        const float *srcrow = Sp->src + (long long)it * Sp->nsrc;
+        for (int e = t; e < ninj; e += kFt) {
+            const InjEntry &E = Sp->inj[inj0 + e];
+            sm[L::VAL + e] = E.mt ? (E.wa * srcrow[E.ia] - E.wb * srcrow[E.ib]) : E.wa * srcrow[E.ia];
+            if (it + 1 < nt) asm volatile("prefetch.global.L2 [%0];" ::"l"(srcrow + Sp->nsrc + E.ia));
+        }
     }
     float fp0 = 0.f, fp1 = 0.f, fm0 = 0.f, fm1 = 0.f;
     if (GRAD && do_grad) {
@@ -819,6 +911,17 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
                 sm[L::F0 + s_[h]] = a_[h];
                 sm[L::F1 + s_[h]] = b_[h];
             }
+        // the next imaging step's new snapshot, from HBM to L2
+        if (itf - Sp->snap_first >= 2) {
+            const int esz = prec == SNAP_FP32 ? 4 : 2;
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                if (in_[h]) {
+                    const char *p = (const char *)Sp->snap + (so - 2 * Sp->snap_slot + o_[h]) * esz;
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (long long)nxz * esz));
+                }
+        }
     }
     const bool edge = owned && (gz == 0 || gz == nz - 1 || gx == 0 || gx == nx - 1);
     const float *curr = Sp->u[(it + 1) & 1];
@@ -1082,16 +1185,23 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
             at += mdern(L::DT, L::MU);
         }
         // sources of this cell, in the reference's order
-        const int e1 = __float_as_int(SF[SL_E1 * kFt]);
-        int e = __float_as_int(SF[SL_E0 * kFt]);
-        if (e < e1) {
-            const float *srcrow = Sp->src + (long long)it * Sp->nsrc;
-            for (; e < e1; e++) {
-                const InjEntry &E = Sp->inj[e];
-                if (E.gx != gx || E.gz != gz) continue;
-                const float v = E.mt ? (E.wa * srcrow[E.ia] - E.wb * srcrow[E.ib]) : E.wa * srcrow[E.ia];
-                if (XB ? E.comp == 0 : E.comp == 1) an += v;
-                else at += v;
+        // (its entries: first, then the counts of ux and uz entries)
+        const int nx_ = __float_as_int(SF[SL_NX * kFt]), nz_ = __float_as_int(SF[SL_NZ * kFt]);
+        if (nx_ + nz_ > 0) {
+            const int e = __float_as_int(SF[SL_E0 * kFt]);
+            auto value = [&](int k) {
+                if (ninj <= kVal) return sm[L::VAL + k];
+                const float *srcrow = Sp->src + (long long)it * Sp->nsrc;
+                const InjEntry &E = Sp->inj[inj0 + k];
+                return E.mt ? (E.wa * srcrow[E.ia] - E.wb * srcrow[E.ib]) : E.wa * srcrow[E.ia];
+            };
+            for (int k = 0; k < nx_; k++) {
+                if (XB) an += value(e + k);
+                else at += value(e + k);
+            }
+            for (int k = 0; k < nz_; k++) {
+                if (XB) at += value(e + nx_ + k);
+                else an += value(e + nx_ + k);
             }
         }
     }
@@ -1135,8 +1245,8 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
         pn[cell] = n0;
         pn[nxz + cell] = n1;
         amax = fmaxf(fabsf(n0), fabsf(n1));
-        if (!GRAD && (A.flags & F_STORE) && it % C.sub == 0) {
-            const int slot = it / C.sub;
+        const int slot = by(it, C.sub);
+        if (!GRAD && (A.flags & F_STORE) && slot * C.sub == it) {
             const float sc = prec == SNAP_FP32 ? 1.f : snap_scale(Sp->snap_amax, slot);
             const long long o = (long long)slot * Sp->snap_slot + cell;
             snap_store(Sp->snap, o, prec, XB ? un : ut, sc);
@@ -1201,7 +1311,7 @@ template <bool VTI, bool GRAD, bool AE>
 __global__ void __launch_bounds__(kFt, VTI && GRAD ? 3 : (GRAD ? FUSED_GRAD_BLOCKS : FUSED_FWD_BLOCKS))
 fused_steps(const __grid_constant__ FusedArgs A)
 {
-    extern __shared__ __align__(16) float sm[];
+    extern __shared__ __align__(1024) float sm[];
     static_assert(sizeof(ShotDev) % 16 == 0 && sizeof(TileRef) % 16 == 0, "copied in 16-byte pieces");
     __shared__ __align__(16) ShotDev S_[2];
     __shared__ __align__(16) TileRef T_[4];
@@ -1224,7 +1334,15 @@ fused_steps(const __grid_constant__ FusedArgs A)
         }
     auto window = [&](int q) { return A.in + (unit(w0 + q % nw) - A.nband); };
     int q = 0;   // windows done so far
+    unsigned par_lead = 0, par_own = 0;
+    __shared__ unsigned long long bars[2];
+    unsigned long long *const lead = bars, *const own = bars + 1;
     if (nw > 0) {
+        if (threadIdx.x == 0) {
+            bar_init(lead);
+            bar_init(own);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
         fetch16(&T_[0], window(0), sizeof(TileRef), 0);
         fetch16(&T_[1], window(1), sizeof(TileRef), 32);
         fetch16(&S_[0], A.shots + window(0)->shot, sizeof(ShotDev), 64);
@@ -1244,47 +1362,63 @@ fused_steps(const __grid_constant__ FusedArgs A)
             __syncthreads();
         }
         for (int k = 0; k < nw; k++, q++) {
-            const ShotDev &S = S_[q & 1];
-            const TileRef &tr = T_[q & 3];
+            const ShotDev &S = S_[q & 1], &Sn = S_[(q + 1) & 1];
+            const TileRef &tr = T_[q & 3], &tn = T_[(q + 1) & 3];
             const bool active = it < S.nt - 1;
             if (k == 0) {
+                // the first window of a step: what no step writes, then the meeting, then the fields
                 if (active) {
-                    if (!keep) lead_model<VTI, GRAD, AE>(A, S, tr, sm);
-                    own_model<VTI, GRAD, AE>(A, S, tr, it, keep, sm);
+                    if (threadIdx.x == 0) {
+                        fence_async();
+                        bar_expect(lead, lead_bytes<VTI>(!keep));
+                        issue_lead<VTI, GRAD, AE>(A, S, tr, it, !keep, false, sm, lead);
+                        issue_own_static<VTI, GRAD, AE>(A, S, tr, it, !keep, sm, own);
+                    }
+                    load_snaps16<VTI, GRAD, AE>(A, S, tr, it, sm);
                 }
-                if (first && !meet(A, it)) {
-                    cp_wait();
-                    return;
+                if (first && !meet(A, it)) return;
+                if (active && threadIdx.x == 0) {
+                    fence_async();
+                    issue_lead<VTI, GRAD, AE>(A, S, tr, it, false, true, sm, lead);
+                    issue_own_fields<VTI, GRAD, AE>(A, S, tr, it, sm, own);
                 }
-                if (active) lead_fields<VTI, GRAD, AE>(S, tr, it, sm);
-                cp_commit();
-                if (active) own_fields<VTI, GRAD, AE>(A, S, tr, it, sm);
-                cp_commit();
             }
-            cp_wait_but_one();
-            __syncthreads();   // the Lead group
-            fetch16(&T_[(q + 2) & 3], window(q + 2), sizeof(TileRef), 0);
-            fetch16(&S_[(q + 1) & 1], A.shots + T_[(q + 1) & 3].shot, sizeof(ShotDev), 32);
+            fetch16(&T_[(q + 2) & 3], window(q + 2), sizeof(TileRef), 32);
+            fetch16(&S_[(q + 1) & 1], A.shots + tn.shot, sizeof(ShotDev), 64);
+            // between the halves: the Own group and the next entries have arrived, all
+            // threads have left the first half
             auto ahead = [&]() {
-                if (k + 1 < nw && it < S_[(q + 1) & 1].nt - 1) {
-                    lead_model<VTI, GRAD, AE>(A, S_[(q + 1) & 1], T_[(q + 1) & 3], sm);
-                    lead_fields<VTI, GRAD, AE>(S_[(q + 1) & 1], T_[(q + 1) & 3], it, sm);
+                const bool ok = !active || wait_bar(A, own, par_own, it);
+                cp_wait();
+                if (__syncthreads_or(!ok)) return false;
+                if (k + 1 < nw && it < Sn.nt - 1 && threadIdx.x == 0) {
+                    fence_async();
+                    bar_expect(lead, lead_bytes<VTI>(true));
+                    issue_lead<VTI, GRAD, AE>(A, Sn, tn, it, true, true, sm, lead);
                 }
-                cp_commit();
+                return true;
             };
             if (active) {
-                window_step<VTI, GRAD, AE>(A, S, tr, it, sm, ahead);
-            } else {
-                cp_wait();
-                __syncthreads();
-                ahead();
+                const bool ok = wait_bar(A, lead, par_lead, it);
+                if (__syncthreads_or(!ok)) return;
+                if (!window_step<VTI, GRAD, AE>(A, S, tr, it, sm, ahead)) return;
+            } else if (!ahead()) {
+                return;
             }
-            __syncthreads();   // the second half's arrays, and this step's writes before the arrival
-            if (k + 1 < nw && it < S_[(q + 1) & 1].nt - 1) {
-                own_model<VTI, GRAD, AE>(A, S_[(q + 1) & 1], T_[(q + 1) & 3], it, false, sm);
-                own_fields<VTI, GRAD, AE>(A, S_[(q + 1) & 1], T_[(q + 1) & 3], it, sm);
+            if (k + 1 == nw) fence_async();   // this step's writes, before the arrival
+            __syncthreads();
+            if (k + 1 < nw && it < Sn.nt - 1) {
+                if (threadIdx.x == 0) {
+                    fence_async();
+                    issue_own_static<VTI, GRAD, AE>(A, Sn, tn, it, true, sm, own);
+                    issue_own_fields<VTI, GRAD, AE>(A, Sn, tn, it, sm, own);
+                }
+                load_snaps16<VTI, GRAD, AE>(A, Sn, tn, it, sm);
             }
-            cp_commit();
+        }
+        if (nw == 0) {
+            fence_async();
+            __syncthreads();
         }
         if (threadIdx.x == 0 && it + 1 < A.it1) arrive(A);
     }
@@ -1353,6 +1487,68 @@ static cudaError_t launch_fused_t(const FusedArgs &A, cudaStream_t st)
     return cudaLaunchKernelEx(&cfg, kernel, A);
 }
 
+// ---- tensor maps ----------------------------------------------------------------
+// cuTensorMapEncodeTiled through the runtime (the library does not link the driver)
+static cudaError_t encode(CUtensorMap *m, const void *base, int rank, const cuuint64_t *dim, const cuuint32_t *box)
+{
+    using Fn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                            const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                            CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q);
+    if (e != cudaSuccess) return e;
+    if (!f || q != cudaDriverEntryPointSuccess) return cudaErrorNotSupported;
+    cuuint64_t stride[3];
+    cuuint32_t one[4] = {1, 1, 1, 1};
+    cuuint64_t s = sizeof(float);
+    for (int i = 0; i + 1 < rank; i++) stride[i] = s *= dim[i];
+    const CUresult r = ((Fn)f)(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, rank, const_cast<void *>(base), dim, stride, box, one,
+                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+size_t fused_maps_bytes() { return SM_COUNT * sizeof(CUtensorMap); }
+
+cudaError_t fused_shot_maps(void *out, int nx, int ldz, const float *u0, const float *u1, const float *grad,
+                            const float *snap, int nslot)
+{
+    CUtensorMap *m = (CUtensorMap *)out;
+    std::memset(m, 0, fused_maps_bytes());
+    const cuuint64_t d2[3] = {(cuuint64_t)ldz, (cuuint64_t)nx, 2}, d3[3] = {(cuuint64_t)ldz, (cuuint64_t)nx, 3};
+    const cuuint64_t ds[4] = {(cuuint64_t)ldz, (cuuint64_t)nx, 2, (cuuint64_t)nslot};
+    const cuuint32_t lead[3] = {kFs, kFx + 8, 2}, own[4] = {kFz, kFx, 2, 1}, g[3] = {kFz, kFx, 3}, sl[4] = {kFs, kFx + 4, 2, 1};
+    cudaError_t e = cudaSuccess;
+    const float *u[2] = {u0, u1};
+    for (int b = 0; b < 2 && e == cudaSuccess; b++) {
+        e = encode(m + SM_LEAD + b, u[b], 3, d2, lead);
+        if (e == cudaSuccess) e = encode(m + SM_OWN + b, u[b], 3, d2, own);
+    }
+    if (e == cudaSuccess && grad) e = encode(m + SM_GRAD, grad, 3, d3, g);
+    if (e == cudaSuccess && snap && nslot > 0) {
+        e = encode(m + SM_SNAP_LEAD, snap, 4, ds, sl);
+        if (e == cudaSuccess) e = encode(m + SM_SNAP_OWN, snap, 4, ds, own);
+    }
+    return e;
+}
+
+static cudaError_t model_maps(CUtensorMap *m, int kind, const ModelDev &M)
+{
+    const cuuint64_t dim[2] = {(cuuint64_t)M.ldz, (cuuint64_t)M.nx};
+    const cuuint32_t halo[2] = {kFs, kFx + 4}, own[2] = {kFz, kFx};
+    const bool vti = kind == KIND_VTI;
+    const float *p[MM_COUNT] = {M.p1, vti ? M.fxx : M.p0, M.lbis, M.c13, M.p0, M.p2, M.irho, M.eps, M.gv2, M.gv3};
+    for (int i = 0; i < MM_COUNT; i++) {
+        std::memset(m + i, 0, sizeof(CUtensorMap));
+        const bool used = vti || i == MM_MU || i == MM_Q || i == MM_RHO || i == MM_IR;
+        if (!used) continue;
+        const cudaError_t e = encode(m + i, p[i], 2, dim, i < MM_RHO ? halo : own);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 cudaError_t launch_fused(int kind, const ShotDev *shots, const BandRef *bands, int nband, const TileRef *in, int nin,
                          const ModelDev &M, const StepConst &C, int it0, int it1, int flags, float dtg, unsigned *count,
                          int *status, cudaStream_t st)
@@ -1372,6 +1568,8 @@ cudaError_t launch_fused(int kind, const ShotDev *shots, const BandRef *bands, i
     A.dtg = dtg;
     A.count = count;
     A.status = status;
+    const cudaError_t e = model_maps(A.mm, kind, M);
+    if (e != cudaSuccess) return e;
     const bool g = (flags & F_GRAD) != 0;
     if (kind == KIND_VTI) return g ? launch_fused_t<true, true, false>(A, st) : launch_fused_t<true, false, false>(A, st);
     if (kind == KIND_AE) return g ? launch_fused_t<false, true, true>(A, st) : launch_fused_t<false, false, true>(A, st);

@@ -1,5 +1,6 @@
 // Host entry points of the kernels in kernels.cu.
 #pragma once
+#include <cstddef>
 #include "engine.h"
 
 namespace fwi2d {
@@ -35,6 +36,10 @@ void upload_fused_tables(const float *b1, const float *b2, const float *c2, cons
 cudaError_t launch_fused(int kind, const ShotDev *shots, const BandRef *bands, int nband, const TileRef *in, int nin,
                          const ModelDev &M, const StepConst &C, int it0, int it1, int flags, float dtg, unsigned *count,
                          int *status, cudaStream_t st);
+// tensor maps of a shot (ShotMap, host memory of fused_maps_bytes()); grad / snap may be null
+size_t fused_maps_bytes();
+cudaError_t fused_shot_maps(void *out, int nx, int ldz, const float *u0, const float *u1, const float *grad,
+                            const float *snap, int nslot);
 // closure sums of the six rows next to both ends of an axis of n samples (stride sn) on `lines` lines (stride sl)
 void launch_closures(const float *f, float *out, int lines, int ld, int n, long long sl, long long sn, cudaStream_t st);
 // top / bottom band kernel (rows clear of the x bands), zband_rows(split)

@@ -365,6 +365,8 @@ struct Plan {
     // device status word of the bounded waits (launch_take_timeout after each
     // pass) and its pinned host copy, read after the pass has finished
     DevBuf d_status;
+    std::vector<WinRef> wins;      // fused plans: interior windows (numbered as itiles)
+    DevBuf d_wins;
     DevBuf d_count;                // fused plans: arrivals of the launch's CTAs
     DevBuf d_maps;                 // and the shots' tensor maps: [shot], then [shot] of the replay fields
     int *h_status = nullptr;
@@ -1547,6 +1549,23 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
         P->marches.insert(P->marches.end(), U.marches.begin(), U.marches.end());
         P->bands.insert(P->bands.end(), U.bands.begin(), U.bands.end());
         P->itiles.insert(P->itiles.end(), U.itiles.begin(), U.itiles.end());
+        if (P->fused)
+            for (const TileRef &r : U.itiles) {
+                WinRef w;
+                w.shot = r.shot;
+                w.wx0 = r.wx0;
+                w.ox1 = r.ox1;
+                w.wz0 = r.wz0;
+                w.oz0 = r.oz0;
+                w.oz1 = r.oz1;
+                w.ef0 = S->inj_f_off[r.unit];
+                w.ef1 = S->inj_f_off[r.unit + 1];
+                w.ea0 = S->inj_a_off[r.unit];
+                w.ea1 = S->inj_a_off[r.unit + 1];
+                w.r0 = S->ext_f_off[r.unit];
+                w.r1 = S->ext_f_off[r.unit + 1];
+                P->wins.push_back(w);
+            }
         P->shots.push_back(std::move(S));
     }
     P->have_snapshots = p.sub > 0;
@@ -1556,6 +1575,7 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
     P->d_march.upload(P->marches, ctx->st);
     P->d_bands.upload(P->bands, ctx->st);
     P->d_itiles.upload(P->itiles, ctx->st);
+    P->d_wins.upload(P->wins, ctx->st);
     std::vector<ShotDev> sf(nshots), sa(nshots);
     for (int s = 0; s < nshots; s++) {
         shot_dev(*P, *P->shots[s], M, false, sf[s]);
@@ -1687,7 +1707,7 @@ static int launch_step(fwi2d_ctx *ctx, const Plan &P, const ShotDev *shots, cons
                              flags & STEP_EXTRACT, st);
         if (P.fused)
             CK(launch_fused(P.kind, shots, P.d_bands.as<BandRef>() + R.b0, R.b1 - R.b0,
-                            P.d_itiles.as<TileRef>() + R.i0, R.i1 - R.i0, md, P.C, it, it + 1, flags, P.dtg,
+                            P.d_wins.as<WinRef>() + R.i0, R.i1 - R.i0, md, P.C, it, it + 1, flags, P.dtg,
                             P.d_count.as<unsigned>(), P.d_status.as<int>(), st));
         else
             launch_ae_elastic_step(P.tshape, shots, tiles, ntiles, md, P.C, it, flags, P.dtg, st);
@@ -1733,7 +1753,7 @@ static long long launch_steps(fwi2d_ctx *ctx, const Plan &P, const ShotDev *shot
     if (it1 <= it0) return 0;
     if (P.fused && !P.ae) {
         const Plan::Wave &R = wave ? *wave : P.all;
-        CK(launch_fused(P.kind, shots, P.d_bands.as<BandRef>() + R.b0, R.b1 - R.b0, P.d_itiles.as<TileRef>() + R.i0,
+        CK(launch_fused(P.kind, shots, P.d_bands.as<BandRef>() + R.b0, R.b1 - R.b0, P.d_wins.as<WinRef>() + R.i0,
                         R.i1 - R.i0, md, P.C, it0, it1, flags, P.dtg, P.d_count.as<unsigned>(), P.d_status.as<int>(),
                         st));
         return 1;

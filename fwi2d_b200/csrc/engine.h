@@ -125,6 +125,15 @@ struct alignas(16) TileRef {
     int wz0, oz0, oz1;
 };
 
+// Interior window of a fused plan: it starts at (wx0, wz0) and owns the cells
+// [wx0, ox1) x [oz0, oz1); its injection entries of the forward [ef0, ef1) and of
+// the adjoint [ea0, ea1), its receivers [r0, r1).
+struct alignas(16) WinRef {
+    int shot, wx0, ox1, wz0;
+    int oz0, oz1, ef0, ef1;
+    int ea0, ea1, r0, r1;
+};
+
 // Work unit of the x-marching kernel: rows [xb, xe) (all clear of the x
 // boundary bands) of a z window of 2*blockDim.x cells starting at za (even,
 // -2 for the first window) that writes the cells of [oz0, oz1).  roff is the

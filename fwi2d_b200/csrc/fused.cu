@@ -256,7 +256,7 @@ struct alignas(64) FusedArgs {
     CUtensorMap mm[MM_COUNT];
     const ShotDev *shots;
     const BandRef *bands;   // x bands (side 2, 3), then z bands (side 0, 1)
-    const TileRef *in;
+    const WinRef *in;
     int nband, nunit;       // band units, all units
     ModelDev M;
     StepConst C;
@@ -376,7 +376,7 @@ __device__ __forceinline__ Imaging imaging(const ShotDev &S, const StepConst &C,
 
 // by one thread
 template <bool VTI, bool GRAD, bool AE>
-__device__ __forceinline__ void issue_lead(const FusedArgs &A, const ShotDev &S, const TileRef &tr, int it, bool model,
+__device__ __forceinline__ void issue_lead(const FusedArgs &A, const ShotDev &S, const WinRef &tr, int it, bool model,
                                            bool fields, float *sm, unsigned long long *bar)
 {
     using L = InLayout<VTI, GRAD, AE>;
@@ -400,7 +400,7 @@ __device__ __forceinline__ unsigned lead_bytes(bool model)
 
 // model: density and its reciprocal (VTI imaging: its coefficients); snapshots (FP32; no step of this launch writes them)
 template <bool VTI, bool GRAD, bool AE>
-__device__ __forceinline__ void issue_own_static(const FusedArgs &A, const ShotDev &S, const TileRef &tr, int it, bool model,
+__device__ __forceinline__ void issue_own_static(const FusedArgs &A, const ShotDev &S, const WinRef &tr, int it, bool model,
                                                  float *sm, unsigned long long *bar)
 {
     using L = InLayout<VTI, GRAD, AE>;
@@ -435,7 +435,7 @@ __device__ __forceinline__ void issue_own_static(const FusedArgs &A, const ShotD
     }
 }
 template <bool VTI, bool GRAD, bool AE>
-__device__ __forceinline__ void issue_own_fields(const FusedArgs &A, const ShotDev &S, const TileRef &tr, int it, float *sm,
+__device__ __forceinline__ void issue_own_fields(const FusedArgs &A, const ShotDev &S, const WinRef &tr, int it, float *sm,
                                                  unsigned long long *bar)
 {
     using L = InLayout<VTI, GRAD, AE>;
@@ -446,7 +446,7 @@ __device__ __forceinline__ void issue_own_fields(const FusedArgs &A, const ShotD
 
 // 16-bit snapshots of a window: converted on the way to shared memory by all threads
 template <bool VTI, bool GRAD, bool AE>
-__device__ __forceinline__ void load_snaps16(const FusedArgs &A, const ShotDev &S, const TileRef &tr, int it, float *sm)
+__device__ __forceinline__ void load_snaps16(const FusedArgs &A, const ShotDev &S, const WinRef &tr, int it, float *sm)
 {
     using L = InLayout<VTI, GRAD, AE>;
     const int prec = A.C.snap_prec;
@@ -475,10 +475,10 @@ __device__ __forceinline__ void load_snaps16(const FusedArgs &A, const ShotDev &
     }
 }
 
-// The window's step, its Lead group present; mid() runs between its halves.
-template <bool VTI, bool GRAD, bool AE, class Mid>
-__device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S, const TileRef &tr, const int it, float *sm,
-                                            Mid mid)
+// The window's step: wait_lead() before it reads the Lead group, mid() between its halves.
+template <bool VTI, bool GRAD, bool AE, class Lead, class Mid>
+__device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S, const WinRef &tr, const int it, float *sm,
+                                            Lead wait_lead, Mid mid)
 {
     using L = InLayout<VTI, GRAD, AE>;
     const StepConst &C = A.C;
@@ -488,8 +488,15 @@ __device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S
     const bool do_grad = im.on;
     const int tx = t >> 4, pz = 2 * (t & 15);
     const int gx = tr.wx0 + tx, gz = tr.wz0 + pz;
-    const bool ownx = gx >= tr.ox0 && gx < tr.ox1;
+    const bool ownx = gx < tr.ox1;
     const bool own0 = ownx && gz >= tr.oz0 && gz < tr.oz1, own1 = ownx && gz + 1 >= tr.oz0 && gz + 1 < tr.oz1;
+    float2 tzv = make_float2(0.f, 0.f);   // used in the second half
+    float txv = 0.f;
+    if (own0 || own1) {
+        tzv = *reinterpret_cast<const float2 *>(S.tz + gz);
+        txv = S.tx[gx];
+    }
+    const bool here = wait_lead();
     const float *U0 = sm + L::U0 + 2 * kFs, *U1 = sm + L::U1 + 2 * kFs;   // indexed as the 2-halo arrays
     const float *MU = sm + L::MU, *Q = sm + L::Q;
     float *P = sm + L::P, *R = sm + L::R, *T = sm + L::S, *P1 = sm + L::P1;
@@ -562,8 +569,7 @@ __device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S
     }
     // receivers (forward): one thread per receiver of this window
     if (!GRAD && (A.flags & F_EXTRACT)) {
-        const int r0 = S.ext_off[tr.unit], r1 = S.ext_off[tr.unit + 1];
-        for (int e = r0 + t; e < r1; e += kFt) {
+        for (int e = tr.r0 + t; e < tr.r1; e += kFt) {
             const ExtEntry &E = S.ext[e];
             const float *U = sm + (E.comp == 0 ? L::U0 : L::U1) + (E.gx0 - tr.wx0 + 4) * kFs + (E.gz0 - tr.wz0 + 4);
             float o = 0.f;
@@ -575,7 +581,7 @@ __device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S
         }
     }
     const float2 a00 = ld2(U0, i), b00 = ld2(U1, i);
-    if (!mid()) return false;   // the Own group is there; U and the coefficients are free for the next window
+    if (!mid(here)) return false;   // the Own group is there; U and the coefficients are free for the next window
 
     // ---- mixed terms
     auto along_x = [&](const float *p, float s) {
@@ -593,7 +599,7 @@ __device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S
 
     const int cell = gx * ldz + gz;
     // sources, cell by cell in the reference's order
-    const int e0 = S.inj_off[tr.unit], e1 = S.inj_off[tr.unit + 1];
+    const int e0 = GRAD ? tr.ea0 : tr.ef0, e1 = GRAD ? tr.ea1 : tr.ef1;
     if (e0 < e1) {
         const float *srcrow = S.src + (long long)it * S.nsrc;
         for (int e = e0; e < e1; e++) {
@@ -611,12 +617,6 @@ __device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S
         }
     }
     float *pn = S.u[it & 1];   // prev in, next out
-    float2 tzv = make_float2(0.f, 0.f);
-    float txv = 0.f;
-    if (own0 || own1) {
-        tzv = *reinterpret_cast<const float2 *>(S.tz + gz);
-        txv = S.tx[gx];
-    }
     // leapfrog: dt^2 n / rho + 2 curr - prev, tapered; prev takes its second taper here
     const int oi = tx * kFz + pz;
     float2 p0 = ld2(sm + L::PV0, oi), p1 = ld2(sm + L::PV1, oi);
@@ -1294,7 +1294,7 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
 }
 
 #ifndef FUSED_FWD_BLOCKS
-#define FUSED_FWD_BLOCKS 4
+#define FUSED_FWD_BLOCKS 5
 #endif
 #ifndef FUSED_GRAD_BLOCKS
 #define FUSED_GRAD_BLOCKS 4
@@ -1312,9 +1312,9 @@ __global__ void __launch_bounds__(kFt, VTI && GRAD ? 3 : (GRAD ? FUSED_GRAD_BLOC
 fused_steps(const __grid_constant__ FusedArgs A)
 {
     extern __shared__ __align__(1024) float sm[];
-    static_assert(sizeof(ShotDev) % 16 == 0 && sizeof(TileRef) % 16 == 0, "copied in 16-byte pieces");
+    static_assert(sizeof(ShotDev) % 16 == 0 && sizeof(WinRef) % 16 == 0, "copied in 16-byte pieces");
     __shared__ __align__(16) ShotDev S_[2];
-    __shared__ __align__(16) TileRef T_[4];
+    __shared__ __align__(16) WinRef T_[4];
     const int G = gridDim.x;
     // slots blockIdx.x, + G, ... of the units (band units first) rotated so that, with
     // fewer than two units per CTA, the band units (the longest) get a CTA of their own
@@ -1343,8 +1343,8 @@ fused_steps(const __grid_constant__ FusedArgs A)
             bar_init(own);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
-        fetch16(&T_[0], window(0), sizeof(TileRef), 0);
-        fetch16(&T_[1], window(1), sizeof(TileRef), 32);
+        fetch16(&T_[0], window(0), sizeof(WinRef), 0);
+        fetch16(&T_[1], window(1), sizeof(WinRef), 32);
         fetch16(&S_[0], A.shots + window(0)->shot, sizeof(ShotDev), 64);
         cp_wait();
         __syncthreads();
@@ -1363,7 +1363,7 @@ fused_steps(const __grid_constant__ FusedArgs A)
         }
         for (int k = 0; k < nw; k++, q++) {
             const ShotDev &S = S_[q & 1], &Sn = S_[(q + 1) & 1];
-            const TileRef &tr = T_[q & 3], &tn = T_[(q + 1) & 3];
+            const WinRef &tr = T_[q & 3], &tn = T_[(q + 1) & 3];
             const bool active = it < S.nt - 1;
             if (k == 0) {
                 // the first window of a step: what no step writes, then the meeting, then the fields
@@ -1383,12 +1383,12 @@ fused_steps(const __grid_constant__ FusedArgs A)
                     issue_own_fields<VTI, GRAD, AE>(A, S, tr, it, sm, own);
                 }
             }
-            fetch16(&T_[(q + 2) & 3], window(q + 2), sizeof(TileRef), 32);
+            fetch16(&T_[(q + 2) & 3], window(q + 2), sizeof(WinRef), 32);
             fetch16(&S_[(q + 1) & 1], A.shots + tn.shot, sizeof(ShotDev), 64);
             // between the halves: the Own group and the next entries have arrived, all
             // threads have left the first half
-            auto ahead = [&]() {
-                const bool ok = !active || wait_bar(A, own, par_own, it);
+            auto ahead = [&](bool lead_ok) {
+                const bool ok = !active || (wait_bar(A, own, par_own, it) && lead_ok);
                 cp_wait();
                 if (__syncthreads_or(!ok)) return false;
                 if (k + 1 < nw && it < Sn.nt - 1 && threadIdx.x == 0) {
@@ -1399,10 +1399,10 @@ fused_steps(const __grid_constant__ FusedArgs A)
                 return true;
             };
             if (active) {
-                const bool ok = wait_bar(A, lead, par_lead, it);
-                if (__syncthreads_or(!ok)) return;
-                if (!window_step<VTI, GRAD, AE>(A, S, tr, it, sm, ahead)) return;
-            } else if (!ahead()) {
+                if (!window_step<VTI, GRAD, AE>(
+                        A, S, tr, it, sm, [&]() { return wait_bar(A, lead, par_lead, it); }, ahead))
+                    return;
+            } else if (!ahead(true)) {
                 return;
             }
             if (k + 1 == nw) fence_async();   // this step's writes, before the arrival
@@ -1549,7 +1549,7 @@ static cudaError_t model_maps(CUtensorMap *m, int kind, const ModelDev &M)
     return cudaSuccess;
 }
 
-cudaError_t launch_fused(int kind, const ShotDev *shots, const BandRef *bands, int nband, const TileRef *in, int nin,
+cudaError_t launch_fused(int kind, const ShotDev *shots, const BandRef *bands, int nband, const WinRef *in, int nin,
                          const ModelDev &M, const StepConst &C, int it0, int it1, int flags, float dtg, unsigned *count,
                          int *status, cudaStream_t st)
 {

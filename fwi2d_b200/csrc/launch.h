@@ -33,7 +33,7 @@ void launch_elastic_march(bool vti, const ShotDev *shots, const MarchRef *units,
 // gave up.
 constexpr int kFusedZ = 32, kFusedX = 16, kFusedBand = 28;
 void upload_fused_tables(const float *b1, const float *b2, const float *c2, const float *c1, const float *sc);
-cudaError_t launch_fused(int kind, const ShotDev *shots, const BandRef *bands, int nband, const TileRef *in, int nin,
+cudaError_t launch_fused(int kind, const ShotDev *shots, const BandRef *bands, int nband, const WinRef *in, int nin,
                          const ModelDev &M, const StepConst &C, int it0, int it1, int flags, float dtg, unsigned *count,
                          int *status, cudaStream_t st);
 // tensor maps of a shot (ShotMap, host memory of fused_maps_bytes()); grad / snap may be null

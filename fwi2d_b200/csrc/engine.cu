@@ -323,7 +323,8 @@ struct Plan {
     int nza = 0, ldzw = 0, nx_max = 0;
     float Kw = 0.f, val0 = 0.f;
     StepConst Cw;
-    DevBuf wK, wIR;
+    DevBuf wK, wIR, wzclos;
+    int model_nx = 0;
     std::vector<TileRef> wtiles;
     DevBuf d_wtiles, d_wshots_f, d_wshots_a;
     std::vector<InitCell> wicells[2];
@@ -333,8 +334,10 @@ struct Plan {
     {
         ModelDev m;
         std::memset(&m, 0, sizeof(m));
+        m.nx = model_nx;
         m.nz = nza;
         m.ldz = ldzw;
+        m.zclos = wzclos.as<float>();
         m.p0 = wK.as<float>();
         m.p1 = wIR.as<float>();
         return m;
@@ -448,17 +451,18 @@ static void upload_model_values(fwi2d_ctx *ctx, const float *model)
     // device copies straight from the caller's array (which may be pinned)
     up(M.p0, model);
     up(M.p1, model + nxz);
+    // z-closure sums of mu (acoustic: 1/rho) for the fused time loop
+    M.zclos.ensure((size_t)96 * nx * sizeof(float));
+    launch_closures(M.p1.as<float>(), M.zclos.as<float>(), nx, nx, nz, M.ldz, 1, ctx->st);
+    CK(cudaGetLastError());
     if (kind != KIND_ACOUSTIC) {
         up(M.p2, model + 2 * nxz);
         M.irho.ensure(pitched * sizeof(float));
         k_reciprocal<<<592, 256, 0, ctx->st>>>(M.p2.as<float>(), M.irho.as<float>(), (long long)pitched);
-        M.zclos.ensure((size_t)96 * nx * sizeof(float));
-        launch_closures(M.p1.as<float>(), M.zclos.as<float>(), nx, nx, nz, M.ldz, 1, ctx->st);
         CK(cudaGetLastError());
     } else {
         M.p2.release();
         M.irho.release();
-        M.zclos.release();
     }
     // a live plan's graphs hold these addresses: an update keeps the buffers
     if (kind != KIND_VTI) {
@@ -524,6 +528,7 @@ static const MarchShape kMarchShapes[] = {{224, 64}, {256, 64}, {192, 64}, {128,
 static const int kNumMarch = sizeof(kMarchShapes) / sizeof(kMarchShapes[0]);
 static const int kBandTile = 3;    // (TZ, TX) = (32, 8): band windows of 8 columns own 6
 static const int kBand = 6;
+static const int kAcousticTile = 2;   // tile shape (32 x 16) of the acoustic time loop's units, and of a fluid layer's
 static const int kFusedZ0 = 4;     // first row of the fused step's interior windows
 // Framed tile plans: the tile kernel's interior path on windows of one of
 // these tile shapes over the cells clear of all four boundary bands, and the
@@ -1076,6 +1081,7 @@ static void shot_dev_fluid(const Plan &P, const ShotPlan &s, bool adjoint, ShotD
     d.den = w.den.as<float>();
     d.tz = w.tz.as<float>();
     d.tx = w.tx.as<float>();
+    d.xclos = w.xclos.as<float>();
     d.halo_save = w.halo.as<float>();
 }
 
@@ -1256,6 +1262,17 @@ static void build_xclos(fwi2d_ctx *ctx, Plan &P)
 {
     if (!P.fused) return;
     const ModelState &M = ctx->M;
+    if (P.ae) {
+        // the fluid layer's 1/rho
+        P.wzclos.ensure((size_t)96 * M.nx * sizeof(float));
+        launch_closures(P.wIR.as<float>(), P.wzclos.as<float>(), M.nx, M.nx, P.nza, P.ldzw, 1, ctx->st);
+        for (auto &S : P.shots) {
+            ShotPlan &W = *S->fluid;
+            W.xclos.ensure((size_t)96 * P.ldzw * sizeof(float));
+            launch_closures(P.wIR.as<float>() + (long long)W.x0 * P.ldzw, W.xclos.as<float>(), P.nza, P.ldzw, W.nx, 1,
+                            P.ldzw, ctx->st);
+        }
+    }
     const size_t n = (size_t)96 * M.ldz;
     for (auto &S : P.shots) {
         S->xclos.ensure((M.kind == KIND_VTI ? 2 : 1) * n * sizeof(float));
@@ -1323,6 +1340,7 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
         P->ae_src_fluid = p.acoustic_source != 0;
         P->nza = p.nza;
         P->ldzw = round_up(p.nza, 32);
+        P->model_nx = M.nx;
         const float rw = p.water_density;
         P->Kw = rw * p.water_velocity * p.water_velocity;
         const float h = (float)((double)M.dz * (17.0 / 48));   // interface row weight, we_op.cpp:2490
@@ -1335,9 +1353,9 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
     // shape: the requested one, else the marching kernel where it has enough
     // units to fill the GPU, else the first tile shape that fits every shot
     auto shape_ok = [&](int i) {
-        if ((acoustic || ae) && !acoustic_shape_ok(i) && !(ae && i == fused_shape())) return false;
+        if ((acoustic || ae) && !acoustic_shape_ok(i) && i != fused_shape()) return false;
         for (int s = 0; s < nshots; s++)
-            if (!shape_fits(i, shots[s].nx, M.nz)) return false;
+            if (!shape_fits(acoustic && i == fused_shape() ? kAcousticTile : i, shots[s].nx, M.nz)) return false;
         return true;
     };
     int shape = p.tile_shape;
@@ -1359,7 +1377,7 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
     P->march = is_march_shape(shape);
     P->framed = is_framed_shape(shape);
     P->fused = shape == fused_shape();
-    P->tshape = P->march || P->framed || P->fused ? kBandTile : shape;
+    P->tshape = P->fused ? kAcousticTile : P->march || P->framed ? kBandTile : shape;
     if (P->framed) P->ishape = framed_tile_shape(shape);
     P->band_split = (P->march || P->framed) && band_split_for(nshots, M.nz);
     elastic_tile_shape(P->tshape, &P->TZ, &P->TX);
@@ -1398,7 +1416,8 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
         S->nx = sh.nx;
         S->nt = sh.nt;
         S->ncomp = acoustic ? 1 : 2;
-        const ShotUnits U = make_units(shape, s, sh.nx, M.nz, P->band_split);
+        const bool loop = P->fused && !acoustic;   // band units and windows
+        const ShotUnits U = make_units(P->fused && acoustic ? kAcousticTile : shape, s, sh.nx, M.nz, P->band_split);
         const int nunits = U.nunits();
         S->ntr_src = src_fluid ? sh.src_water.ntr : sh.src.ntr;
         S->ncomp_src = acoustic || src_fluid ? 1 : (p.mt ? 3 : 2);
@@ -1509,7 +1528,7 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
         S->d_mrow_f.upload(S->mrow_f, ctx->st);
         S->d_mrow_a.upload(S->mrow_a, ctx->st);
         std::vector<int4> brf, bra;
-        if (P->fused) {
+        if (loop) {
             brf = band_ranges(U, S->inj_f, S->inj_f_off);
             bra = band_ranges(U, S->inj_a, S->inj_a_off);
             S->d_brange_f.upload(brf, ctx->st);
@@ -1549,7 +1568,7 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
         P->marches.insert(P->marches.end(), U.marches.begin(), U.marches.end());
         P->bands.insert(P->bands.end(), U.bands.begin(), U.bands.end());
         P->itiles.insert(P->itiles.end(), U.itiles.begin(), U.itiles.end());
-        if (P->fused)
+        if (loop)
             for (const TileRef &r : U.itiles) {
                 WinRef w;
                 w.shot = r.shot;
@@ -1584,7 +1603,7 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
     for (int s = 0; s < nshots; s++) sf[s].ckpt = P->shots[s]->ckpt.as<float>();
     const size_t mb = fused_maps_bytes();
     std::vector<unsigned char> maps;
-    if (P->fused) {
+    if (P->fused && !acoustic) {
         const bool replay = p.checkpoint_every > 0, f32 = p.snapshot_precision == FWI2D_SNAP_FP32;
         maps.resize((replay ? 2 : 1) * nshots * mb);
         for (int s = 0; s < nshots; s++) {
@@ -1637,7 +1656,7 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
                 ShotDev a = sa[s];
                 a.snap = win;
                 a.snap_first = (int)base;
-                if (P->fused) r.maps = P->d_maps.as<char>() + (nshots + s) * mb;
+                if (P->fused && !acoustic) r.maps = P->d_maps.as<char>() + (nshots + s) * mb;
                 sr[(size_t)k * nshots + s] = r;
                 sc[(size_t)k * nshots + s] = a;
             }
@@ -1705,12 +1724,7 @@ static int launch_step(fwi2d_ctx *ctx, const Plan &P, const ShotDev *shots, cons
         const ShotDev *wshots = (adj ? P.d_wshots_a : P.d_wshots_f).as<ShotDev>();
         launch_ae_fluid_step(P.tshape, wshots, P.d_wtiles.as<TileRef>() + R.w0, R.w1 - R.w0, P.wdev(), P.Cw, it,
                              flags & STEP_EXTRACT, st);
-        if (P.fused)
-            CK(launch_fused(P.kind, shots, P.d_bands.as<BandRef>() + R.b0, R.b1 - R.b0,
-                            P.d_wins.as<WinRef>() + R.i0, R.i1 - R.i0, md, P.C, it, it + 1, flags, P.dtg,
-                            P.d_count.as<unsigned>(), P.d_status.as<int>(), st));
-        else
-            launch_ae_elastic_step(P.tshape, shots, tiles, ntiles, md, P.C, it, flags, P.dtg, st);
+        launch_ae_elastic_step(P.tshape, shots, tiles, ntiles, md, P.C, it, flags, P.dtg, st);
         launch_ae_couple(shots + R.s0, wshots + R.s0, R.s1 - R.s0, P.nx_max, md, P.C, it, flags, P.dtg, P.Kw, P.val0,
                          adj ? -1 : 1, st);
         return 3;
@@ -1751,11 +1765,32 @@ static long long launch_steps(fwi2d_ctx *ctx, const Plan &P, const ShotDev *shot
                               int flags, cudaStream_t st, const Plan::Wave *wave = nullptr)
 {
     if (it1 <= it0) return 0;
-    if (P.fused && !P.ae) {
+    if (P.fused) {
         const Plan::Wave &R = wave ? *wave : P.all;
+        unsigned *count = P.d_count.as<unsigned>();
+        int *status = P.d_status.as<int>();
+        if (P.kind == KIND_ACOUSTIC) {
+            CK(launch_acoustic_loop(shots, P.d_tiles.as<TileRef>() + R.t0, R.t1 - R.t0, md, P.C, it0, it1, flags, P.dtg,
+                                    count, status, st));
+            return 1;
+        }
+        FluidArgs W;
+        if (P.ae) {
+            const bool adj = (flags & STEP_GRAD) != 0;
+            W.shots = (adj ? P.d_wshots_a : P.d_wshots_f).as<ShotDev>();
+            W.tiles = P.d_wtiles.as<TileRef>() + R.w0;
+            W.ntile = R.w1 - R.w0;
+            W.ncol = P.nx_max;
+            W.s0 = R.s0;
+            W.nshot = R.s1 - R.s0;
+            W.sign = adj ? -1 : 1;
+            W.M = P.wdev();
+            W.C = P.Cw;
+            W.Kw = P.Kw;
+            W.val0 = P.val0;
+        }
         CK(launch_fused(P.kind, shots, P.d_bands.as<BandRef>() + R.b0, R.b1 - R.b0, P.d_wins.as<WinRef>() + R.i0,
-                        R.i1 - R.i0, md, P.C, it0, it1, flags, P.dtg, P.d_count.as<unsigned>(), P.d_status.as<int>(),
-                        st));
+                        R.i1 - R.i0, md, P.C, it0, it1, flags, P.dtg, count, status, P.ae ? &W : nullptr, st));
         return 1;
     }
     long long n = 0;
@@ -1940,8 +1975,9 @@ static void set_shots(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, const
 {
     REQ(par != nullptr && shots != nullptr && nshots > 0, "no shots");
     fwi2d_params p = *par;
-    bool fused = ctx->M.kind != KIND_ACOUSTIC;
-    for (int i = 0; i < nshots && fused; i++) fused = shape_fits(fused_shape(), shots[i].nx, ctx->M.nz);
+    const int fshape = ctx->M.kind == KIND_ACOUSTIC ? kAcousticTile : fused_shape();
+    bool fused = true;
+    for (int i = 0; i < nshots && fused; i++) fused = shape_fits(fshape, shots[i].nx, ctx->M.nz);
     // the fused time loop is the fastest shape wherever it fits: nothing to time
     if (p.tile_shape < 0 && ctx->M.kind >= 0 && !fused) {
         static std::vector<std::pair<std::string, int>> cache;
@@ -2857,7 +2893,7 @@ int fwi2d_ctx_create(int device, fwi2d_ctx **out)
     c->st = c->own;
     const SbpTables &t = sbp_tables();
     upload_sbp_tables(&t.b1[0][0], &t.b2[0][0][0], t.c2, t.c1, t.sc, t.hc);
-    upload_fused_tables(&t.b1[0][0], &t.b2[0][0][0], t.c2, t.c1, t.sc);
+    upload_fused_tables(&t.b1[0][0], &t.b2[0][0][0], t.c2, t.c1, t.sc, t.hc);
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
     *out = c.release();
@@ -3005,7 +3041,7 @@ int fwi2d_plan_info(fwi2d_ctx *ctx, long long *lf, long long *la, int *shape, lo
     REQ(ctx, "null context");
     Plan &P = need_plan(ctx);
     const long long per = (P.march || P.framed || P.ae) ? 3 : 1;
-    const bool loop = P.fused && !P.ae;   // one launch per run of steps
+    const bool loop = P.fused;   // one launch per run of steps
     const long long nseg = P.ckpt > 0 ? (long long)P.cuts.size() - 1 : 0;
     const long long acf = P.kind == KIND_ACOUSTIC ? 1 : 0;
     // per wave -- forward: init, steps, last sample (+ checkpoint copies);

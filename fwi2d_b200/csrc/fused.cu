@@ -28,6 +28,7 @@
 #include "engine.h"
 #include "sbp.cuh"
 #include "snap.cuh"
+#include "asat.cuh"
 #include "launch.h"
 
 namespace fwi2d {
@@ -264,37 +265,44 @@ struct alignas(64) FusedArgs {
     float dtg;
     unsigned *count;        // arrivals of this launch's steps, zero at its start
     int *status;            // step + 1 of a wait that gave up
+    FluidArgs W;            // acoustic-elastic: the fluid layer
 };
 
 // ---- the meeting point of a launch's CTAs -------------------------------------
-__device__ __forceinline__ void arrive(const FusedArgs &A)
+__device__ __forceinline__ void arrive(unsigned *count)
 {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(A.count) : "memory");
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
 }
-__device__ __forceinline__ bool reached(const FusedArgs &A, unsigned target)
+__device__ __forceinline__ bool reached(const unsigned *count, unsigned target)
 {
     unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(A.count) : "memory");
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
     return v >= target;
 }
 // Waits until every CTA has finished the steps before `it`.  The launch is
 // cooperative, so all of them are resident.  Bounded twice: past StepConst::spin
 // polls the step is reported, past kHardPolls more the CTA leaves (false).
 constexpr int kHardPolls = 1 << 22;
-__device__ __forceinline__ bool meet(const FusedArgs &A, int it)
+__device__ __forceinline__ bool meet_at(const unsigned *count, int *status, int spin, unsigned rounds, int it)
 {
     int lost = 0;
-    if (threadIdx.x == 0 && it > A.it0) {
-        const unsigned target = (unsigned)(it - A.it0) * gridDim.x;
+    if (threadIdx.x == 0 && rounds > 0) {
+        const unsigned target = rounds * gridDim.x;
         bool ok = false;
-        for (int k = 0; k < A.C.spin && !ok; k++) ok = reached(A, target);
+        for (int k = 0; k < spin && !ok; k++) ok = reached(count, target);
         if (!ok) {
-            atomicCAS(A.status, 0, it + 1);
-            for (int k = 0; k < kHardPolls && !ok; k++) ok = reached(A, target);
+            atomicCAS(status, 0, it + 1);
+            for (int k = 0; k < kHardPolls && !ok; k++) ok = reached(count, target);
             lost = !ok;
         }
     }
     return !__syncthreads_or(lost);
+}
+// (acoustic-elastic steps have two meetings: before the step and before its coupling)
+template <bool AE>
+__device__ __forceinline__ bool meet(const FusedArgs &A, int it)
+{
+    return meet_at(A.count, A.status, A.C.spin, (AE ? 2u : 1u) * (unsigned)(it - A.it0), it);
 }
 
 // max |next| of a CTA for the scale of the next 16-bit snapshot
@@ -927,7 +935,7 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
     const float *curr = Sp->u[(it + 1) & 1];
     float *pn = Sp->u[it & 1];
 
-    if (first && !meet(A, it)) return false;
+    if (first && !meet<AE>(A, it)) return false;
     if (it >= nt - 1) return true;
 
     float p0 = 0.f, p1 = 0.f, g0 = 0.f, g1 = 0.f, g2 = 0.f, c0 = 0.f, c1 = 0.f;
@@ -1293,12 +1301,295 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
     return true;
 }
 
-#ifndef FUSED_FWD_BLOCKS
-#define FUSED_FWD_BLOCKS 5
-#endif
-#ifndef FUSED_GRAD_BLOCKS
-#define FUSED_GRAD_BLOCKS 4
-#endif
+// ---------------------------------------------------------------------------
+// Acoustic unit: a window of 32 (z) x 16 (x) cells of a shot's pressure (or of
+// the fluid layer's potential, FLUID), the tile kernel's windows and arithmetic
+// (acoustic.cuh, src/cpp/we_op.cpp:1937-2134).  Windows clear of the closures
+// take the z-pair form of the elastic windows; the others update two cells per
+// thread through the general forms.
+// ---------------------------------------------------------------------------
+template <bool GRAD>
+struct AcLayout {
+    static constexpr int U = 0, IR = kFu, F = IR + kFw, RED = F + (GRAD ? kFw : 0), FLOATS = RED + 8;
+};
+
+// imaging condition of one cell at the start of a step (nl_we_op_a::compute_gradients, we_op.cpp:1883-1935)
+__device__ __forceinline__ void acoustic_image(float &g0, float &g1, float t0, float t1, float t2, float t3, float f, float adj,
+                                               float K, float fp, float fm, float w, float dtg, int itf, int last)
+{
+    const double c = (double)w * 1.0 / (double)(dtg * K * K) * (double)adj;
+    const float s = itf > 0 && itf < last ? fp - 2 * f + fm : itf == 0 ? fp - f : -f + fm;
+    g0 = (float)((double)g0 - c * (double)s);
+    if (itf == 0) g1 = (float)((double)g1 + (double)w * 0.5 * (double)dtg * (double)(t2 * t0 + t3 * t1));
+    else g1 += w * dtg * (t2 * t0 + t3 * t1);
+}
+
+template <bool GRAD, bool FLUID, class Meet>
+__device__ __forceinline__ bool acoustic_unit(const ShotDev *__restrict__ Sp, const ModelDev &M, const StepConst &C,
+                                              const TileRef tr, const int it, const int flags, const float dtg,
+                                              const bool keep, float *sm, Meet meet_first)
+{
+    using L = AcLayout<GRAD>;
+    const int t = threadIdx.x, nt = Sp->nt, nx = Sp->nx, nz = Sp->nz, ldz = Sp->ldz, mld = M.ldz;
+    const int wx0 = tr.wx0, wz0 = tr.wz0, prec = C.snap_prec;
+    const long long mofs = (long long)Sp->x0 * mld, nxz = (long long)nx * ldz;
+    const bool inner = wx0 >= 6 && wx0 + kFx + 6 <= nx && wz0 >= 6 && wz0 + kFz + 6 <= nz && (wz0 & 3) == 0;
+    // snapshot (nt-1-it)/sub, skipped at it == 0 (we_op.cpp:2044-2046)
+    const int kk = nt - 1 - it, itf = GRAD ? by(kk, C.sub) : 0, last = by(nt, C.sub);
+    const bool do_grad = GRAD && it != 0 && kk > 0 && itf * C.sub == kk;
+    float finv = 1.f;
+    if (GRAD && do_grad && prec != SNAP_FP32) finv = 1.f / snap_scale(Sp->snap_amax, itf);
+    const int xr = t / 10, xq = 4 * (t - 10 * xr);
+
+    // ---- what no step writes
+    if (inner) {
+        if (t < (kFx + 4) * 10) {
+            const int s = xr * kFs + xq;
+            if (!keep) cp16(sm + L::IR + s, M.p1 + mofs + (long long)(wx0 - 2 + xr) * mld + wz0 - 4 + xq, true);
+            if (GRAD && do_grad) {
+                const long long so = (long long)itf * Sp->snap_slot + (long long)(wx0 - 2 + xr) * ldz + wz0 - 4 + xq;
+                if (prec == SNAP_FP32) cp16(sm + L::F + s, (const float *)Sp->snap + so, true);
+                else *reinterpret_cast<float4 *>(sm + L::F + s) = snap_load4(Sp->snap, so, prec, finv);
+            }
+        }
+    } else {
+        for (int i = t; i < kFw; i += kFt) {
+            const int r = i / kFs, q = i - r * kFs, x = wx0 - 2 + r, z = wz0 - 4 + q;
+            const bool in = x >= 0 && x < nx && z >= 0 && z < nz;
+            if (!keep) sm[L::IR + i] = in ? M.p1[mofs + (long long)x * mld + z] : 0.f;
+            if (GRAD && do_grad)
+                sm[L::F + i] = in ? snap_load(Sp->snap, (long long)itf * Sp->snap_slot + (long long)x * ldz + z, prec, finv) : 0.f;
+        }
+    }
+    const float *curr = Sp->u[(it + 1) & 1];
+    float *pn = Sp->u[it & 1];
+    if (!meet_first()) {
+        cp_wait();
+        return false;
+    }
+    if (it >= nt - 1) {
+        cp_wait();
+        return true;
+    }
+    if (inner) {
+        if (t < (kFx + 8) * 10)
+            cp16(sm + L::U + xr * kFs + xq, curr + (long long)(wx0 - 4 + xr) * ldz + wz0 - 4 + xq, true);
+        cp_wait();
+    } else {
+        float v[4];
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+            const int i = t + h * kFt, r = i / kFs, q = i - r * kFs, x = wx0 - 4 + r, z = wz0 - 4 + q;
+            v[h] = i < kFu && x >= 0 && x < nx && z >= 0 && z < nz ? __ldcg(curr + (long long)x * ldz + z) : 0.f;
+        }
+#pragma unroll
+        for (int h = 0; h < 4; h++)
+            if (t + h * kFt < kFu) sm[L::U + t + h * kFt] = v[h];
+    }
+    __syncthreads();
+
+    const float *U = sm + L::U + 2 * kFs, *IR = sm + L::IR, *F = sm + L::F;   // one index for all
+    if (!GRAD && (flags & F_EXTRACT)) {
+        const int r1 = Sp->ext_off[tr.unit + 1];
+        for (int e = Sp->ext_off[tr.unit] + t; e < r1; e += kFt) {
+            const ExtEntry &E = Sp->ext[e];
+            const float *u = sm + L::U + (E.gx0 - wx0 + 4) * kFs + (E.gz0 - wz0 + 4);
+            float o = 0.f;
+#pragma unroll
+            for (int a = 0; a < 3; a++)
+#pragma unroll
+                for (int b = 0; b < 3; b++) o += E.w[a * 3 + b] * u[a * kFs + b];
+            Sp->rcv[(long long)it * Sp->nrcv + E.row] = o;
+        }
+    }
+    const int e0 = Sp->inj_off[tr.unit], e1 = Sp->inj_off[tr.unit + 1];
+    const float *srcrow = Sp->src + (long long)it * Sp->nsrc;
+    const int slot = by(it, C.sub);
+    const bool store = !GRAD && (flags & F_STORE) && slot * C.sub == it;
+    float amax = 0.f;
+
+    if (inner) {
+        const int tx = t >> 4, pz = 2 * (t & 15), gx = wx0 + tx, gz = wz0 + pz, i = (tx + 2) * kFs + 4 + pz;
+        const bool ownx = gx >= tr.ox0 && gx < tr.ox1;
+        const bool own0 = ownx && gz >= tr.oz0 && gz < tr.oz1, own1 = ownx && gz + 1 >= tr.oz0 && gz + 1 < tr.oz1;
+        const long long cell = (long long)gx * ldz + gz;
+        const float2 p = __ldcg(reinterpret_cast<const float2 *>(pn + cell));
+        const float2 K = *reinterpret_cast<const float2 *>(M.p0 + mofs + (long long)gx * mld + gz);
+        const float2 tzv = *reinterpret_cast<const float2 *>(Sp->tz + gz), tzx = bc2(Sp->tx[gx]);
+        const float2 um2 = ld2(U, i - 2 * kFs), um1 = ld2(U, i - kFs), u0 = ld2(U, i), up1 = ld2(U, i + kFs),
+                     up2 = ld2(U, i + 2 * kFs), ulo = ld2(U, i - 2), uhi = ld2(U, i + 2);
+        if (GRAD && do_grad && (own0 || own1)) {
+            const float2 f = ld2(F, i);
+            const float2 t0 = der_x(ld2(F, i - 2 * kFs), ld2(F, i - kFs), ld2(F, i + kFs), ld2(F, i + 2 * kFs), C.sdx);
+            const float2 t1 = der_z(ld2(F, i - 2), f, ld2(F, i + 2), C.sdz);
+            const float2 t2 = der_x(um2, um1, up1, up2, C.sdx), t3 = der_z(ulo, u0, uhi, C.sdz);
+            float2 fp = make_float2(0.f, 0.f), fm = fp;
+            if (itf + 1 <= last) {
+                const float inv = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, itf + 1);
+                fp = snap_load2(Sp->snap, (long long)(itf + 1) * Sp->snap_slot + cell, prec, inv);
+            }
+            {
+                const float inv = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, itf - 1);
+                fm = snap_load2(Sp->snap, (long long)(itf - 1) * Sp->snap_slot + cell, prec, inv);
+            }
+            const float w = Sp->gwt[itf];
+            float *g = Sp->grad + cell;
+            float2 g0 = __ldcg(reinterpret_cast<const float2 *>(g)), g1 = __ldcg(reinterpret_cast<const float2 *>(g + nxz));
+            acoustic_image(g0.x, g1.x, t0.x, t1.x, t2.x, t3.x, f.x, u0.x, K.x, fp.x, fm.x, w, dtg, itf, last);
+            acoustic_image(g0.y, g1.y, t0.y, t1.y, t2.y, t3.y, f.y, u0.y, K.y, fp.y, fm.y, w, dtg, itf, last);
+            if (own0) {
+                g[0] = g0.x;
+                g[nxz] = g1.x;
+            }
+            if (own1) {
+                g[1] = g0.y;
+                g[nxz + 1] = g1.y;
+            }
+        }
+        const float2 r00 = ld2(IR, i), rlo = ld2(IR, i - 2), rhi = ld2(IR, i + 2);
+        const Brk2 bx = brackets2(ld2(IR, i - 2 * kFs), ld2(IR, i - kFs), r00, ld2(IR, i + kFs), ld2(IR, i + 2 * kFs));
+        float2 n = mul2(bc2(C.inv_d2x), sum_x(bx, um2, um1, u0, up1, up2));
+        const Brk2 bz = brackets2(rlo, zsh(rlo, r00), r00, zsh(r00, rhi), rhi);
+        n = add2(n, mul2(bc2(C.inv_d2z), sum_z(bz, ulo, u0, uhi)));
+        for (int e = e0; e < e1; e++) {
+            const InjEntry &E = Sp->inj[e];
+            if (E.gx == gx && (E.gz == gz || E.gz == gz + 1)) {
+                const float v = E.wa * srcrow[E.ia];
+                if (E.gz == gz) n.x += v;
+                else n.y += v;
+            }
+        }
+        float2 q = p;
+        if (it > 0) q = mul2(mul2(q, tzv), tzx);
+        // dt^2 n K + 2 curr - prev, tapered
+        n = dif2(fma2(bc2(2.f), u0, mul2(mul2(bc2(C.dt2), n), K)), q);
+        n = mul2(mul2(n, tzv), tzx);
+        if (own0) pn[cell] = n.x;
+        if (own1) pn[cell + 1] = n.y;
+        if (store) {
+            const float sc = prec == SNAP_FP32 ? 1.f : snap_scale(Sp->snap_amax, slot);
+            const long long o = (long long)slot * Sp->snap_slot + cell;
+            if (own0) snap_store(Sp->snap, o, prec, u0.x, sc);
+            if (own1) snap_store(Sp->snap, o + 1, prec, u0.y, sc);
+        }
+        if (own0) amax = fabsf(n.x);
+        if (own1) amax = fmaxf(amax, fabsf(n.y));
+    } else {
+#pragma unroll 1
+        for (int h = 0; h < 2; h++) {
+            const int tz = t & 31, tx = (t >> 5) + 8 * h, gx = wx0 + tx, gz = wz0 + tz;
+            if (!(gx >= tr.ox0 && gx < tr.ox1 && gz >= tr.oz0 && gz < tr.oz1)) continue;
+            const int i = (tx + 2) * kFs + 4 + tz;
+            const long long cell = (long long)gx * ldz + gz;
+            const float u0 = U[i], K = M.p0[mofs + (long long)gx * mld + gz];
+            float p = __ldcg(pn + cell);
+            if (store) {
+                const float sc = prec == SNAP_FP32 ? 1.f : snap_scale(Sp->snap_amax, slot);
+                snap_store(Sp->snap, (long long)slot * Sp->snap_slot + cell, prec, u0, sc);
+            }
+            if (GRAD && do_grad) {
+                const float t0 = d1(F + i, kFs, gx, nx, C.dx, C.sdx), t1 = d1(F + i, 1, gz, nz, C.dz, C.sdz);
+                const float t2 = d1(U + i, kFs, gx, nx, C.dx, C.sdx), t3 = d1(U + i, 1, gz, nz, C.dz, C.sdz);
+                float fp = 0.f, fm = 0.f;
+                if (itf + 1 <= last) {
+                    const float inv = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, itf + 1);
+                    fp = snap_load(Sp->snap, (long long)(itf + 1) * Sp->snap_slot + cell, prec, inv);
+                }
+                {
+                    const float inv = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, itf - 1);
+                    fm = snap_load(Sp->snap, (long long)(itf - 1) * Sp->snap_slot + cell, prec, inv);
+                }
+                float *g = Sp->grad + cell;
+                float g0 = __ldcg(g), g1 = __ldcg(g + nxz);
+                acoustic_image(g0, g1, t0, t1, t2, t3, F[i], u0, K, fp, fm, Sp->gwt[itf], dtg, itf, last);
+                g[0] = g0;
+                g[nxz] = g1;
+            }
+            float n = 0.f;
+            // second derivative along x, then z; the closures' coefficient sums come from k_closures
+#pragma unroll 1
+            for (int ax = 0; ax < 2; ax++) {
+                const int g = ax ? gz : gx, na = ax ? nz : nx, st = ax ? 1 : kFs;
+                if (g >= 6 && g < na - 6) {
+                    n = d2i(n, brackets(IR + i, st), U + i, st, ax ? C.inv_d2z : C.inv_d2x);
+                    continue;
+                }
+                const bool far = g >= 6;
+                const int r = far ? na - 1 - g : g, in = far ? -st : st;
+                const float *u = U + i + (far ? r : -r) * st;
+                const int ld = ax ? M.nx : ldz;
+                const float *cl = (ax ? M.zclos + Sp->x0 + gx : Sp->xclos + gz) + (long long)((far ? 48 : 0) + r * 8) * ld;
+                const double id2 = ax ? C.id2z64 : C.id2x64;
+                float v[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) v[j] = cl[(long long)j * ld];
+#pragma unroll
+                for (int j = 0; j < 8; j++) n += div64(v[j] * u[j * in], id2);
+            }
+            for (int e = e0; e < e1; e++) {
+                const InjEntry &E = Sp->inj[e];
+                if (E.gx == gx && E.gz == gz) n += E.wa * srcrow[E.ia];
+            }
+            const float tzv = Sp->tz[gz], txv = Sp->tx[gx];
+            if (it > 0) p = p * tzv * txv;
+            // sides in the reference's order: top, bottom, left, right (the fluid's interface, its bottom, last)
+#pragma unroll 1
+            for (int k = 0; k < 4; k++) {
+                const int side = !FLUID ? k : (k == 0 ? 0 : k == 3 ? 1 : k + 1);
+                const int bc = side == 0 ? C.bc[0] : side == 1 ? C.bc[1] : side == 2 ? C.bc[2] : C.bc[3];
+                const int dist = side == 0 ? gz : side == 1 ? nz - 1 - gz : side == 2 ? gx : nx - 1 - gx;
+                if (bc < 1 || bc > 3 || dist >= 4) continue;
+                const int st = side == 0 ? 1 : side == 1 ? -1 : side == 2 ? kFs : -kFs;
+                n = asat_cell(n, side, bc, dist, U + i, st, IR + i, st, p, K, C);
+            }
+            n = C.dt2 * n * K + 2 * u0 - p;
+            if (gz == 0 || gz == nz - 1 || gx == 0 || gx == nx - 1) {
+                const int q = gz == 0 ? gx : gz == nz - 1 ? nx + gx : gx == 0 ? 2 * nx + gz : 2 * nx + nz + gz;
+                if (n != 0.f) n = n / Sp->den[q];   // den > 0
+            }
+            if (FLUID && gz == nz - 1) Sp->halo_save[gx] = p;   // interface row: coupled and tapered there
+            else n = n * tzv * txv;
+            pn[cell] = n;
+            amax = fmaxf(amax, fabsf(n));
+        }
+    }
+    if (!GRAD && !FLUID && (flags & F_AMAX) && (it + 1) % C.sub == 0)
+        block_amax(amax, sm + L::RED, Sp->snap_amax + (it + 1) / C.sub);
+    return true;
+}
+
+struct AcousticArgs {
+    const ShotDev *shots;
+    const TileRef *tiles;
+    int ntile;
+    ModelDev M;
+    StepConst C;
+    int it0, it1, flags;
+    float dtg;
+    unsigned *count;
+    int *status;
+};
+
+// The time loop of the acoustic propagator.
+template <bool GRAD>
+__global__ void __launch_bounds__(kFt, GRAD ? 3 : 4) acoustic_steps(const __grid_constant__ AcousticArgs A)
+{
+    extern __shared__ __align__(1024) float sm[];
+    const int G = gridDim.x;
+    for (int it = A.it0; it < A.it1; it++) {
+        for (int u = blockIdx.x; u < A.ntile; u += G) {
+            const TileRef tr = A.tiles[u];
+            const bool first = u == (int)blockIdx.x, keep = (int)blockIdx.x + G >= A.ntile && it > A.it0;
+            if (!acoustic_unit<GRAD, false>(A.shots + tr.shot, A.M, A.C, tr, it, A.flags, A.dtg, keep, sm, [&]() {
+                    return !first || meet_at(A.count, A.status, A.C.spin, (unsigned)(it - A.it0), it);
+                }))
+                return;
+            __syncthreads();
+        }
+        if (threadIdx.x == 0 && it + 1 < A.it1) arrive(A.count);
+    }
+}
+
 // Table entries of the windows to come, copied ahead: the next window's shot and
 // the tile after it (whose address needs nothing that is still on its way).
 __device__ __forceinline__ void fetch16(void *dst, const void *src, int bytes, int lane0)
@@ -1307,8 +1598,14 @@ __device__ __forceinline__ void fetch16(void *dst, const void *src, int bytes, i
     if (q >= 0 && q < bytes / 16) cp16((float *)dst + 4 * q, (const float *)src + 4 * q, true);
 }
 
-template <bool VTI, bool GRAD, bool AE>
-__global__ void __launch_bounds__(kFt, VTI && GRAD ? 3 : (GRAD ? FUSED_GRAD_BLOCKS : FUSED_FWD_BLOCKS))
+// BLOCKS: resident CTAs per SM asked of the compiler.  The adjoint's shared memory
+// allows four (VTI: three).  The forward takes five (48 registers, a few spills)
+// where there are units for them, and four (64 registers) where each CTA has its
+// one unit anyway and a step lasts as long as a band unit's chain of
+// instructions: 8 shots of 801 x 401 52.1 -> 45.7 us a step with five, but one
+// 81 x 61 shot 5.9 -> 6.4 us.
+template <bool VTI, bool GRAD, bool AE, int BLOCKS>
+__global__ void __launch_bounds__(kFt, BLOCKS)
 fused_steps(const __grid_constant__ FusedArgs A)
 {
     extern __shared__ __align__(1024) float sm[];
@@ -1324,7 +1621,8 @@ fused_steps(const __grid_constant__ FusedArgs A)
         return slot >= off ? slot - off : slot - off + A.nunit;
     };
     const int n = (A.nunit - (int)blockIdx.x + G - 1) / G;   // this CTA's units
-    const bool one = n == 1;
+    // its only unit (a tile of the fluid layer would take the same shared memory)
+    const bool one = n == 1 && !(AE && G - 1 - (int)blockIdx.x < A.W.ntile);
     // its windows are the slots [w0, w0 + nw), the others are band units
     int w0 = 0, nw = 0;
     for (int m = 0; m < n; m++)
@@ -1361,6 +1659,17 @@ fused_steps(const __grid_constant__ FusedArgs A)
             first = false;
             __syncthreads();
         }
+        if (AE) {
+            // tiles of the fluid layer, from the last CTA on
+            for (int u = G - 1 - (int)blockIdx.x; u < A.W.ntile; u += G) {
+                const TileRef tr = A.W.tiles[u];
+                if (!acoustic_unit<false, true>(A.W.shots + tr.shot, A.W.M, A.W.C, tr, it, A.flags & F_EXTRACT, 1.f, false, sm,
+                                                [&]() { return !first || meet<AE>(A, it); }))
+                    return;
+                first = false;
+                __syncthreads();
+            }
+        }
         for (int k = 0; k < nw; k++, q++) {
             const ShotDev &S = S_[q & 1], &Sn = S_[(q + 1) & 1];
             const WinRef &tr = T_[q & 3], &tn = T_[(q + 1) & 3];
@@ -1376,7 +1685,7 @@ fused_steps(const __grid_constant__ FusedArgs A)
                     }
                     load_snaps16<VTI, GRAD, AE>(A, S, tr, it, sm);
                 }
-                if (first && !meet(A, it)) return;
+                if (first && !meet<AE>(A, it)) return;
                 if (active && threadIdx.x == 0) {
                     fence_async();
                     issue_lead<VTI, GRAD, AE>(A, S, tr, it, false, true, sm, lead);
@@ -1417,10 +1726,24 @@ fused_steps(const __grid_constant__ FusedArgs A)
             }
         }
         if (nw == 0) {
+            if (AE && first && !meet<AE>(A, it)) return;
             fence_async();
             __syncthreads();
         }
-        if (threadIdx.x == 0 && it + 1 < A.it1) arrive(A);
+        if (AE) {
+            // the coupling of fluid and elastic rows, column by column
+            if (threadIdx.x == 0) arrive(A.count);
+            if (!meet_at(A.count, A.status, A.C.spin, 2u * (unsigned)(it - A.it0) + 1u, it)) return;
+            const int per = (A.W.ncol + kFt - 1) / kFt;
+            for (int c = blockIdx.x; c < per * A.W.nshot; c += G) {
+                const int sh = A.W.s0 + c / per;
+                ae_couple_column(A.shots[sh], A.W.shots[sh], (c % per) * kFt + threadIdx.x, A.M, A.C, it, A.flags, A.dtg,
+                                 A.W.Kw, A.W.val0, A.W.sign);
+            }
+            fence_async();
+            __syncthreads();
+        }
+        if (threadIdx.x == 0 && it + 1 < A.it1) arrive(A.count);
     }
 }
 
@@ -1449,8 +1772,10 @@ void launch_closures(const float *f, float *out, int lines, int ld, int n, long 
     k_closures<<<dim3((ld + 127) / 128, 48, 2), 128, 0, st>>>(f, out, lines, ld, n, sl, sn);
 }
 
-void upload_fused_tables(const float *b1, const float *b2, const float *c2, const float *c1, const float *sc)
+void upload_fused_tables(const float *b1, const float *b2, const float *c2, const float *c1, const float *sc,
+                         const float *hc)
 {
+    cudaMemcpyToSymbol(kHC, hc, sizeof(float) * 4);
     cudaMemcpyToSymbol(kB1, b1, sizeof(float) * 24);
     cudaMemcpyToSymbol(kB2, b2, sizeof(float) * 384);
     cudaMemcpyToSymbol(kC2, c2, sizeof(float) * 10);
@@ -1461,21 +1786,21 @@ void upload_fused_tables(const float *b1, const float *b2, const float *c2, cons
     cudaMemcpyToSymbol(kMinus2, &minus, sizeof(minus));
 }
 
-template <bool VTI, bool GRAD, bool AE>
-static cudaError_t launch_fused_t(const FusedArgs &A, cudaStream_t st)
+// A cooperative launch of at most the resident CTAs over `units`.
+template <class Args>
+static cudaError_t launch_loop(void (*kernel)(const Args), const Args &A, int units, size_t bytes, unsigned *count,
+                               cudaStream_t st)
 {
-    constexpr size_t bytes = fused_bytes<VTI, GRAD, AE>();
-    auto kernel = fused_steps<VTI, GRAD, AE>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     int dev = 0, sms = 0, per = 0;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kFt, bytes);
-    if (e == cudaSuccess) e = cudaMemsetAsync(A.count, 0, sizeof(unsigned), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(count, 0, sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
     const long long room = (long long)sms * per;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(A.nunit < room ? A.nunit : room));
+    cfg.gridDim = dim3((unsigned)(units < room ? units : room));
     cfg.blockDim = dim3(kFt);
     cfg.dynamicSmemBytes = bytes;
     cfg.stream = st;
@@ -1485,6 +1810,22 @@ static cudaError_t launch_fused_t(const FusedArgs &A, cudaStream_t st)
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, A);
+}
+
+template <bool VTI, bool GRAD, bool AE>
+static cudaError_t launch_fused_t(const FusedArgs &A, cudaStream_t st)
+{
+    constexpr size_t bytes = fused_bytes<VTI, GRAD, AE>();
+    if constexpr (GRAD) {
+        return launch_loop(fused_steps<VTI, GRAD, AE, VTI ? 3 : 4>, A, A.nunit, bytes, A.count, st);
+    } else {
+        int dev = 0, sms = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        if (A.nunit <= 4 * sms) return launch_loop(fused_steps<VTI, GRAD, AE, 4>, A, A.nunit, bytes, A.count, st);
+        return launch_loop(fused_steps<VTI, GRAD, AE, 5>, A, A.nunit, bytes, A.count, st);
+    }
 }
 
 // ---- tensor maps ----------------------------------------------------------------
@@ -1551,7 +1892,7 @@ static cudaError_t model_maps(CUtensorMap *m, int kind, const ModelDev &M)
 
 cudaError_t launch_fused(int kind, const ShotDev *shots, const BandRef *bands, int nband, const WinRef *in, int nin,
                          const ModelDev &M, const StepConst &C, int it0, int it1, int flags, float dtg, unsigned *count,
-                         int *status, cudaStream_t st)
+                         int *status, const FluidArgs *fluid, cudaStream_t st)
 {
     if (nband + nin <= 0 || it1 <= it0) return cudaSuccess;
     FusedArgs A;
@@ -1568,12 +1909,22 @@ cudaError_t launch_fused(int kind, const ShotDev *shots, const BandRef *bands, i
     A.dtg = dtg;
     A.count = count;
     A.status = status;
+    if (fluid) A.W = *fluid;
     const cudaError_t e = model_maps(A.mm, kind, M);
     if (e != cudaSuccess) return e;
     const bool g = (flags & F_GRAD) != 0;
     if (kind == KIND_VTI) return g ? launch_fused_t<true, true, false>(A, st) : launch_fused_t<true, false, false>(A, st);
     if (kind == KIND_AE) return g ? launch_fused_t<false, true, true>(A, st) : launch_fused_t<false, false, true>(A, st);
     return g ? launch_fused_t<false, true, false>(A, st) : launch_fused_t<false, false, false>(A, st);
+}
+
+cudaError_t launch_acoustic_loop(const ShotDev *shots, const TileRef *tiles, int ntile, const ModelDev &M, const StepConst &C,
+                                 int it0, int it1, int flags, float dtg, unsigned *count, int *status, cudaStream_t st)
+{
+    if (ntile <= 0 || it1 <= it0) return cudaSuccess;
+    const AcousticArgs A = {shots, tiles, ntile, M, C, it0, it1, flags, dtg, count, status};
+    if (flags & F_GRAD) return launch_loop(acoustic_steps<true>, A, ntile, sizeof(float) * AcLayout<true>::FLOATS, count, st);
+    return launch_loop(acoustic_steps<false>, A, ntile, sizeof(float) * AcLayout<false>::FLOATS, count, st);
 }
 
 }  // namespace fwi2d

@@ -32,10 +32,24 @@ void launch_elastic_march(bool vti, const ShotDev *shots, const MarchRef *units,
 // device memory of the plan's own; status: receives step + 1 of a wait that
 // gave up.
 constexpr int kFusedZ = 32, kFusedX = 16, kFusedBand = 28;
-void upload_fused_tables(const float *b1, const float *b2, const float *c2, const float *c1, const float *sc);
+void upload_fused_tables(const float *b1, const float *b2, const float *c2, const float *c1, const float *sc,
+                         const float *hc);
+// the fluid layer of acoustic-elastic shots: its tables, tiles and constants, and
+// the interface (ncol: columns of the widest shot, nshot shots from s0)
+struct FluidArgs {
+    const ShotDev *shots;
+    const TileRef *tiles;
+    int ntile, ncol, s0, nshot, sign;
+    ModelDev M;
+    StepConst C;
+    float Kw, val0;
+};
 cudaError_t launch_fused(int kind, const ShotDev *shots, const BandRef *bands, int nband, const WinRef *in, int nin,
                          const ModelDev &M, const StepConst &C, int it0, int it1, int flags, float dtg, unsigned *count,
-                         int *status, cudaStream_t st);
+                         int *status, const FluidArgs *fluid, cudaStream_t st);
+// the same for the acoustic propagator, over 32 x 16 tiles of the whole grid
+cudaError_t launch_acoustic_loop(const ShotDev *shots, const TileRef *tiles, int ntile, const ModelDev &M, const StepConst &C,
+                                 int it0, int it1, int flags, float dtg, unsigned *count, int *status, cudaStream_t st);
 // tensor maps of a shot (ShotMap, host memory of fused_maps_bytes()); grad / snap may be null
 size_t fused_maps_bytes();
 cudaError_t fused_shot_maps(void *out, int nx, int ldz, const float *u0, const float *u1, const float *grad,

@@ -79,9 +79,10 @@ def _gradient(kind, shape, prec, every, compensated, nx=150, nz=75, nt=97):
         if kind == O.KIND_AE:
             kw = dict(water_src_x=sx, water_src_z=[0.05], water_rcv_x=rx, water_rcv_z=np.full(11, 0.03, np.float32))
         shots.append(F.ShotSpec(x0, w, n, sx, [sz[0] + oz], rx, rz + np.float32(oz), **kw))
-        ns = 1 if kind == O.KIND_AE else 2
-        src.append(K.sources(ns, n, 1e-3, f0=25.0, t0=0.03))
-        obs.append(rng.normal(size=(3 if kind == O.KIND_AE else 2, 11, n)).astype(np.float32))
+        ns = 1 if kind in (O.KIND_AE, O.KIND_ACOUSTIC) else 2
+        nc = {O.KIND_AE: 3, O.KIND_ACOUSTIC: 1}.get(kind, 2)
+        src.append(K.sources(ns, n, 1e-3, f0=25.0, t0=0.03).reshape(ns, 1, n))
+        obs.append(rng.normal(size=(nc, 11, n)).astype(np.float32))
     P = F.Propagator(0)
     P.set_model(kind, mc, d, d, 0.0, oz)
     P.set_shots(F.make_params(**pd, tile_shape=shape, snapshot_precision=prec, checkpoint_every=every,
@@ -92,7 +93,7 @@ def _gradient(kind, shape, prec, every, compensated, nx=150, nz=75, nt=97):
     return out, rcv
 
 
-@pytest.mark.parametrize("kind", [O.KIND_ELASTIC, O.KIND_VTI, O.KIND_AE])
+@pytest.mark.parametrize("kind", [O.KIND_ELASTIC, O.KIND_VTI, O.KIND_AE, O.KIND_ACOUSTIC])
 @pytest.mark.parametrize("prec,every,compensated", [(0, 0, 0), (2, 0, 1), (1, 20, 0), (0, 7, 1)])
 def test_fused_plan_equals_tile_plan(kind, prec, every, compensated):
     """Uneven windows and records, 16-bit snapshots, replayed segments and
@@ -106,6 +107,27 @@ def test_fused_plan_equals_tile_plan(kind, prec, every, compensated):
         assert fa == fb and np.array_equal(ga, gb)
     for x, y in zip(ra, rb):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("bc", [(1, 2, 2, 2), (3, 1, 2, 3)])
+@pytest.mark.parametrize("grid", [(24, 40), (40, 47), (61, 107), (150, 210)])
+def test_acoustic_loop_vs_oracle(bc, grid):
+    """The acoustic time loop: tiles of the closures only, and z-pair windows."""
+    nx, nz = grid
+    kind, d, nt = O.KIND_ACOUSTIC, 0.01, 150
+    mc = K.converted(kind, K.model_case(kind, nx, nz, d, seed=3))
+    sl, rl = K.geometry(nx, nz, d, nr=14, sz=0.2)
+    pd = K.par_dict(nt=nt, dt=1e-3, bc=bc, taper=(0, 6, 5, 6))
+    src = K.sources(1, nt, 1e-3, f0=25.0, t0=0.03)
+    port = O.Port(32)
+    par = O.make_par(**pd, ns=1, nr=14)
+    rcv_o, full_o = K.oracle_forward(port, kind, mc, src, par, nx, nz, d, sl, rl)
+    adj = np.ascontiguousarray(rcv_o[:, :, ::-1])
+    g_o = K.oracle_adjoint(port, kind, mc, adj, par, nx, nz, d, sl, rl, full_o)
+    rcv_g, g_g, _ = run_gpu(kind, mc, src, pd, nx, nz, d, sl, rl, adj_src=adj, shape=fused_shape())
+    assert np.abs(g_o).max() > 0
+    assert np.array_equal(rcv_g, rcv_o)
+    assert np.array_equal(g_g, g_o)
 
 
 def test_fused_wait_limit_returns_timeout(monkeypatch):

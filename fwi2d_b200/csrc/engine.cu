@@ -568,6 +568,7 @@ struct ShotUnits {
     bool march = false;            // marching plan: x-band tiles, bands, marching units
     bool framed = false;           // framed tile plan: x-band tiles, bands, interior tiles
     bool fused = false;            // fused plan: band units (nxband x bands first) and interior windows
+    bool sort_all = false;         // every unit's entries sorted by cell (acoustic time loop)
     int nxband = 0;
     std::vector<int> xzo;          // fused: z starts of the x-band units, plus nz
     int nx = 0, nz = 0;
@@ -608,7 +609,7 @@ struct ShotUnits {
     // (band and marching units)
     bool row_sorted(int u) const
     {
-        return u >= (int)tiles.size() && u < (int)(tiles.size() + bands.size() + marches.size());
+        return sort_all || (u >= (int)tiles.size() && u < (int)(tiles.size() + bands.size() + marches.size()));
     }
     struct RowUnit {
         int unit, xb, xe, roff;
@@ -804,6 +805,27 @@ static ShotUnits make_units(int shape, int shot, int nx, int nz, bool band_split
             U.marches.push_back(m);
         }
     return U;
+}
+
+// Tiles of the acoustic time loop: those that touch a closure (fused.cu
+// acoustic_unit) are cut into units of 8 columns, and come first.
+static std::vector<TileRef> acoustic_units(const std::vector<TileRef> &tiles, int nx, int nz)
+{
+    std::vector<TileRef> edge, inner;
+    for (const TileRef &r : tiles) {
+        if (r.wx0 >= 6 && r.wx0 + kFusedX + 6 <= nx && r.wz0 >= 6 && r.wz0 + kFusedZ + 6 <= nz && (r.wz0 & 3) == 0) {
+            inner.push_back(r);
+            continue;
+        }
+        for (int h = 0; h < 2; h++) {
+            TileRef q = r;
+            q.ox0 = std::max(r.ox0, r.wx0 + 8 * h);
+            q.ox1 = std::min(r.ox1, r.wx0 + 8 * h + 8);
+            if (q.ox0 < q.ox1) edge.push_back(q);
+        }
+    }
+    edge.insert(edge.end(), inner.begin(), inner.end());
+    return edge;
 }
 
 // Group entries by unit (stable: the reference's order survives within a
@@ -1417,7 +1439,8 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
         S->nt = sh.nt;
         S->ncomp = acoustic ? 1 : 2;
         const bool loop = P->fused && !acoustic;   // band units and windows
-        const ShotUnits U = make_units(P->fused && acoustic ? kAcousticTile : shape, s, sh.nx, M.nz, P->band_split);
+        ShotUnits U = make_units(P->fused && acoustic ? kAcousticTile : shape, s, sh.nx, M.nz, P->band_split);
+        U.sort_all = P->fused;
         const int nunits = U.nunits();
         S->ntr_src = src_fluid ? sh.src_water.ntr : sh.src.ntr;
         S->ncomp_src = acoustic || src_fluid ? 1 : (p.mt ? 3 : 2);
@@ -1467,7 +1490,8 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
             W->nt = sh.nt;
             W->ncomp = 1;
             W->nr = sh.rcv_water.ntr;
-            const ShotUnits UW = make_units(P->tshape, s, sh.nx, p.nza, P->band_split);
+            ShotUnits UW = make_units(P->tshape, s, sh.nx, p.nza, P->band_split);
+            UW.sort_all = P->fused;
             int wa[2] = {0, 0}, wb[2] = {0, 0};
             build_inj(src_fluid ? sh.src_water : none, 1, wa, wb, UW, W->inj_f, W->inj_f_off, W->inj_f_roff);
             build_inj(sh.rcv_water, 1, wa, wb, UW, W->inj_a, W->inj_a_off, W->inj_a_roff);
@@ -1494,7 +1518,8 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
             W->tz.upload(wtz, ctx->st);
             W->tx.upload(wtx, ctx->st);
             S->u_w0 = (int)P->wtiles.size();
-            P->wtiles.insert(P->wtiles.end(), UW.tiles.begin(), UW.tiles.end());
+            const std::vector<TileRef> wt = P->fused ? acoustic_units(UW.tiles, sh.nx, p.nza) : UW.tiles;
+            P->wtiles.insert(P->wtiles.end(), wt.begin(), wt.end());
             S->halo.alloc((size_t)sh.nx * sizeof(float));
             S->fluid = std::move(W);
             P->nx_max = std::max(P->nx_max, sh.nx);
@@ -1564,7 +1589,8 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
         S->u_m0 = (int)P->marches.size();
         S->u_b0 = (int)P->bands.size();
         S->u_i0 = (int)P->itiles.size();
-        P->tiles.insert(P->tiles.end(), U.tiles.begin(), U.tiles.end());
+        const std::vector<TileRef> units = P->fused && acoustic ? acoustic_units(U.tiles, sh.nx, M.nz) : U.tiles;
+        P->tiles.insert(P->tiles.end(), units.begin(), units.end());
         P->marches.insert(P->marches.end(), U.marches.begin(), U.marches.end());
         P->bands.insert(P->bands.end(), U.bands.begin(), U.bands.end());
         P->itiles.insert(P->itiles.end(), U.itiles.begin(), U.itiles.end());

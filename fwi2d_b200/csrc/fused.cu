@@ -1305,12 +1305,14 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
 // Acoustic unit: a window of 32 (z) x 16 (x) cells of a shot's pressure (or of
 // the fluid layer's potential, FLUID), the tile kernel's windows and arithmetic
 // (acoustic.cuh, src/cpp/we_op.cpp:1937-2134).  Windows clear of the closures
-// take the z-pair form of the elastic windows; the others update two cells per
-// thread through the general forms.
+// take the z-pair form of the elastic windows; the others are cut into units of
+// 8 columns (their owned cells), one cell per thread through the general forms:
+// such a unit's time is one thread's chain, which sets the step on small plans.
 // ---------------------------------------------------------------------------
 template <bool GRAD>
 struct AcLayout {
-    static constexpr int U = 0, IR = kFu, F = IR + kFw, RED = F + (GRAD ? kFw : 0), FLOATS = RED + 8;
+    static constexpr int U = 0, IR = kFu, F = IR + kFw, VAL = F + (GRAD ? kFw : 0), KEY = VAL + kVal;
+    static constexpr int RED = KEY + kVal, FLOATS = RED + 8;
 };
 
 // imaging condition of one cell at the start of a step (nl_we_op_a::compute_gradients, we_op.cpp:1883-1935)
@@ -1361,6 +1363,55 @@ __device__ __forceinline__ bool acoustic_unit(const ShotDev *__restrict__ Sp, co
                 sm[L::F + i] = in ? snap_load(Sp->snap, (long long)itf * Sp->snap_slot + (long long)x * ldz + z, prec, finv) : 0.f;
         }
     }
+    // this step's injected values and their cells (sorted by cell, the reference's order within one)
+    const int inj0 = Sp->inj_off[tr.unit], ninj = Sp->inj_off[tr.unit + 1] - inj0;
+    const float *srcrow = Sp->src + (long long)it * Sp->nsrc;
+    if (it < nt - 1 && ninj <= kVal)
+        for (int e = t; e < ninj; e += kFt) {
+            const InjEntry &E = Sp->inj[inj0 + e];
+            sm[L::VAL + e] = E.wa * srcrow[E.ia];
+            sm[L::KEY + e] = __int_as_float((E.gx - wx0) * kFz + E.gz - wz0);
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(srcrow + Sp->nsrc + E.ia));
+        }
+    auto value = [&](int e) {
+        if (ninj <= kVal) return sm[L::VAL + e];
+        const InjEntry &E = Sp->inj[inj0 + e];
+        return E.wa * srcrow[E.ia];
+    };
+    auto key = [&](int e) {
+        if (ninj <= kVal) return __float_as_int(sm[L::KEY + e]);
+        const InjEntry &E = Sp->inj[inj0 + e];
+        return (E.gx - wx0) * kFz + E.gz - wz0;
+    };
+    auto first_entry = [&](int k) {   // of the cells from k on
+        int lo = 0, hi = ninj;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (key(mid) < k) lo = mid + 1;
+            else hi = mid;
+        }
+        return lo;
+    };
+    // general form: this thread's cell and what it needs of the model
+    const int half = (tr.ox0 - wx0) >> 3, ctz = t & 31, ctx = (t >> 5) + 8 * half, cgx = wx0 + ctx, cgz = wz0 + ctz;
+    const bool cown = !inner && cgx >= tr.ox0 && cgx < tr.ox1 && cgz >= tr.oz0 && cgz < tr.oz1;
+    // closure coefficients of the axis (0 x, 1 z) at this cell
+    auto closure = [&](int ax, float (&v)[8]) {
+        const int g = ax ? cgz : cgx, na = ax ? nz : nx, ld = ax ? M.nx : ldz;
+        const bool far = g >= 6;
+        const float *cl = (ax ? M.zclos + Sp->x0 + cgx : Sp->xclos + cgz) +
+                          (long long)((far ? 48 : 0) + (far ? na - 1 - g : g) * 8) * ld;
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = cl[(long long)j * ld];
+    };
+    const bool cx = cown && (cgx < 6 || cgx >= nx - 6), cz = cown && (cgz < 6 || cgz >= nz - 6);
+    float K = 0.f, tzv = 0.f, txv = 0.f, v[8];
+    if (cown) {
+        K = M.p0[mofs + (long long)cgx * mld + cgz];
+        tzv = Sp->tz[cgz];
+        txv = Sp->tx[cgx];
+        if (cx || cz) closure(cx ? 0 : 1, v);
+    }
     const float *curr = Sp->u[(it + 1) & 1];
     float *pn = Sp->u[it & 1];
     if (!meet_first()) {
@@ -1376,15 +1427,15 @@ __device__ __forceinline__ bool acoustic_unit(const ShotDev *__restrict__ Sp, co
             cp16(sm + L::U + xr * kFs + xq, curr + (long long)(wx0 - 4 + xr) * ldz + wz0 - 4 + xq, true);
         cp_wait();
     } else {
-        float v[4];
+        float w[4];
 #pragma unroll
         for (int h = 0; h < 4; h++) {
             const int i = t + h * kFt, r = i / kFs, q = i - r * kFs, x = wx0 - 4 + r, z = wz0 - 4 + q;
-            v[h] = i < kFu && x >= 0 && x < nx && z >= 0 && z < nz ? __ldcg(curr + (long long)x * ldz + z) : 0.f;
+            w[h] = i < kFu && x >= 0 && x < nx && z >= 0 && z < nz ? __ldcg(curr + (long long)x * ldz + z) : 0.f;
         }
 #pragma unroll
         for (int h = 0; h < 4; h++)
-            if (t + h * kFt < kFu) sm[L::U + t + h * kFt] = v[h];
+            if (t + h * kFt < kFu) sm[L::U + t + h * kFt] = w[h];
     }
     __syncthreads();
 
@@ -1402,8 +1453,6 @@ __device__ __forceinline__ bool acoustic_unit(const ShotDev *__restrict__ Sp, co
             Sp->rcv[(long long)it * Sp->nrcv + E.row] = o;
         }
     }
-    const int e0 = Sp->inj_off[tr.unit], e1 = Sp->inj_off[tr.unit + 1];
-    const float *srcrow = Sp->src + (long long)it * Sp->nsrc;
     const int slot = by(it, C.sub);
     const bool store = !GRAD && (flags & F_STORE) && slot * C.sub == it;
     float amax = 0.f;
@@ -1414,8 +1463,8 @@ __device__ __forceinline__ bool acoustic_unit(const ShotDev *__restrict__ Sp, co
         const bool own0 = ownx && gz >= tr.oz0 && gz < tr.oz1, own1 = ownx && gz + 1 >= tr.oz0 && gz + 1 < tr.oz1;
         const long long cell = (long long)gx * ldz + gz;
         const float2 p = __ldcg(reinterpret_cast<const float2 *>(pn + cell));
-        const float2 K = *reinterpret_cast<const float2 *>(M.p0 + mofs + (long long)gx * mld + gz);
-        const float2 tzv = *reinterpret_cast<const float2 *>(Sp->tz + gz), tzx = bc2(Sp->tx[gx]);
+        const float2 K2 = *reinterpret_cast<const float2 *>(M.p0 + mofs + (long long)gx * mld + gz);
+        const float2 tz2 = *reinterpret_cast<const float2 *>(Sp->tz + gz), tzx = bc2(Sp->tx[gx]);
         const float2 um2 = ld2(U, i - 2 * kFs), um1 = ld2(U, i - kFs), u0 = ld2(U, i), up1 = ld2(U, i + kFs),
                      up2 = ld2(U, i + 2 * kFs), ulo = ld2(U, i - 2), uhi = ld2(U, i + 2);
         if (GRAD && do_grad && (own0 || own1)) {
@@ -1435,8 +1484,8 @@ __device__ __forceinline__ bool acoustic_unit(const ShotDev *__restrict__ Sp, co
             const float w = Sp->gwt[itf];
             float *g = Sp->grad + cell;
             float2 g0 = __ldcg(reinterpret_cast<const float2 *>(g)), g1 = __ldcg(reinterpret_cast<const float2 *>(g + nxz));
-            acoustic_image(g0.x, g1.x, t0.x, t1.x, t2.x, t3.x, f.x, u0.x, K.x, fp.x, fm.x, w, dtg, itf, last);
-            acoustic_image(g0.y, g1.y, t0.y, t1.y, t2.y, t3.y, f.y, u0.y, K.y, fp.y, fm.y, w, dtg, itf, last);
+            acoustic_image(g0.x, g1.x, t0.x, t1.x, t2.x, t3.x, f.x, u0.x, K2.x, fp.x, fm.x, w, dtg, itf, last);
+            acoustic_image(g0.y, g1.y, t0.y, t1.y, t2.y, t3.y, f.y, u0.y, K2.y, fp.y, fm.y, w, dtg, itf, last);
             if (own0) {
                 g[0] = g0.x;
                 g[nxz] = g1.x;
@@ -1451,19 +1500,18 @@ __device__ __forceinline__ bool acoustic_unit(const ShotDev *__restrict__ Sp, co
         float2 n = mul2(bc2(C.inv_d2x), sum_x(bx, um2, um1, u0, up1, up2));
         const Brk2 bz = brackets2(rlo, zsh(rlo, r00), r00, zsh(r00, rhi), rhi);
         n = add2(n, mul2(bc2(C.inv_d2z), sum_z(bz, ulo, u0, uhi)));
-        for (int e = e0; e < e1; e++) {
-            const InjEntry &E = Sp->inj[e];
-            if (E.gx == gx && (E.gz == gz || E.gz == gz + 1)) {
-                const float v = E.wa * srcrow[E.ia];
-                if (E.gz == gz) n.x += v;
-                else n.y += v;
+        if (ninj > 0) {
+            const int k = tx * kFz + pz;
+            for (int e = first_entry(k); e < ninj && key(e) <= k + 1; e++) {
+                if (key(e) == k) n.x += value(e);
+                else n.y += value(e);
             }
         }
         float2 q = p;
-        if (it > 0) q = mul2(mul2(q, tzv), tzx);
+        if (it > 0) q = mul2(mul2(q, tz2), tzx);
         // dt^2 n K + 2 curr - prev, tapered
-        n = dif2(fma2(bc2(2.f), u0, mul2(mul2(bc2(C.dt2), n), K)), q);
-        n = mul2(mul2(n, tzv), tzx);
+        n = dif2(fma2(bc2(2.f), u0, mul2(mul2(bc2(C.dt2), n), K2)), q);
+        n = mul2(mul2(n, tz2), tzx);
         if (own0) pn[cell] = n.x;
         if (own1) pn[cell + 1] = n.y;
         if (store) {
@@ -1474,14 +1522,11 @@ __device__ __forceinline__ bool acoustic_unit(const ShotDev *__restrict__ Sp, co
         }
         if (own0) amax = fabsf(n.x);
         if (own1) amax = fmaxf(amax, fabsf(n.y));
-    } else {
-#pragma unroll 1
-        for (int h = 0; h < 2; h++) {
-            const int tz = t & 31, tx = (t >> 5) + 8 * h, gx = wx0 + tx, gz = wz0 + tz;
-            if (!(gx >= tr.ox0 && gx < tr.ox1 && gz >= tr.oz0 && gz < tr.oz1)) continue;
-            const int i = (tx + 2) * kFs + 4 + tz;
+    } else if (cown) {
+        {
+            const int gx = cgx, gz = cgz, i = (ctx + 2) * kFs + 4 + ctz;
             const long long cell = (long long)gx * ldz + gz;
-            const float u0 = U[i], K = M.p0[mofs + (long long)gx * mld + gz];
+            const float u0 = U[i];
             float p = __ldcg(pn + cell);
             if (store) {
                 const float sc = prec == SNAP_FP32 ? 1.f : snap_scale(Sp->snap_amax, slot);
@@ -1506,31 +1551,25 @@ __device__ __forceinline__ bool acoustic_unit(const ShotDev *__restrict__ Sp, co
                 g[nxz] = g1;
             }
             float n = 0.f;
-            // second derivative along x, then z; the closures' coefficient sums come from k_closures
-#pragma unroll 1
+            // second derivative along x, then z
+#pragma unroll
             for (int ax = 0; ax < 2; ax++) {
                 const int g = ax ? gz : gx, na = ax ? nz : nx, st = ax ? 1 : kFs;
-                if (g >= 6 && g < na - 6) {
+                if (!(ax ? cz : cx)) {
                     n = d2i(n, brackets(IR + i, st), U + i, st, ax ? C.inv_d2z : C.inv_d2x);
                     continue;
                 }
+                if (ax && cx) closure(1, v);   // a corner cell
                 const bool far = g >= 6;
-                const int r = far ? na - 1 - g : g, in = far ? -st : st;
-                const float *u = U + i + (far ? r : -r) * st;
-                const int ld = ax ? M.nx : ldz;
-                const float *cl = (ax ? M.zclos + Sp->x0 + gx : Sp->xclos + gz) + (long long)((far ? 48 : 0) + r * 8) * ld;
-                const double id2 = ax ? C.id2z64 : C.id2x64;
-                float v[8];
+                const int in = far ? -st : st;
+                const float *u = U + i + (far ? na - 1 - g : -g) * st;
 #pragma unroll
-                for (int j = 0; j < 8; j++) v[j] = cl[(long long)j * ld];
-#pragma unroll
-                for (int j = 0; j < 8; j++) n += div64(v[j] * u[j * in], id2);
+                for (int j = 0; j < 8; j++) n += div64(v[j] * u[j * in], ax ? C.id2z64 : C.id2x64);
             }
-            for (int e = e0; e < e1; e++) {
-                const InjEntry &E = Sp->inj[e];
-                if (E.gx == gx && E.gz == gz) n += E.wa * srcrow[E.ia];
+            if (ninj > 0) {
+                const int k = ctx * kFz + ctz;
+                for (int e = first_entry(k); e < ninj && key(e) == k; e++) n += value(e);
             }
-            const float tzv = Sp->tz[gz], txv = Sp->tx[gx];
             if (it > 0) p = p * tzv * txv;
             // sides in the reference's order: top, bottom, left, right (the fluid's interface, its bottom, last)
 #pragma unroll 1

@@ -1630,16 +1630,15 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
     const size_t mb = fused_maps_bytes();
     std::vector<unsigned char> maps;
     if (P->fused && !acoustic) {
-        const bool replay = p.checkpoint_every > 0, f32 = p.snapshot_precision == FWI2D_SNAP_FP32;
+        const bool replay = p.checkpoint_every > 0, half = p.snapshot_precision != FWI2D_SNAP_FP32;
         maps.resize((replay ? 2 : 1) * nshots * mb);
         for (int s = 0; s < nshots; s++) {
             const ShotPlan &S = *P->shots[s];
-            const float *snap = f32 ? (const float *)S.snap_base : nullptr;
-            CK(fused_shot_maps(&maps[s * mb], S.nx, M.ldz, S.u0.as<float>(), S.u1.as<float>(), S.grad.as<float>(), snap,
-                               S.nbuf));
+            CK(fused_shot_maps(&maps[s * mb], S.nx, M.ldz, S.u0.as<float>(), S.u1.as<float>(), S.grad.as<float>(),
+                               S.snap_base, S.nbuf, half));
             if (replay && S.r0.p)
                 CK(fused_shot_maps(&maps[(nshots + s) * mb], S.nx, M.ldz, S.r0.as<float>(), S.r1.as<float>(), nullptr,
-                                   nullptr, 0));
+                                   nullptr, 0, false));
         }
         P->d_maps.upload(maps, ctx->st);
         for (int s = 0; s < nshots; s++) sf[s].maps = sa[s].maps = P->d_maps.as<char>() + s * mb;

@@ -81,7 +81,7 @@ struct alignas(16) ShotDev {
 };
 
 // Tensor maps of a shot (fused.cu): field buffers 0 and 1 with the windows'
-// 4-cell halo and their own cells only, the gradient, FP32 snapshots likewise.
+// 4-cell halo and their own cells only, the gradient, the snapshots likewise.
 enum ShotMap { SM_LEAD = 0, SM_OWN = 2, SM_GRAD = 4, SM_SNAP_LEAD, SM_SNAP_OWN, SM_COUNT = 8 };
 
 // Model on the full grid; shots index it at column x0 + ix.

@@ -227,15 +227,21 @@ struct BandLayout {
     static constexpr int A = kFb * kFs, CL = 6 * 8 * kFusedBand;
     static constexpr int UN = 0, UT = A, MU = 2 * A, Q = 3 * A, D = 4 * A, DS = 5 * A, DT = 6 * A;
     static constexpr int D1 = 7 * A, LB = D1 + (VTI || AE ? A : 0), LC = LB + (VTI ? A : 0), LA = LC + (VTI ? A : 0);
-    static constexpr int F0 = LA + (VTI ? A : 0), F1 = F0 + (GRAD ? A : 0), C0 = F1 + (GRAD ? A : 0);
+    static constexpr int F = LA + (VTI ? A : 0);           // snapshots [index & 3][2 components]
+    static constexpr int C0 = F + (GRAD ? 8 * A : 0);
     static constexpr int C1 = C0 + CL;                     // VTI x bands: closure of (1+2eps)2mu
     static constexpr int ZC = C1 + (VTI ? CL : 0);
     // per thread, set once per unit: doubles 1/rho and 1/den (two components), then the floats of Slot
     static constexpr int SD = ZC + 2 * 6 * 8 * 6;
     static constexpr int SF = SD + 3 * 2 * kFt;
     static constexpr int SAT = SF + 7 * kFt;               // [own side, corner][along, across, normal][32]
-    static constexpr int VAL = SAT + 6 * 32;               // this step's injected values, one per entry of the unit
-    static constexpr int RED = VAL + kVal;
+    // injection entries of the unit: up to NVAL of them cached (weights and rows; the forward's moment
+    // tensors have two) with this step's values
+    static constexpr int NVAL = GRAD ? 512 : 256;
+    static constexpr int VAL = SAT + 6 * 32, WA = VAL + NVAL, IA = WA + NVAL, WB = IA + NVAL;
+    static constexpr int IB = WB + (GRAD ? 0 : NVAL), VEND = IB + (GRAD ? 0 : NVAL);
+    static __device__ __forceinline__ int snap(int k, int c) { return F + ((k & 3) * 2 + c) * A; }
+    static constexpr int RED = VEND;
     static constexpr int FLOATS = RED + 8;
     static_assert(SD % 2 == 0, "doubles");
 };
@@ -415,11 +421,12 @@ __device__ __forceinline__ void issue_own_static(const FusedArgs &A, const ShotD
     const CUtensorMap *sp = (const CUtensorMap *)S.maps;
     const int z = tr.wz0, x = tr.wx0, xm = S.x0 + x;
     const Imaging g = imaging<GRAD, AE>(S, A.C, it);
-    const bool f32 = GRAD && g.on && A.C.snap_prec == SNAP_FP32;
+    const bool snaps = GRAD && g.on, f32 = A.C.snap_prec == SNAP_FP32;
     unsigned bytes = 4u * kFo * (2 + (model ? 2 : 0));
     if (GRAD && g.on) bytes += 4u * kFo * 3;
     if (VTI && GRAD && model) bytes += 4u * kFo * 3;
-    if (f32) bytes += 4u * (2 * kFw + kFo * ((g.itf + 1 <= g.last ? 2 : 0) + (g.itf > 0 ? 2 : 0)));
+    const int near = (g.itf + 1 <= g.last ? 2 : 0) + (g.itf > 0 ? 2 : 0);
+    if (snaps) bytes += f32 ? 4u * (2 * kFw + kFo * near) : 2u * (2 * kFw + kFx * kFs * near);
     bar_expect(bar, bytes);
     if (model) {
         tma2(sm + L::RHO, &A.mm[MM_RHO], z, xm, bar);
@@ -430,14 +437,14 @@ __device__ __forceinline__ void issue_own_static(const FusedArgs &A, const ShotD
             tma2(sm + L::E + 2 * kFo, &A.mm[MM_V3], z, xm, bar);
         }
     }
-    if (f32) {
-        const int k = g.itf - S.snap_first;
+    if (snaps) {
+        const int k = g.itf - S.snap_first, zo = f32 ? z : z - 4;
         tma4(sm + L::F0, sp + SM_SNAP_LEAD, z - 4, x - 2, 0, k, bar);
-        if (g.itf + 1 <= g.last) tma4(sm + L::FP0, sp + SM_SNAP_OWN, z, x, 0, k + 1, bar);
-        if (g.itf > 0) tma4(sm + L::FM0, sp + SM_SNAP_OWN, z, x, 0, k - 1, bar);
+        if (g.itf + 1 <= g.last) tma4(sm + L::FP0, sp + SM_SNAP_OWN, zo, x, 0, k + 1, bar);
+        if (g.itf > 0) tma4(sm + L::FM0, sp + SM_SNAP_OWN, zo, x, 0, k - 1, bar);
         // the next imaging step's new snapshot, from HBM to L2
         if (k >= 2)
-            asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global [%0, {%1, %2, %3, %4}];" ::"l"(sp + SM_SNAP_OWN), "r"(z),
+            asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global [%0, {%1, %2, %3, %4}];" ::"l"(sp + SM_SNAP_OWN), "r"(zo),
                          "r"(x), "r"(0), "r"(k - 2)
                          : "memory");
     }
@@ -452,41 +459,29 @@ __device__ __forceinline__ void issue_own_fields(const FusedArgs &A, const ShotD
     if (GRAD && imaging<GRAD, AE>(S, A.C, it).on) tma3(sm + L::G0, sp + SM_GRAD, tr.wz0, tr.wx0, 0, bar);
 }
 
-// 16-bit snapshots of a window: converted on the way to shared memory by all threads
-template <bool VTI, bool GRAD, bool AE>
-__device__ __forceinline__ void load_snaps16(const FusedArgs &A, const ShotDev &S, const WinRef &tr, int it, float *sm)
+// 16-bit snapshots of a window lie raw in the F, FP and FM arrays (the own cells' ones in rows
+// of kFs, whose first sample keeps the copies' 16-byte alignment); their factors are set by three threads.
+__device__ __forceinline__ void set_factors(const ShotDev &S, const Imaging &g, float *inv)
 {
-    using L = InLayout<VTI, GRAD, AE>;
-    const int prec = A.C.snap_prec;
-    if (!GRAD || prec == SNAP_FP32) return;
-    const Imaging g = imaging<GRAD, AE>(S, A.C, it);
-    if (!g.on) return;
-    const int t = threadIdx.x, h = t >> 7, row = (t >> 3) & 15, q = 4 * (t & 7);
-    const int gx = tr.wx0 + row, gz = tr.wz0 + q;
-    const long long nxz = (long long)S.nx * S.ldz;
-    const int s = h * kFo + row * kFz + q;
-    const float inv = 1.f / snap_scale(S.snap_amax, g.itf);
-    if (gx < S.nx && gz < S.ldz) {
-        const long long c = (long long)g.itf * S.snap_slot + h * nxz + (long long)gx * S.ldz + gz;
-        if (g.itf + 1 <= g.last)
-            *reinterpret_cast<float4 *>(sm + L::FP0 + s) =
-                snap_load4(S.snap, c + S.snap_slot, prec, 1.f / snap_scale(S.snap_amax, g.itf + 1));
-        if (g.itf > 0)
-            *reinterpret_cast<float4 *>(sm + L::FM0 + s) =
-                snap_load4(S.snap, c - S.snap_slot, prec, 1.f / snap_scale(S.snap_amax, g.itf - 1));
-    }
-    const int xr = t / 10, xq = 4 * (t - 10 * xr), x = tr.wx0 - 2 + xr, z = tr.wz0 - 4 + xq;
-    if (t < (kFx + 4) * 10 && x < S.nx && z < S.ldz) {
-        const long long o = (long long)g.itf * S.snap_slot + (long long)x * S.ldz + z;
-        *reinterpret_cast<float4 *>(sm + L::F0 + xr * kFs + xq) = snap_load4(S.snap, o, prec, inv);
-        *reinterpret_cast<float4 *>(sm + L::F1 + xr * kFs + xq) = snap_load4(S.snap, o + nxz, prec, inv);
-    }
+    const int d = (int)threadIdx.x - 224;
+    if (!g.on || d < 0 || d > 2) return;
+    const int k = g.itf - 1 + d;
+    if (k >= 0 && k <= g.last) inv[d] = 1.f / snap_scale(S.snap_amax, k);
+}
+// a pair of raw 16-bit samples at an even index
+__device__ __forceinline__ float2 raw2(const float *base, int i, int prec, float inv)
+{
+    const unsigned w = reinterpret_cast<const unsigned *>(base)[i >> 1];
+    float2 v;
+    if (prec == SNAP_BF16) v = make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+    else v = __half22float2(*reinterpret_cast<const __half2 *>(&w));
+    return make_float2(v.x * inv, v.y * inv);
 }
 
 // The window's step: wait_lead() before it reads the Lead group, mid() between its halves.
-template <bool VTI, bool GRAD, bool AE, class Lead, class Mid>
+template <bool VTI, bool GRAD, bool AE, bool S16, class Lead, class Mid>
 __device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S, const WinRef &tr, const int it, float *sm,
-                                            Lead wait_lead, Mid mid)
+                                            const float *inv, Lead wait_lead, Mid mid)
 {
     using L = InLayout<VTI, GRAD, AE>;
     const StepConst &C = A.C;
@@ -672,12 +667,15 @@ __device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S
 
     // ---- zero-lag imaging condition (we_op.cpp:505-562, VTI :1478-1557)
     if (GRAD && do_grad && (own0 || own1)) {
-        const float *F0 = sm + L::F0, *F1 = sm + L::F1;
-        const float2 t0 = der_x(ld2(F0, i - 2 * kFs), ld2(F0, i - kFs), ld2(F0, i + kFs), ld2(F0, i + 2 * kFs), C.sdx);
-        const float2 t2 = der_x(ld2(F1, i - 2 * kFs), ld2(F1, i - kFs), ld2(F1, i + kFs), ld2(F1, i + 2 * kFs), C.sdx);
-        const float2 f0 = ld2(F0, i), f1 = ld2(F1, i);
-        const float2 t1 = der_z(ld2(F1, i - 2), f1, ld2(F1, i + 2), C.sdz);
-        const float2 t3 = der_z(ld2(F0, i - 2), f0, ld2(F0, i + 2), C.sdz);
+        auto f = [&](int c, int j) {
+            if (S16) return raw2(sm + L::F0, c * kFw + j, prec, inv[1]);
+            return ld2(sm + L::F0, c * kFw + j);
+        };
+        const float2 t0 = der_x(f(0, i - 2 * kFs), f(0, i - kFs), f(0, i + kFs), f(0, i + 2 * kFs), C.sdx);
+        const float2 t2 = der_x(f(1, i - 2 * kFs), f(1, i - kFs), f(1, i + kFs), f(1, i + 2 * kFs), C.sdx);
+        const float2 f0 = f(0, i), f1 = f(1, i);
+        const float2 t1 = der_z(f(1, i - 2), f1, f(1, i + 2), C.sdz);
+        const float2 t3 = der_z(f(0, i - 2), f0, f(0, i + 2), C.sdz);
         float2 dl = make_float2(0.f, 0.f), dm;
         // (two ax0) t0 + ...: doubling is exact, so it commutes with the rounding of every product
         if (!VTI) {
@@ -712,8 +710,13 @@ __device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S
             g1.x = (float)((double)g1.x + wh * (double)dm.x);
             g1.y = (float)((double)g1.y + wh * (double)dm.y);
         }
-        const float2 fp0 = ld2(sm + L::FP0, oi), fp1 = ld2(sm + L::FP0 + kFo, oi);
-        const float2 fm0 = ld2(sm + L::FM0, oi), fm1 = ld2(sm + L::FM0 + kFo, oi);
+        auto near = [&](int base, int c, float iv) {
+            if (S16) return raw2(sm + base, c * kFx * kFs + tx * kFs + pz + 4, prec, iv);
+            return ld2(sm + base + c * kFo, oi);
+        };
+        const float iv0 = S16 ? inv[0] : 1.f, iv2 = S16 ? inv[2] : 1.f;
+        const float2 fp0 = near(L::FP0, 0, iv2), fp1 = near(L::FP0, 1, iv2);
+        const float2 fm0 = near(L::FM0, 0, iv0), fm1 = near(L::FM0, 1, iv0);
         g2.x = density_term(g2.x, wdt, itf, last, n0.x, n1.x, f0.x, f1.x, fp0.x, fp1.x, fm0.x, fm1.x);
         g2.y = density_term(g2.y, wdt, itf, last, n0.y, n1.y, f0.y, f1.y, fp0.y, fp1.y, fm0.y, fm1.y);
         float *G = S.grad + cell;
@@ -754,11 +757,14 @@ __device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S
 // One such CTA sets the time of a step on small plans, and its time is one
 // warp's chain of instructions: so the SAT terms of the edge row, which need
 // the fields only, are formed by warps 6 and 7 beside the rows' derivatives,
-// and whatever depends on the model alone is set up once per unit (keep).
+// and whatever depends on the model alone is set up once per unit (keep).  In
+// the adjoint such a CTA holds the three snapshots around the imaging time and
+// fetches the next one a step ahead (one: the CTA has this unit only; ring: the
+// snapshots are there from the last step).
 // ---------------------------------------------------------------------------
 template <bool XB, bool VTI, bool GRAD, bool AE>
 __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br, const int it, const bool first,
-                                           const bool keep, float *sm)
+                                           const bool keep, const bool one, bool &ring, float *sm)
 {
     using L = BandLayout<VTI, GRAD, AE>;
     const ModelDev &M = A.M;
@@ -882,54 +888,102 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
         SF[SL_R0 * kFt] = __int_as_float(r0);
         SF[SL_R1 * kFt] = __int_as_float(r1);
     }
-    // this step's injected values, in the entries' order, and a look ahead at the next row
+    // loads that nothing waits for yet: the rows of this step's injected values, the snapshot two
+    // imaging times on; then the snapshots around this one where they are not there from the last step
     const int inj0 = Sp->inj_off[br.unit], ninj = Sp->inj_off[br.unit + 1] - inj0;
-    if (it < nt - 1 && ninj <= kVal) {
-        const float *srcrow = Sp->src + (long long)it * Sp->nsrc;
+    const bool cached = ninj <= L::NVAL, act = it < nt - 1;
+    const float *srcrow = Sp->src + (long long)it * Sp->nsrc;
+    constexpr int NE = L::NVAL / kFt;
+    if (!one && act && cached) {
         for (int e = t; e < ninj; e += kFt) {
             const InjEntry &E = Sp->inj[inj0 + e];
             sm[L::VAL + e] = E.mt ? (E.wa * srcrow[E.ia] - E.wb * srcrow[E.ib]) : E.wa * srcrow[E.ia];
-            if (it + 1 < nt) asm volatile("prefetch.global.L2 [%0];" ::"l"(srcrow + Sp->nsrc + E.ia));
         }
     }
-    float fp0 = 0.f, fp1 = 0.f, fm0 = 0.f, fm1 = 0.f;
-    if (GRAD && do_grad) {
-        // loads first: they come from HBM
-        const long long so = (long long)itf * Sp->snap_slot;
-        float a_[2], b_[2];
-        const float inv = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, itf);
+    if (one && !keep && cached) {
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            a_[h] = in_[h] ? snap_load(Sp->snap, so + o_[h], prec, inv) : 0.f;
-            b_[h] = in_[h] ? snap_load(Sp->snap, so + o_[h] + nxz, prec, inv) : 0.f;
-        }
-        if (owned && itf + 1 <= last) {
-            const float ip = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, itf + 1);
-            fp0 = snap_load(Sp->snap, so + Sp->snap_slot + cell, prec, ip);
-            fp1 = snap_load(Sp->snap, so + Sp->snap_slot + cell + nxz, prec, ip);
-        }
-        if (owned && itf > 0) {
-            const float im = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, itf - 1);
-            fm0 = snap_load(Sp->snap, so - Sp->snap_slot + cell, prec, im);
-            fm1 = snap_load(Sp->snap, so - Sp->snap_slot + cell + nxz, prec, im);
-        }
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-            if (s_[h] >= 0) {
-                sm[L::F0 + s_[h]] = a_[h];
-                sm[L::F1 + s_[h]] = b_[h];
-            }
-        // the next imaging step's new snapshot, from HBM to L2
-        if (itf - Sp->snap_first >= 2) {
-            const int esz = prec == SNAP_FP32 ? 4 : 2;
-#pragma unroll
-            for (int h = 0; h < 2; h++)
-                if (in_[h]) {
-                    const char *p = (const char *)Sp->snap + (so - 2 * Sp->snap_slot + o_[h]) * esz;
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (long long)nxz * esz));
+        for (int h = 0; h < NE; h++) {
+            const int e = t + h * kFt;
+            if (e < ninj) {
+                const InjEntry E = Sp->inj[inj0 + e];
+                sm[L::WA + e] = E.wa;
+                sm[L::IA + e] = __int_as_float(E.ia);
+                if (!GRAD) {
+                    sm[L::WB + e] = E.wb;
+                    sm[L::IB + e] = __int_as_float(E.mt ? E.ib : -1);
                 }
+            }
         }
+    }
+    float sv[NE], sw = 0.f;
+#pragma unroll
+    for (int h = 0; h < NE; h++) {
+        const int e = t + h * kFt;
+        sv[h] = 0.f;
+        if (one && act && cached && e < ninj) {
+            const int ia = __float_as_int(sm[L::IA + e]);
+            sv[h] = srcrow[ia];
+            if (!GRAD) {
+                const int ib = __float_as_int(sm[L::IB + e]);
+                if (ib >= 0) sw = srcrow[ib];
+            }
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(srcrow + Sp->nsrc + ia));
+        }
+    }
+    float na_[2] = {0.f, 0.f}, nb_[2] = {0.f, 0.f};
+    const bool more = GRAD && do_grad && itf - Sp->snap_first >= 2;
+    if (GRAD && do_grad) {
+        auto load = [&](int k, float (&a)[2], float (&b)[2]) {
+            const float inv = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, k);
+            const long long so = (long long)k * Sp->snap_slot;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                a[h] = in_[h] ? snap_load(Sp->snap, so + o_[h], prec, inv) : 0.f;
+                b[h] = in_[h] ? snap_load(Sp->snap, so + o_[h] + nxz, prec, inv) : 0.f;
+            }
+        };
+        if (ring) {
+            if (more) load(itf - 2, na_, nb_);
+        } else {
+            // the window at this time; the neighbours at the own cells (a unit that is kept: their windows)
+            float a[2], b[2];
+            auto own = [&](int k, bool have, float &x, float &y) {
+                x = y = 0.f;
+                if (!owned || !have) return;
+                const float inv = prec == SNAP_FP32 ? 1.f : 1.f / snap_scale(Sp->snap_amax, k);
+                x = snap_load(Sp->snap, (long long)k * Sp->snap_slot + cell, prec, inv);
+                y = snap_load(Sp->snap, (long long)k * Sp->snap_slot + cell + nxz, prec, inv);
+            };
+            auto put = [&](int k) {
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    if (s_[h] >= 0) {
+                        sm[L::snap(k, 0) + s_[h]] = a[h];
+                        sm[L::snap(k, 1) + s_[h]] = b[h];
+                    }
+            };
+            float fp0, fp1, fm0, fm1;
+            load(itf, a, b);
+            own(itf + 1, itf + 1 <= last, fp0, fp1);
+            own(itf - 1, !one && itf > 0, fm0, fm1);
+            put(itf);
+            const int c = row * kFs + lane + 2;
+            if (owned) {
+                sm[L::snap(itf + 1, 0) + c] = fp0;
+                sm[L::snap(itf + 1, 1) + c] = fp1;
+            }
+            if (one) {
+                if (itf > 0) {
+                    load(itf - 1, a, b);
+                    put(itf - 1);
+                }
+                if (more) load(itf - 2, na_, nb_);
+            } else if (owned) {
+                sm[L::snap(itf - 1, 0) + c] = fm0;
+                sm[L::snap(itf - 1, 1) + c] = fm1;
+            }
+        }
+        ring = one;
     }
     const bool edge = owned && (gz == 0 || gz == nz - 1 || gx == 0 || gx == nx - 1);
     const float *curr = Sp->u[(it + 1) & 1];
@@ -964,7 +1018,20 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
             if (s_[h] >= 0) {
                 sm[L::UN + s_[h]] = a_[h];
                 sm[L::UT + s_[h]] = b_[h];
+                if (GRAD && more && one) {
+                    sm[L::snap(itf - 2, 0) + s_[h]] = na_[h];
+                    sm[L::snap(itf - 2, 1) + s_[h]] = nb_[h];
+                }
             }
+#pragma unroll
+        for (int h = 0; h < NE; h++) {
+            const int e = t + h * kFt;
+            if (one && cached && e < ninj) {
+                float v = sm[L::WA + e] * sv[h];
+                if (!GRAD && __float_as_int(sm[L::IB + e]) >= 0) v = v - sm[L::WB + e] * sw;
+                sm[L::VAL + e] = v;
+            }
+        }
     }
     __syncthreads();
 
@@ -1198,8 +1265,7 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
         if (nx_ + nz_ > 0) {
             const int e = __float_as_int(SF[SL_E0 * kFt]);
             auto value = [&](int k) {
-                if (ninj <= kVal) return sm[L::VAL + k];
-                const float *srcrow = Sp->src + (long long)it * Sp->nsrc;
+                if (cached) return sm[L::VAL + k];
                 const InjEntry &E = Sp->inj[inj0 + k];
                 return E.mt ? (E.wa * srcrow[E.ia] - E.wb * srcrow[E.ib]) : E.wa * srcrow[E.ia];
             };
@@ -1264,7 +1330,7 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
         if (GRAD && do_grad) {
             // strains of the adjoint field (this thread's own) and of the snapshot
             const float ax0 = XB ? en : et, az1 = XB ? et : en, ax1 = XB ? es : eq, az0 = XB ? eq : es;
-            const int FN = XB ? L::F0 : L::F1, FT = XB ? L::F1 : L::F0;
+            const int F0 = L::snap(itf, 0), F1 = L::snap(itf, 1), FN = XB ? F0 : F1, FT = XB ? F1 : F0;
             const float qn = dern(FN), qt = dert(FT), qs = dern(FT), qq = dert(FN);
             const float q0 = XB ? qn : qt, q1 = XB ? qt : qn, q2 = XB ? qs : qq, q3 = XB ? qq : qs;
             float dl = 0.f, dm;
@@ -1292,8 +1358,9 @@ __device__ __forceinline__ bool fused_band(const FusedArgs &A, const BandRef br,
             G[nxz] = g1;
             // interface row: the density term needs the coupled uz (ae_couple)
             if (!AE || gz != 0)
-                G[2 * (long long)nxz] = density_term(g2, wdt, itf, last, n0, n1, sm[L::F0 + i], sm[L::F1 + i], fp0, fp1,
-                                                     fm0, fm1);
+                G[2 * (long long)nxz] = density_term(g2, wdt, itf, last, n0, n1, sm[F0 + i], sm[F1 + i],
+                                                     sm[L::snap(itf + 1, 0) + i], sm[L::snap(itf + 1, 1) + i],
+                                                     sm[L::snap(itf - 1, 0) + i], sm[L::snap(itf - 1, 1) + i]);
         }
     }
     if (!GRAD && (A.flags & F_AMAX) && (it + 1) % C.sub == 0)
@@ -1643,7 +1710,7 @@ __device__ __forceinline__ void fetch16(void *dst, const void *src, int bytes, i
 // one unit anyway and a step lasts as long as a band unit's chain of
 // instructions: 8 shots of 801 x 401 52.1 -> 45.7 us a step with five, but one
 // 81 x 61 shot 5.9 -> 6.4 us.
-template <bool VTI, bool GRAD, bool AE, int BLOCKS>
+template <bool VTI, bool GRAD, bool AE, bool S16, int BLOCKS>
 __global__ void __launch_bounds__(kFt, BLOCKS)
 fused_steps(const __grid_constant__ FusedArgs A)
 {
@@ -1672,7 +1739,9 @@ fused_steps(const __grid_constant__ FusedArgs A)
     auto window = [&](int q) { return A.in + (unit(w0 + q % nw) - A.nband); };
     int q = 0;   // windows done so far
     unsigned par_lead = 0, par_own = 0;
+    bool ring = false;
     __shared__ unsigned long long bars[2];
+    __shared__ float inv_[2][3];   // S16: factors of the snapshots before, at and after the imaging time
     unsigned long long *const lead = bars, *const own = bars + 1;
     if (nw > 0) {
         if (threadIdx.x == 0) {
@@ -1692,8 +1761,8 @@ fused_steps(const __grid_constant__ FusedArgs A)
         for (int m = 0; m < n; m++) {
             if (nw > 0 && m >= w0 && m < w0 + nw) continue;
             const BandRef br = A.bands[unit(m)];
-            const bool ok = br.side >= 2 ? fused_band<true, VTI, GRAD, AE>(A, br, it, first, keep, sm)
-                                         : fused_band<false, VTI, GRAD, AE>(A, br, it, first, keep, sm);
+            const bool ok = br.side >= 2 ? fused_band<true, VTI, GRAD, AE>(A, br, it, first, keep, one, ring, sm)
+                                         : fused_band<false, VTI, GRAD, AE>(A, br, it, first, keep, one, ring, sm);
             if (!ok) return;
             first = false;
             __syncthreads();
@@ -1722,7 +1791,7 @@ fused_steps(const __grid_constant__ FusedArgs A)
                         issue_lead<VTI, GRAD, AE>(A, S, tr, it, !keep, false, sm, lead);
                         issue_own_static<VTI, GRAD, AE>(A, S, tr, it, !keep, sm, own);
                     }
-                    load_snaps16<VTI, GRAD, AE>(A, S, tr, it, sm);
+                    if (S16) set_factors(S, imaging<GRAD, AE>(S, A.C, it), inv_[q & 1]);
                 }
                 if (first && !meet<AE>(A, it)) return;
                 if (active && threadIdx.x == 0) {
@@ -1747,8 +1816,8 @@ fused_steps(const __grid_constant__ FusedArgs A)
                 return true;
             };
             if (active) {
-                if (!window_step<VTI, GRAD, AE>(
-                        A, S, tr, it, sm, [&]() { return wait_bar(A, lead, par_lead, it); }, ahead))
+                if (!window_step<VTI, GRAD, AE, S16>(
+                        A, S, tr, it, sm, inv_[q & 1], [&]() { return wait_bar(A, lead, par_lead, it); }, ahead))
                     return;
             } else if (!ahead(true)) {
                 return;
@@ -1761,7 +1830,7 @@ fused_steps(const __grid_constant__ FusedArgs A)
                     issue_own_static<VTI, GRAD, AE>(A, Sn, tn, it, true, sm, own);
                     issue_own_fields<VTI, GRAD, AE>(A, Sn, tn, it, sm, own);
                 }
-                load_snaps16<VTI, GRAD, AE>(A, Sn, tn, it, sm);
+                if (S16) set_factors(Sn, imaging<GRAD, AE>(Sn, A.C, it), inv_[(q + 1) & 1]);
             }
         }
         if (nw == 0) {
@@ -1856,20 +1925,24 @@ static cudaError_t launch_fused_t(const FusedArgs &A, cudaStream_t st)
 {
     constexpr size_t bytes = fused_bytes<VTI, GRAD, AE>();
     if constexpr (GRAD) {
-        return launch_loop(fused_steps<VTI, GRAD, AE, VTI ? 3 : 4>, A, A.nunit, bytes, A.count, st);
+        constexpr int blocks = VTI ? 3 : 4;
+        if (A.C.snap_prec != SNAP_FP32)
+            return launch_loop(fused_steps<VTI, GRAD, AE, true, blocks>, A, A.nunit, bytes, A.count, st);
+        return launch_loop(fused_steps<VTI, GRAD, AE, false, blocks>, A, A.nunit, bytes, A.count, st);
     } else {
         int dev = 0, sms = 0;
         cudaError_t e = cudaGetDevice(&dev);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return e;
-        if (A.nunit <= 4 * sms) return launch_loop(fused_steps<VTI, GRAD, AE, 4>, A, A.nunit, bytes, A.count, st);
-        return launch_loop(fused_steps<VTI, GRAD, AE, 5>, A, A.nunit, bytes, A.count, st);
+        if (A.nunit <= 4 * sms) return launch_loop(fused_steps<VTI, GRAD, AE, false, 4>, A, A.nunit, bytes, A.count, st);
+        return launch_loop(fused_steps<VTI, GRAD, AE, false, 5>, A, A.nunit, bytes, A.count, st);
     }
 }
 
 // ---- tensor maps ----------------------------------------------------------------
 // cuTensorMapEncodeTiled through the runtime (the library does not link the driver)
-static cudaError_t encode(CUtensorMap *m, const void *base, int rank, const cuuint64_t *dim, const cuuint32_t *box)
+static cudaError_t encode(CUtensorMap *m, const void *base, int rank, const cuuint64_t *dim, const cuuint32_t *box,
+                          bool half = false)
 {
     using Fn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                             const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -1881,9 +1954,9 @@ static cudaError_t encode(CUtensorMap *m, const void *base, int rank, const cuui
     if (!f || q != cudaDriverEntryPointSuccess) return cudaErrorNotSupported;
     cuuint64_t stride[3];
     cuuint32_t one[4] = {1, 1, 1, 1};
-    cuuint64_t s = sizeof(float);
+    cuuint64_t s = half ? 2 : 4;
     for (int i = 0; i + 1 < rank; i++) stride[i] = s *= dim[i];
-    const CUresult r = ((Fn)f)(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, rank, const_cast<void *>(base), dim, stride, box, one,
+    const CUresult r = ((Fn)f)(m, half ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, rank, const_cast<void *>(base), dim, stride, box, one,
                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
@@ -1892,7 +1965,7 @@ static cudaError_t encode(CUtensorMap *m, const void *base, int rank, const cuui
 size_t fused_maps_bytes() { return SM_COUNT * sizeof(CUtensorMap); }
 
 cudaError_t fused_shot_maps(void *out, int nx, int ldz, const float *u0, const float *u1, const float *grad,
-                            const float *snap, int nslot)
+                            const void *snap, int nslot, bool half)
 {
     CUtensorMap *m = (CUtensorMap *)out;
     std::memset(m, 0, fused_maps_bytes());
@@ -1907,8 +1980,10 @@ cudaError_t fused_shot_maps(void *out, int nx, int ldz, const float *u0, const f
     }
     if (e == cudaSuccess && grad) e = encode(m + SM_GRAD, grad, 3, d3, g);
     if (e == cudaSuccess && snap && nslot > 0) {
-        e = encode(m + SM_SNAP_LEAD, snap, 4, ds, sl);
-        if (e == cudaSuccess) e = encode(m + SM_SNAP_OWN, snap, 4, ds, own);
+        // 16-bit: the own cells from the window's first sample but four on, a multiple of 16 bytes
+        const cuuint32_t raw[4] = {kFs, kFx, 2, 1};
+        e = encode(m + SM_SNAP_LEAD, snap, 4, ds, sl, half);
+        if (e == cudaSuccess) e = encode(m + SM_SNAP_OWN, snap, 4, ds, half ? raw : own, half);
     }
     return e;
 }

@@ -50,10 +50,11 @@ cudaError_t launch_fused(int kind, const ShotDev *shots, const BandRef *bands, i
 // the same for the acoustic propagator, over 32 x 16 tiles of the whole grid
 cudaError_t launch_acoustic_loop(const ShotDev *shots, const TileRef *tiles, int ntile, const ModelDev &M, const StepConst &C,
                                  int it0, int it1, int flags, float dtg, unsigned *count, int *status, cudaStream_t st);
-// tensor maps of a shot (ShotMap, host memory of fused_maps_bytes()); grad / snap may be null
+// tensor maps of a shot (ShotMap, host memory of fused_maps_bytes()); grad / snap may be null;
+// half: 16-bit snapshots
 size_t fused_maps_bytes();
 cudaError_t fused_shot_maps(void *out, int nx, int ldz, const float *u0, const float *u1, const float *grad,
-                            const float *snap, int nslot);
+                            const void *snap, int nslot, bool half);
 // closure sums of the six rows next to both ends of an axis of n samples (stride sn) on `lines` lines (stride sl)
 void launch_closures(const float *f, float *out, int lines, int ld, int n, long long sl, long long sn, cudaStream_t st);
 // top / bottom band kernel (rows clear of the x bands), zband_rows(split)

@@ -202,6 +202,7 @@ __device__ __forceinline__ float2 der_z(float2 lo, float2 mid, float2 hi, float 
 // S: the products lambda (ux_x + uz_z), mu ux_z and mu uz_x of the mixed terms,
 // formed once per cell (VTI: P = tmp_x and P1 = tmp_z; acoustic-elastic: P =
 // lambda ux_x, P1 = lambda uz_z).  O: the window's own cells, 32 x 16 each.
+constexpr int kWin = 256;   // injection entries of a window that are staged
 template <bool VTI, bool GRAD, bool AE>
 struct InLayout {
     static constexpr int U0 = 0, U1 = kFu, MU = 2 * kFu, Q = MU + kFw, P = Q + kFw, R = P + kFw, S = R + kFw;
@@ -212,7 +213,8 @@ struct InLayout {
     static constexpr int PV0 = O, PV1 = O + kFo, RHO = O + 2 * kFo, IR = O + 3 * kFo, G0 = O + 4 * kFo;
     static constexpr int FP0 = G0 + (GRAD ? 3 * kFo : 0), FM0 = FP0 + (GRAD ? 2 * kFo : 0);
     static constexpr int E = FM0 + (GRAD ? 2 * kFo : 0);   // VTI imaging: eps, v2, v3
-    static constexpr int RED = E + (VTI && GRAD ? 3 * kFo : 0);
+    static constexpr int VAL = E + (VTI && GRAD ? 3 * kFo : 0), KEY = VAL + kWin;   // injected values and their cells
+    static constexpr int RED = KEY + kWin;
     static constexpr int FLOATS = RED + 8;
 };
 
@@ -499,6 +501,14 @@ __device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S
         tzv = *reinterpret_cast<const float2 *>(S.tz + gz);
         txv = S.tx[gx];
     }
+    // the window's injected values and their cells and components (entries sorted by cell)
+    const int e0 = GRAD ? tr.ea0 : tr.ef0, ne = (GRAD ? tr.ea1 : tr.ef1) - e0;
+    const float *srcrow = S.src + (long long)it * S.nsrc;
+    if (ne > 0 && ne <= kWin && t < ne) {
+        const InjEntry &E = S.inj[e0 + t];
+        sm[L::VAL + t] = E.mt ? (E.wa * srcrow[E.ia] - E.wb * srcrow[E.ib]) : E.wa * srcrow[E.ia];
+        sm[L::KEY + t] = __int_as_float(2 * ((E.gx - tr.wx0) * kFz + E.gz - tr.wz0) + E.comp);
+    }
     const bool here = wait_lead();
     const float *U0 = sm + L::U0 + 2 * kFs, *U1 = sm + L::U1 + 2 * kFs;   // indexed as the 2-halo arrays
     const float *MU = sm + L::MU, *Q = sm + L::Q;
@@ -602,21 +612,31 @@ __device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S
 
     const int cell = gx * ldz + gz;
     // sources, cell by cell in the reference's order
-    const int e0 = GRAD ? tr.ea0 : tr.ef0, e1 = GRAD ? tr.ea1 : tr.ef1;
-    if (e0 < e1) {
-        const float *srcrow = S.src + (long long)it * S.nsrc;
-        for (int e = e0; e < e1; e++) {
-            const InjEntry &E = S.inj[e];
-            if (E.gx == gx && (E.gz == gz || E.gz == gz + 1)) {
-                const float v = E.mt ? (E.wa * srcrow[E.ia] - E.wb * srcrow[E.ib]) : E.wa * srcrow[E.ia];
-                if (E.comp == 0) {
-                    if (E.gz == gz) n0.x += v;
-                    else n0.y += v;
-                } else {
-                    if (E.gz == gz) n1.x += v;
-                    else n1.y += v;
-                }
-            }
+    if (ne > 0) {
+        auto value = [&](int e) {
+            if (ne <= kWin) return sm[L::VAL + e];
+            const InjEntry &E = S.inj[e0 + e];
+            return E.mt ? (E.wa * srcrow[E.ia] - E.wb * srcrow[E.ib]) : E.wa * srcrow[E.ia];
+        };
+        auto key = [&](int e) {
+            if (ne <= kWin) return __float_as_int(sm[L::KEY + e]);
+            const InjEntry &E = S.inj[e0 + e];
+            return 2 * ((E.gx - tr.wx0) * kFz + E.gz - tr.wz0) + E.comp;
+        };
+        const int k = 2 * (tx * kFz + pz);   // of the pair's first cell: keys k .. k + 3
+        int lo = 0, hi = ne;
+        while (lo < hi) {
+            const int m = (lo + hi) >> 1;
+            if (key(m) < k) lo = m + 1;
+            else hi = m;
+        }
+        for (; lo < ne && key(lo) <= k + 3; lo++) {
+            const float v = value(lo);
+            const int d = key(lo) - k;
+            if (d == 0) n0.x += v;
+            else if (d == 1) n1.x += v;
+            else if (d == 2) n0.y += v;
+            else n1.y += v;
         }
     }
     float *pn = S.u[it & 1];   // prev in, next out

@@ -101,11 +101,19 @@ FRAMED_CAPTURES = {
 }
 
 
+# the fused time loop (the last shape), and the DRAM bytes of one adjoint step of
+# the single-shot grid from an ncu capture of 50 steps (152.0 MB read, 5.0 MB written)
+FUSED_SHAPE, FUSED_STEP_BYTES = 18, 3.15e6
+
+
 def roof_kernel(shape, config):
     if config == "single" and shape in FRAMED_CAPTURES:
         return ("adjoint + imaging step of the framed plan: interior %s with the band kernels elastic_xband and "
                 "elastic_zband<SPLIT> (a cell's two components in two warps) overlapped on two side streams "
                 "(one step = one launch of each)" % FRAMED_CAPTURES[shape]["core"])
+    if config == "single" and shape == FUSED_SHAPE:
+        return ("fused_steps<GRAD>: the whole adjoint loop with imaging in one cooperative launch over band units and "
+                "32 x 16 windows (achieved: per step)")
     if config == "single":
         return "adjoint + imaging step (tile shape %d)" % shape
     return "adjoint loop: interior, band and imaging kernels"
@@ -114,6 +122,8 @@ def roof_kernel(shape, config):
 def step_traffic(shape, config):
     """DRAM bytes of one adjoint step from the committed ncu summaries, or
     None when the plan's launches are not captured."""
+    if config == "single" and shape == FUSED_SHAPE:
+        return FUSED_STEP_BYTES
     cap = FRAMED_CAPTURES.get(shape) if config == "single" else None
     if not cap or not cap["traffic"]:
         return None
@@ -664,7 +674,8 @@ def run_batched(local, steps, warmup):
     half = cells / 2
     fwd_gbs = (BYTES_FWD + VTI_EXTRA) * half / (fwd_ms / 1e3) / 1e9
     adj_gbs = (BYTES_ADJ + VTI_EXTRA) * half / (adj_ms / 1e3) / 1e9
-    roof = {"bound": "hbm", "kernel": "elastic_march<VTI> + band kernels (adjoint + imaging)", "achieved": adj_gbs,
+    roof = {"bound": "hbm", "kernel": ("fused_steps<VTI, GRAD> (adjoint + imaging)" if info["tile_shape"] == FUSED_SHAPE
+                                       else "launch-per-step plan (adjoint + imaging)"), "achieved": adj_gbs,
             "peak": peak, "unit": "GB/s", "frac": adj_gbs / peak, "peak_source": peak_kind,
             "bytes_per_cell_update": {"forward": BYTES_FWD + VTI_EXTRA, "adjoint": BYTES_ADJ + VTI_EXTRA},
             "forward_achieved": fwd_gbs, "forward_frac": fwd_gbs / peak}
@@ -684,13 +695,6 @@ def run_batched(local, steps, warmup):
     except Exception as e:
         out["fp64_error"] = {"unavailable": "failed: %s" % e}
     return out
-
-
-# plan of the large-grid workload, pinned so that the bench does not run the
-# tuner's whole-pass stage, whose passes take tens of seconds on this grid:
-# the framed plan with 32 x 8 interior windows (on 2 shots it measured 18.9
-# Gcell/s against 17.7 for the best marching shape, 224 x 32)
-LARGE_TILE_SHAPE = 14
 
 
 def run_ae(local, nshots=8):
@@ -774,7 +778,7 @@ def run_large(local, nshots=4):
     checkpoint-and-recompute every 200 steps) on one GPU; returns a dict."""
     from fwi2d_b200 import workloads as W
     wl = W.elastic_large(nshots=nshots)
-    ms, fwd_ms, adj_ms, info, nwaves, _ = timed_gradients(wl, local, 1, 1, tile_shape=LARGE_TILE_SHAPE)
+    ms, fwd_ms, adj_ms, info, nwaves, _ = timed_gradients(wl, local, 1, 1)
     cells = cells_per_step(wl)
     out = {"workload": "elastic FWI gradient, %d shots of the 1201 x 4001 grid at 2.5 m, nt = 16001, FP16 "
                        "snapshots rebuilt by checkpoint-and-recompute every 200 steps" % nshots,

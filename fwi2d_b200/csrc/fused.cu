@@ -20,6 +20,16 @@
 // for the others, and keeps it in shared memory from step to step when it has
 // one unit only.
 //
+// What bounds it (801 x 401, FP32 snapshots every step, forward / adjoint):
+//   one shot     the meetings: 10 of the cycles between a warp's instructions are
+//                waits at a barrier; 8.3 / 11.9 us a step, 16.1 / 21.5 in three
+//                launches a step;
+//   eight shots  latency between a window's halves (0.53 / 0.39 instructions per
+//                cycle and scheduler), then the shared-memory pipe (62 / 49 %);
+//                47.6 / 81 us a step, 87 / 139 before.
+// One 4001 x 1201 shot: 77.6 / 111 us a step, the adjoint at 68 % of a copy's DRAM
+// rate (98 B per cell and step).
+//
 // Everything a step writes is read through L2 (.cg), written by the SM that
 // owns the cell and read by its neighbours after the counter.
 #include <cuda.h>
@@ -1696,7 +1706,10 @@ struct AcousticArgs {
     int *status;
 };
 
-// The time loop of the acoustic propagator.
+// The time loop of the acoustic propagator.  Bound by the tiles beside a closure
+// (general forms, double-precision quotients), which 8-column units keep short:
+// three 401 x 301 shots 23 / 30 us a step forward / adjoint in launches per step,
+// 11.5 / 21.7 here.
 template <bool GRAD>
 __global__ void __launch_bounds__(kFt, GRAD ? 3 : 4) acoustic_steps(const __grid_constant__ AcousticArgs A)
 {

@@ -246,7 +246,9 @@ int fwi2d_last_timing(fwi2d_ctx *ctx, float *forward_ms, float *adjoint_ms);
  * cell each, marching runs of tx rows) for the cells clear of the boundary
  * bands, then framed tile shapes (tz x tx tiles of the tile kernel's interior
  * path over those cells); marching and framed plans run the boundary bands on
- * the band kernels. */
+ * the band kernels.  The last shape is the fused time loop: all steps of a
+ * pass in one launch over tz x tx windows and band units; a plan that leaves
+ * the shape open takes it wherever its grids fit. */
 int fwi2d_tile_shape_count(void);
 int fwi2d_tile_shape(int index, int *tz, int *tx);
 

@@ -561,7 +561,7 @@ static bool band_split_for(int nshots, int nz)
 // Microseconds a step, forward / adjoint, launch-per-step plan as tuned -> fused:
 // one 801 x 401 shot 16.1 / 21.5 -> 8.3 / 11.9, eight of them 87 / 139 -> 48 / 81;
 // one 81 x 61 shot 14.6 / 15 or more -> 4.8 / 7.1; three acoustic 401 x 301 shots
-// 23 / 30 -> 11.5 / 21.7.
+// 23 / 30 -> 11.5 / 19.1.
 static int fused_shape() { return elastic_tile_count() + kNumMarch + kNumFramed; }
 static int shape_count() { return fused_shape() + 1; }
 static bool is_march_shape(int s) { return s >= elastic_tile_count() && s < elastic_tile_count() + kNumMarch; }

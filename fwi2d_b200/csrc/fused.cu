@@ -1709,9 +1709,11 @@ struct AcousticArgs {
 // The time loop of the acoustic propagator.  Bound by the tiles beside a closure
 // (general forms, double-precision quotients), which 8-column units keep short:
 // three 401 x 301 shots 23 / 30 us a step forward / adjoint in launches per step,
-// 11.5 / 21.7 here.
+// 11.5 / 19.1 here.  Four CTAs per SM: the adjoint takes 21.4 us with three (its
+// units are many more than the CTAs), the forward 17.2 with five;
+// one 201 x 151 shot, a tile per CTA, 7.88 us and 7.76 with three.
 template <bool GRAD>
-__global__ void __launch_bounds__(kFt, GRAD ? 3 : 4) acoustic_steps(const __grid_constant__ AcousticArgs A)
+__global__ void __launch_bounds__(kFt, 4) acoustic_steps(const __grid_constant__ AcousticArgs A)
 {
     extern __shared__ __align__(1024) float sm[];
     const int G = gridDim.x;

@@ -745,7 +745,11 @@ __device__ __forceinline__ bool window_step(const FusedArgs &A, const ShotDev &S
             return ld2(sm + base + c * kFo, oi);
         };
         const float iv0 = S16 ? inv[0] : 1.f, iv2 = S16 ? inv[2] : 1.f;
-        const float2 fp0 = near(L::FP0, 0, iv2), fp1 = near(L::FP0, 1, iv2);
+        // no snapshot follows the last one, which is also the first where sub exceeds the record: nothing is
+        // loaded for it then, and it counts as zero
+        const bool next = itf + 1 <= last;
+        const float2 none = make_float2(0.f, 0.f);
+        const float2 fp0 = next ? near(L::FP0, 0, iv2) : none, fp1 = next ? near(L::FP0, 1, iv2) : none;
         const float2 fm0 = near(L::FM0, 0, iv0), fm1 = near(L::FM0, 1, iv0);
         g2.x = density_term(g2.x, wdt, itf, last, n0.x, n1.x, f0.x, f1.x, fp0.x, fp1.x, fm0.x, fm1.x);
         g2.y = density_term(g2.y, wdt, itf, last, n0.y, n1.y, f0.y, f1.y, fp0.y, fp1.y, fm0.y, fm1.y);

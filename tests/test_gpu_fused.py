@@ -111,6 +111,48 @@ def test_fused_plan_equals_tile_plan(kind, prec, every, compensated):
         assert np.array_equal(x, y)
 
 
+def _imaging(kind, shape, prec, sub, nt=61):
+    """Forward and adjoint imaging on one context, first with a snapshot every
+    step, whose values stay in the CTAs' shared memory, then with every sub-th."""
+    nx, nz, d = 61, 107, 0.01
+    base = O.KIND_ELASTIC if kind == O.KIND_AE else kind
+    mc = K.converted(base, K.model_case(base, nx, nz, d, seed=5))
+    oz = 19 * d if kind == O.KIND_AE else 0.0
+    rx, rz = np.linspace(0.05, 0.55, 11).astype(np.float32), np.full(11, 0.04, np.float32)
+    kw = {}
+    if kind == O.KIND_AE:
+        kw = dict(water_src_x=[0.303], water_src_z=[0.12], water_rcv_x=rx, water_rcv_z=rz)
+    shot = F.ShotSpec(0, nx, nt, [0.303], [0.3 + oz], rx, rz + np.float32(oz), **kw)
+    ns = 1 if kind in (O.KIND_AE, O.KIND_ACOUSTIC) else 2
+    nc = {O.KIND_AE: 3, O.KIND_ACOUSTIC: 1}.get(kind, 2)
+    src = [K.sources(ns, nt, 1e-3, f0=25.0, t0=0.03).reshape(ns, 1, nt)]
+    adj = [np.random.default_rng(9).normal(size=(nc, 11, nt)).astype(np.float32)]
+    P = F.Propagator(0)
+    P.set_model(kind, mc, d, d, 0.0, oz)
+    for every in (1, sub):
+        pd = K.par_dict(nt=nt, dt=1e-3, taper=(0, 6, 6, 6), sub=every)
+        if kind == O.KIND_AE:
+            pd.update(nza=20, acoustic_source=1)
+        P.set_shots(F.make_params(**pd, tile_shape=shape, snapshot_precision=prec), [shot])
+        P.forward(src, store=True)
+        g = P.adjoint(adj)
+    P.close()
+    return g
+
+
+@pytest.mark.parametrize("kind", [O.KIND_ELASTIC, O.KIND_VTI, O.KIND_AE, O.KIND_ACOUSTIC])
+@pytest.mark.parametrize("prec,sub", [(0, 2), (0, 7), (0, 59), (0, 60), (0, 62), (2, 3), (2, 100), (1, 63)])
+def test_fused_subsampled_imaging_equals_tile_plan(kind, prec, sub):
+    """Snapshots every sub steps of 61 samples, up to one snapshot only (sub
+    beyond the record: the first is the last, and none follows it)."""
+    if kind == O.KIND_AE and prec:
+        pytest.skip("16-bit snapshots do not hold the acoustic-elastic interface row")
+    a, b = _imaging(kind, fused_shape(), prec, sub), _imaging(kind, 3, prec, sub)
+    assert np.array_equal(a, b)
+    if kind in (O.KIND_ELASTIC, O.KIND_VTI):
+        assert (np.abs(b).max() > 0) == (sub < 62)   # the field at time 0 is zero
+
+
 @pytest.mark.parametrize("bc", [(1, 2, 2, 2), (3, 1, 2, 3)])
 @pytest.mark.parametrize("grid", [(24, 40), (40, 47), (61, 107), (150, 210)])
 def test_acoustic_loop_vs_oracle(bc, grid):

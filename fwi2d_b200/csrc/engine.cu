@@ -498,8 +498,8 @@ static void upload_model_values(fwi2d_ctx *ctx, const float *model)
 // ---- plan construction -------------------------------------------------------
 static int owner_tile(int g, int n, int T)
 {
-    if (g >= n - T) return (n + T - 1) / T - 1;
-    return g / T;
+    const int ntile = (n + T - 1) / T;
+    return ntile > 1 && g >= last_tile_first(n, T) ? ntile - 1 : g / T;
 }
 
 static void check_injector(const fwi2d_injector &J, int nx, int nz, const char *what)

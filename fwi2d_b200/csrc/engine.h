@@ -155,15 +155,23 @@ struct BandRef {
     int side, roff;
 };
 
-// Tile k of an axis of n samples with tiles of T (n == T or n >= T + 8):
-// the window [min(kT, n-T), +T) owns the cells up to the next window, the
-// last window is flush with the far boundary.
+// First sample owned by the last of several tiles of T on an axis of n > T
+// samples.  Its window is flush with the far boundary, at n - T; closer than 8 to
+// the near one it leaves the closure's cells (6, and their 8 samples) to the first
+// tile, whose window holds them: n - T is below 8 on the fluid layers of
+// acoustic-elastic shots only, whose depth and width no tile shape restricts.
+inline int last_tile_first(int n, int T) { return n - T > 8 ? n - T : 8; }
+
+// Tile k of an axis of n samples with tiles of T: the window
+// [min(kT, n-T), +T) owns the cells up to the next window, the last one those
+// from last_tile_first on.
 inline void tile_window_host(int k, int ntile, int n, int T, int &w0, int &o0, int &o1)
 {
     auto w = [&](int i) { return i * T < n - T ? i * T : n - T; };
+    auto first = [&](int i) { return i < ntile - 1 ? i * T : last_tile_first(n, T); };
     w0 = w(k);
-    o0 = k == 0 ? 0 : w(k);
-    o1 = k == ntile - 1 ? n : w(k + 1);
+    o0 = k == 0 ? 0 : first(k);
+    o1 = k == ntile - 1 ? n : first(k + 1);
 }
 
 }  // namespace fwi2d

@@ -117,6 +117,34 @@ def test_ae_vs_oracle(bc, acoustic_source, grid):
     assert e_g <= 1e-5
 
 
+@pytest.mark.parametrize("shape", [-1, 3])
+@pytest.mark.parametrize("bc", [(1, 2, 1, 1), (2, 2, 2, 2)])
+@pytest.mark.parametrize("nx,nza", [(16, 12), (17, 33), (18, 31), (19, 35), (20, 36), (21, 37), (22, 38), (23, 39),
+                                    (24, 40), (41, 37)])
+def test_ae_narrow_and_shallow_fluid_layers(nx, nza, bc, shape):
+    """Widths and depths around one tile of the fluid layer (32 x 16 in the time
+    loop, 32 x 8 in the tile plan): its last tile then starts within the closure
+    of the near boundary, whose cells the first tile keeps."""
+    nz, d, nt = 44, 0.01, 150
+    oz = (nza - 1) * d
+    raw = K.model_case(O.KIND_ELASTIC, nx, nz, d, seed=5)
+    raw[0] += 0.5
+    raw[1] = raw[0] / 1.8
+    mc = K.converted(O.KIND_ELASTIC, raw)
+    pd = K.par_dict(nt=nt, dt=1e-3, bc=bc, taper=(2, 4, 3, 3), nza=nza, acoustic_source=1)
+    rx = np.linspace(0.01, (nx - 2) * d, 9).astype(np.float32)
+    rz_w = np.linspace(0.013, oz - 0.013, 9).astype(np.float32)
+    rz_e = np.full(9, oz + 0.02, np.float32)
+    wsrc = (np.array([0.43 * nx * d], np.float32), np.array([0.052], np.float32))
+    sl = (np.array([0.57 * nx * d], np.float32), np.array([oz + 0.061], np.float32))
+    src = K.sources(1, nt, 1e-3, f0=20.0, t0=0.05).astype(np.float32).reshape(1, 1, nt)
+    r32, g32, _, adj32 = _oracle(32, mc, src, pd, nx, nz, d, oz, sl, rx, rz_e, rz_w, wsrc, 1)
+    rcv, grad, _ = _run(mc, src, pd, nx, nz, d, oz, sl, rx, rz_e, rz_w, wsrc, adj_src=adj32, shape=shape)
+    assert np.abs(rcv).max() > 0 and np.abs(grad).max() > 0
+    assert np.array_equal(rcv, r32)
+    assert np.array_equal(grad, g32)
+
+
 def test_ae_dropin_propagate_matches_reference_golden():
     """fwi2d_propagate with the acoustic-elastic kind: the reference's
     per-shot buffers ([fluid, x, z] traces, [nt+1][2][nx][nz] snapshots) and

@@ -2224,6 +2224,12 @@ static void capture(fwi2d_ctx *ctx, Plan &P, int mode, int w = 0)
         if (adj) CK(cudaMemsetAsync(S->grad.p, 0, S->grad.n, cst));
         if (adj && S->gcomp.p) CK(cudaMemsetAsync(S->gcomp.p, 0, S->gcomp.n, cst));
         if (store && S->amax.p) CK(cudaMemsetAsync(S->amax.p, 0, S->amax.n, cst));
+        // where sub divides nt, slot nt / sub is the neighbour of the last one the forward writes and reads as zero
+        if (store && P.C.sub > 1 && S->nt % P.C.sub == 0) {
+            const size_t slot = (size_t)S->ncomp * S->nx * M.ldz *
+                                (P.par.snapshot_precision == FWI2D_SNAP_FP32 ? 4 : 2);
+            CK(cudaMemsetAsync((char *)S->snap_base + (size_t)(S->nt / P.C.sub) * slot, 0, slot, cst));
+        }
         if (P.ae) {
             CK(cudaMemsetAsync(S->fluid->u0.p, 0, S->fluid->u0.n, cst));
             CK(cudaMemsetAsync(S->fluid->u1.p, 0, S->fluid->u1.n, cst));

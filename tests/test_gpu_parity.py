@@ -115,6 +115,34 @@ def test_deep_source_vs_oracle(kind, shape):
         assert K.rel_l2(g_g[c], g_o[c]) <= GRAD_TOL, "gradient component %d" % c
 
 
+@pytest.mark.parametrize("kind", [O.KIND_ELASTIC, O.KIND_VTI, O.KIND_ACOUSTIC])
+@pytest.mark.parametrize("shape", [-1, 3])
+def test_subsampling_that_divides_the_record_vs_oracle(kind, shape):
+    """sub divides nt: the imaging condition then reads snapshot nt / sub, which
+    no step writes and which counts as zero, whatever the memory held before (a
+    plan with a snapshot every step runs first and leaves its own there)."""
+    nx, nz, d, nt = 60, 64, 0.01, 120
+    mc = K.converted(kind, K.model_case(kind, nx, nz, d, seed=3))
+    sl, rl = K.geometry(nx, nz, d, nr=12)
+    src = K.sources(1 if kind == O.KIND_ACOUSTIC else 2, nt, 1e-3, f0=25.0, t0=0.03)
+    port = O.Port(32)
+    P = F.Propagator(0)
+    P.set_model(kind, mc, d, d)
+    shot = F.ShotSpec(0, nx, nt, sl[0], sl[1], rl[0], rl[1])
+    for sub in (1, 2, 5, nt):
+        pd = K.par_dict(nt=nt, dt=1e-3, sub=sub)
+        par = O.make_par(**pd, ns=1, nr=12)
+        rcv_o, full_o = K.oracle_forward(port, kind, mc, src, par, nx, nz, d, sl, rl)
+        adj = np.ascontiguousarray(rcv_o[:, :, ::-1])
+        g_o = K.oracle_adjoint(port, kind, mc, adj, par, nx, nz, d, sl, rl, full_o)
+        P.set_shots(F.make_params(**pd, tile_shape=shape), [shot])
+        P.forward([src], store=True)
+        g = P.adjoint([adj])
+        for c in range(len(g_o)):
+            assert K.rel_l2(g[c], g_o[c]) <= GRAD_TOL, "sub %d gradient component %d" % (sub, c)
+    P.close()
+
+
 @pytest.mark.parametrize("bc", [(1, 2, 2, 2), (3, 3, 2, 2), (2, 2, 2, 2), (1, 1, 3, 3)])
 @pytest.mark.parametrize("shape,grid", [(2, (72, 80)), (3, (72, 80)), (2, (120, 200)), (3, (60, 251))])
 def test_acoustic_forward_adjoint_vs_oracle(bc, shape, grid):

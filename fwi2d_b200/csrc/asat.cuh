@@ -42,7 +42,7 @@ __device__ __forceinline__ float asat_cell(float n, int side, int bc, int k, con
 // Implicit coupling of the fluid potential and the elastic uz at the
 // interface (we_op.cpp:2486-2512, the it >= 0 branch) in column ix, after the
 // fluid and the elastic part of the step, then the taper of the two interface
-// rows.
+// rows.  Every thread of a warp calls it.
 // e, w: the elastic and fluid tables of the shot; prev of both interface rows
 // (already tapered) is in halo_save.  sign = +1 forward, -1 adjoint.  With
 // F_GRAD, the density term of the imaging condition on the interface row,
@@ -55,6 +55,7 @@ __device__ __forceinline__ void ae_couple_column(const ShotDev &e, const ShotDev
     const long long nxz = (long long)e.nx * e.ldz;
     float *n1 = e.u[it & 1] + nxz;              // next uz, row 0
     float *na = w.u[it & 1] + (w.nz - 1);       // next potential, last fluid row
+    float amax = 0.f;   // of the coupled row, which the elastic kernel's maximum has not seen
     if (ix < e.nx) {
         const long long ie = (long long)ix * e.ldz, ia = (long long)ix * w.ldz;
         const float p1 = __ldcg(e.halo_save + ix), pa = __ldcg(w.halo_save + ix);
@@ -67,6 +68,7 @@ __device__ __forceinline__ void ae_couple_column(const ShotDev &e, const ShotDev
         na[ia] = a * w.tz[w.nz - 1] * w.tx[ix];
         const float a1 = b * e.tz[0] * e.tx[ix];
         n1[ie] = a1;
+        amax = fabsf(a1);
         const int tt = e.nt - 1 - (it + 1);
         if ((flags & F_GRAD) && tt % C.sub == 0 && tt / C.sub != 0) {
             // density term at snapshot itf with the coupled next field, as the
@@ -97,6 +99,11 @@ __device__ __forceinline__ void ae_couple_column(const ShotDev &e, const ShotDev
             else
                 *g2 = (float)((double)__ldcg(g2) + wdt * (double)(a0 * (-f0 + fm0) + a1 * (-f1 + fm1)));
         }
+    }
+    if ((flags & F_AMAX) && (it + 1) % C.sub == 0) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        if ((threadIdx.x & 31) == 0 && amax > 0.f) atomicMax(e.snap_amax + (it + 1) / C.sub, __float_as_uint(amax));
     }
 }
 

@@ -100,8 +100,6 @@ def test_fused_plan_equals_tile_plan(kind, prec, every, compensated):
     compensated accumulation: the loop is cut into several launches there."""
     if kind == O.KIND_AE and every:
         pytest.skip("checkpoint-and-recompute is not available for the acoustic-elastic propagator")
-    if kind == O.KIND_AE and prec:
-        pytest.skip("16-bit snapshots do not hold the acoustic-elastic interface row")
     a, ra = _gradient(kind, fused_shape(), prec, every, compensated)
     b, rb = _gradient(kind, 3, prec, every, compensated)
     for (ga, fa), (gb, fb) in zip(a, b):
@@ -145,8 +143,6 @@ def _imaging(kind, shape, prec, sub, nt=61):
 def test_fused_subsampled_imaging_equals_tile_plan(kind, prec, sub):
     """Snapshots every sub steps of 61 samples, up to one snapshot only (sub
     beyond the record: the first is the last, and none follows it)."""
-    if kind == O.KIND_AE and prec:
-        pytest.skip("16-bit snapshots do not hold the acoustic-elastic interface row")
     a, b = _imaging(kind, fused_shape(), prec, sub), _imaging(kind, 3, prec, sub)
     assert np.array_equal(a, b)
     if kind in (O.KIND_ELASTIC, O.KIND_VTI):

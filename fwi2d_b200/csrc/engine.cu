@@ -3061,7 +3061,7 @@ int fwi2d_snapshot(fwi2d_ctx *ctx, int shot, int slot, float *out)
     if (prec != FWI2D_SNAP_FP32) {
         float m;
         std::memcpy(&m, &amax, 4);
-        if (m > 0.f) inv = 1.f / std::ldexp(1.f, 14 - (std::ilogb(m) + 1));
+        if (m > 0.f) inv = 1.f / std::ldexp(1.f, std::min(14 - (std::ilogb(m) + 1), 126));   // as snap_scale
     }
     for (int c = 0; c < S.ncomp; c++)
         for (int ix = 0; ix < S.nx; ix++)

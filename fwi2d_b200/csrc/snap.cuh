@@ -18,7 +18,7 @@ __device__ __forceinline__ float snap_scale(const unsigned *amax, int slot)
     float m = __uint_as_float(__ldcg(amax + slot));   // earlier steps of the same launch may have set it
     if (!(m > 0.f)) return 1.f;
     int e = ilogbf(m) + 1;                 // m < 2^e
-    return ldexpf(1.f, 14 - e);
+    return ldexpf(1.f, min(14 - e, 126));   // a field below 2^-112 must not push the factor to infinity
 }
 
 __device__ __forceinline__ void snap_store(void *base, long long idx, int prec, float v, float scale)

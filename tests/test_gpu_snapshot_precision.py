@@ -53,3 +53,31 @@ def test_snapshot_precision_vs_fp64_oracle(kind, shape):
     for prec, (e_tr, e_g) in errs.items():
         assert e_tr <= 1e-4
         assert e_g <= BARS[prec]
+
+
+@pytest.mark.parametrize("kind", [O.KIND_ELASTIC, O.KIND_VTI, O.KIND_ACOUSTIC])
+@pytest.mark.parametrize("shape", [-1, 3])
+@pytest.mark.parametrize("prec", [F.SNAP_BF16, F.SNAP_FP16])
+def test_vanishing_fields_keep_a_finite_scale(kind, shape, prec):
+    """A source of 1e-32: the scale that brings a snapshot's largest value just
+    under 2^14 lies beyond the largest FP32 power of two, where it has to stop."""
+    nx, nz, d, nt = 60, 64, 0.01, 100
+    mc = K.converted(kind, K.model_case(kind, nx, nz, d, seed=9))
+    sl, rl = K.geometry(nx, nz, d, nr=12)
+    nc = 1 if kind == O.KIND_ACOUSTIC else 2
+    src = K.sources(nc, nt, 1e-3, f0=25.0, t0=0.03) * np.float32(1e-32)
+    adj = np.random.default_rng(3).normal(size=(nc, 12, nt)).astype(np.float32) * np.float32(1e24)
+    out = {}
+    for p in (F.SNAP_FP32, prec):
+        _, g, snaps = run_gpu(kind, mc, src, K.par_dict(nt=nt, dt=1e-3), nx, nz, d, sl, rl, adj_src=adj, shape=shape,
+                              prec=p)
+        out[p] = g, snaps
+    g32, s32 = out[F.SNAP_FP32]
+    g, s = out[prec]
+    assert 0 < np.abs(s32).max() < 2.0 ** -100 and np.abs(g32).max() > 0
+    assert np.isfinite(g).all() and np.isfinite(s).all()
+    # stored to 8 or 11 bits at worst relative to 2^-140, the smallest normal FP16 value over the largest scale
+    eps = {F.SNAP_BF16: 2.0 ** -8, F.SNAP_FP16: 2.0 ** -11}[prec]
+    assert np.abs(s - s32).max() <= eps * np.abs(s32).max()
+    # the second time difference of the density term amplifies the storage's rounding (as in test_gpu_ae_16bit)
+    assert K.rel_l2(g, g32) < {F.SNAP_BF16: 4e-1, F.SNAP_FP16: 5e-2}[prec]

@@ -297,11 +297,28 @@ __device__ __forceinline__ bool reached(const unsigned *count, unsigned target)
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
     return v >= target;
 }
+constexpr int kHardPolls = 1 << 22;
+// Before a CTA leaves a meeting it has given up: its first window's copies of what no step writes
+// may be on their way into its shared memory.  Their groups also count the fields' bytes, which
+// nobody will ask for; with those taken off, both phases complete once the copies have landed.
+// asked: 0, or 1 + 2 the lead group's phase + 4 the own group's + 8 if that one counts a gradient.
+__device__ __noinline__ void finish_copies(unsigned long long *bars, unsigned asked)
+{
+    if (!asked) return;
+    auto landed = [](unsigned long long *bar, unsigned parity, unsigned missing) {
+        asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(saddr(bar)), "r"(missing) : "memory");
+        for (int k = 0; k < kHardPolls && !bar_done(bar, parity); k++) {}
+    };
+    landed(bars, asked >> 1 & 1, 4u * 2 * kFu);
+    landed(bars + 1, asked >> 2 & 1, 4u * kFo * (asked & 8 ? 5 : 2));
+}
+
 // Waits until every CTA has finished the steps before `it`.  The launch is
 // cooperative, so all of them are resident.  Bounded twice: past StepConst::spin
-// polls the step is reported, past kHardPolls more the CTA leaves (false).
-constexpr int kHardPolls = 1 << 22;
-__device__ __forceinline__ bool meet_at(const unsigned *count, int *status, int spin, unsigned rounds, int it)
+// polls the step is reported, past kHardPolls more the CTA leaves (false); bars, asked:
+// what is on its way meanwhile (finish_copies).
+__device__ __forceinline__ bool meet_at(const unsigned *count, int *status, int spin, unsigned rounds, int it,
+                                        unsigned long long *bars = nullptr, unsigned asked = 0)
 {
     int lost = 0;
     if (threadIdx.x == 0 && rounds > 0) {
@@ -312,15 +329,17 @@ __device__ __forceinline__ bool meet_at(const unsigned *count, int *status, int 
             atomicCAS(status, 0, it + 1);
             for (int k = 0; k < kHardPolls && !ok; k++) ok = reached(count, target);
             lost = !ok;
+            if (lost && asked) finish_copies(bars, asked);
         }
     }
     return !__syncthreads_or(lost);
 }
 // (acoustic-elastic steps have two meetings: before the step and before its coupling)
 template <bool AE>
-__device__ __forceinline__ bool meet(const FusedArgs &A, int it)
+__device__ __forceinline__ bool meet(const FusedArgs &A, int it, unsigned long long *bars = nullptr,
+                                     unsigned asked = 0)
 {
-    return meet_at(A.count, A.status, A.C.spin, (AE ? 2u : 1u) * (unsigned)(it - A.it0), it);
+    return meet_at(A.count, A.status, A.C.spin, (AE ? 2u : 1u) * (unsigned)(it - A.it0), it, bars, asked);
 }
 
 // max |next| of a CTA for the scale of the next 16-bit snapshot
@@ -1832,7 +1851,8 @@ fused_steps(const __grid_constant__ FusedArgs A)
                     }
                     if (S16) set_factors(S, imaging<GRAD, AE>(S, A.C, it), inv_[q & 1]);
                 }
-                if (first && !meet<AE>(A, it)) return;
+                const bool grad = GRAD && imaging<GRAD, AE>(S, A.C, it).on;
+                if (first && !meet<AE>(A, it, bars, active ? 1 + 2 * par_lead + 4 * par_own + 8 * grad : 0)) return;
                 if (active && threadIdx.x == 0) {
                     fence_async();
                     issue_lead<VTI, GRAD, AE>(A, S, tr, it, false, true, sm, lead);

@@ -2003,6 +2003,7 @@ static cudaError_t launch_fused_t(const FusedArgs &A, cudaStream_t st)
 static cudaError_t encode(CUtensorMap *m, const void *base, int rank, const cuuint64_t *dim, const cuuint32_t *box,
                           bool half = false)
 {
+    if ((size_t)m % alignof(CUtensorMap)) return cudaErrorMisalignedAddress;   // the driver's rule, for the host copy too
     using Fn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                             const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                             CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -2026,8 +2027,9 @@ size_t fused_maps_bytes() { return SM_COUNT * sizeof(CUtensorMap); }
 cudaError_t fused_shot_maps(void *out, int nx, int ldz, const float *u0, const float *u1, const float *grad,
                             const void *snap, int nslot, bool half)
 {
-    CUtensorMap *m = (CUtensorMap *)out;
-    std::memset(m, 0, fused_maps_bytes());
+    CUtensorMap m[SM_COUNT];   // aligned as the driver asks, which `out` need not be
+    static_assert(alignof(CUtensorMap) == 64, "alignment of a tensor map");
+    std::memset(m, 0, sizeof(m));
     const cuuint64_t d2[3] = {(cuuint64_t)ldz, (cuuint64_t)nx, 2}, d3[3] = {(cuuint64_t)ldz, (cuuint64_t)nx, 3};
     const cuuint64_t ds[4] = {(cuuint64_t)ldz, (cuuint64_t)nx, 2, (cuuint64_t)nslot};
     const cuuint32_t lead[3] = {kFs, kFx + 8, 2}, own[4] = {kFz, kFx, 2, 1}, g[3] = {kFz, kFx, 3}, sl[4] = {kFs, kFx + 4, 2, 1};
@@ -2044,6 +2046,7 @@ cudaError_t fused_shot_maps(void *out, int nx, int ldz, const float *u0, const f
         e = encode(m + SM_SNAP_LEAD, snap, 4, ds, sl, half);
         if (e == cudaSuccess) e = encode(m + SM_SNAP_OWN, snap, 4, ds, half ? raw : own, half);
     }
+    std::memcpy(out, m, sizeof(m));
     return e;
 }
 

@@ -1560,7 +1560,8 @@ __device__ __forceinline__ bool acoustic_unit(const ShotDev *__restrict__ Sp, co
     __syncthreads();
 
     const float *U = sm + L::U + 2 * kFs, *IR = sm + L::IR, *F = sm + L::F;   // one index for all
-    if (!GRAD && (flags & F_EXTRACT)) {
+    // receivers of the tile: a cut tile's first half takes them all (every tile has one, its window covers both)
+    if (!GRAD && (flags & F_EXTRACT) && (inner || half == 0)) {
         const int r1 = Sp->ext_off[tr.unit + 1];
         for (int e = Sp->ext_off[tr.unit] + t; e < r1; e += kFt) {
             const ExtEntry &E = Sp->ext[e];

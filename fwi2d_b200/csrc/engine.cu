@@ -2134,6 +2134,36 @@ static long long adjoint_steps(fwi2d_ctx *ctx, const Plan &P, const ShotDev *sho
     return n;
 }
 
+// Launches of the steps [it0, it1), and of adjoint steps with their window
+// flushes: what launch_steps and adjoint_steps return.
+static long long count_steps(const Plan &P, int it0, int it1)
+{
+    if (it1 <= it0) return 0;
+    return P.fused ? 1 : (long long)(it1 - it0) * (P.march || P.framed || P.ae ? 3 : 1);
+}
+static long long count_adjoint(const Plan &P, int it0, int it1, int done)
+{
+    if (!P.par.compensated) return count_steps(P, it0, it1);
+    long long n = 0;
+    for (int it = it0; it < it1;) {
+        const int to = std::min(it1, it + kCompWindow - done % kCompWindow);
+        done += to - it;
+        n += count_steps(P, it, to) + (done % kCompWindow == 0);
+        it = to;
+    }
+    return n;
+}
+
+// Adjoint launches [lo, hi] of segment k under checkpointing: those whose
+// imaging times fall in [cuts[k], cuts[k+1]); acoustic imaging at launch it
+// uses time nt-1-it, the elastic one nt-2-it.
+static void checkpoint_adjoint_range(const Plan &P, int k, int &lo, int &hi)
+{
+    const int a = P.kind == KIND_ACOUSTIC ? 1 : 0, nt = P.nt_max, nseg = (int)P.cuts.size() - 1;
+    lo = k == nseg - 1 ? 0 : nt - 1 - P.cuts[k + 1] + a;
+    hi = k == 0 ? nt - 2 : nt - 2 - P.cuts[k] + a;
+}
+
 // Checkpoint-and-recompute time loops (all shots share nt, sub = 1).
 // Forward: receivers and 16-bit snapshot scales as usual, no snapshot store;
 // before launch cuts[k] - 1 (k >= 1) both field buffers of every shot are
@@ -2167,8 +2197,6 @@ static long long capture_checkpointed(fwi2d_ctx *ctx, Plan &P, bool adj, cudaStr
         launch_finalize(shots, nshots, P.C, ncomp, STEP_EXTRACT, cst);
         return n + 1;
     }
-    // acoustic imaging at launch it uses time nt-1-it, the elastic one nt-2-it
-    const int a = P.kind == KIND_ACOUSTIC ? 1 : 0;
     const ShotDev *last_adj = nullptr;
     int nadj = 0;   // adjoint launches so far (compensated accumulation windows)
     for (int k = nseg - 1; k >= 0; k--) {
@@ -2189,8 +2217,8 @@ static long long capture_checkpointed(fwi2d_ctx *ctx, Plan &P, bool adj, cudaStr
         n += launch_steps(ctx, P, rs, md, t0, t1, STEP_STORE, cst);
         launch_finalize(rs, nshots, P.C, ncomp, STEP_STORE, cst, t1);
         n++;
-        const int lo = k == nseg - 1 ? 0 : nt - 1 - P.cuts[k + 1] + a;
-        const int hi = k == 0 ? nt - 2 : nt - 2 - P.cuts[k] + a;
+        int lo, hi;
+        checkpoint_adjoint_range(P, k, lo, hi);
         n += adjoint_steps(ctx, P, as, md, lo, hi + 1, nadj, cst, P.all);
         nadj += hi + 1 - lo;
         last_adj = as;
@@ -3096,24 +3124,36 @@ int fwi2d_plan_info(fwi2d_ctx *ctx, long long *lf, long long *la, int *shape, lo
     ABI_TRY
     REQ(ctx, "null context");
     Plan &P = need_plan(ctx);
-    const long long per = (P.march || P.framed || P.ae) ? 3 : 1;
-    const bool loop = P.fused;   // one launch per run of steps
-    const long long nseg = P.ckpt > 0 ? (long long)P.cuts.size() - 1 : 0;
+    const int nseg = P.ckpt > 0 ? (int)P.cuts.size() - 1 : 0;
     const long long acf = P.kind == KIND_ACOUSTIC ? 1 : 0;
+    const bool flushes = P.par.compensated && !P.shots.empty() && P.shots[0]->gcomp.p;
     // per wave -- forward: init, steps, last sample (+ checkpoint copies);
     // adjoint: init, steps, acoustic final imaging, per-shot scatter (+ replays:
-    // restore, steps, last snapshot) and, with compensated accumulation, one
-    // window flush per kCompWindow adjoint launches plus the final one
+    // restore, steps, last snapshot) and, with compensated accumulation, the
+    // window flushes among the steps and the final one
     long long f = 0, a = 0;
     for (const auto &W : P.waves) {
-        const long long steps = W.nt_max - 1;
-        const long long flushes = P.par.compensated && P.par.sub > 0 ? steps / kCompWindow + 1 : 0;
-        const long long runs = std::max<long long>(nseg, 1);
-        const long long fsteps = loop ? runs : steps * per;
-        const long long asteps = loop ? (flushes ? std::max(flushes, runs) : runs) : steps * per;
-        const long long replay = loop ? nseg : (steps + nseg - 1) * per;
-        f += fsteps + 2 + (P.ae ? 1 : 0) + (nseg > 0 ? nseg - 1 : 0);
-        a += asteps + 1 + acf + (W.s1 - W.s0) + (nseg > 0 ? replay + 2 * nseg : 0) + flushes;
+        const int steps = W.nt_max - 1;
+        long long nf = 2 + (P.ae ? 1 : 0), na = 1 + acf + (flushes ? 1 : 0);
+        if (nseg == 0) {
+            nf += count_steps(P, 0, steps);
+            na += count_adjoint(P, 0, steps, 0);
+        }
+        int from = 0, done = 0;
+        for (int k = 1; k <= nseg; k++) {   // capture_checkpointed's forward
+            const int to = k < nseg ? P.cuts[k] - 1 : steps;
+            nf += count_steps(P, from, to) + (k < nseg ? 1 : 0);
+            from = to;
+        }
+        for (int k = nseg - 1; k >= 0; k--) {   // and adjoint
+            int lo, hi;
+            checkpoint_adjoint_range(P, k, lo, hi);
+            na += 2 + count_steps(P, k == 0 ? 0 : P.cuts[k] - 1, P.cuts[k + 1]) + count_adjoint(P, lo, hi + 1, done);
+            done += hi + 1 - lo;
+        }
+        // what a pass captured, where one has run
+        f += W.launches[0] ? W.launches[0] : nf;
+        a += (W.launches[1] ? W.launches[1] : na) + (W.s1 - W.s0);
     }
     if (lf) *lf = f;
     if (la) *la = a;

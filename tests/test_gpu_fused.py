@@ -195,3 +195,41 @@ def test_fused_wait_limit_returns_timeout(monkeypatch):
         out.append(P.forward(src, store=False)[0])
     P.close()
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("kind,shape,nt,every,compensated,adjoint", [
+    (O.KIND_ELASTIC, -1, 97, 0, 1, 1 + 12 + 12 + 1 + 1),       # 12 windows of 8 steps
+    (O.KIND_ELASTIC, -1, 100, 0, 1, 1 + 13 + 12 + 1 + 1),      # and one of 3
+    (O.KIND_ELASTIC, -1, 97, 20, 1, None),                     # cut by windows and by segments
+    (O.KIND_ACOUSTIC, -1, 60, 7, 1, None),
+    (O.KIND_ELASTIC, -1, 60, 1, 0, None),                      # a segment a step: its first forward run is empty
+    (O.KIND_ELASTIC, -1, 60, 0, 0, 1 + 1 + 1),
+    (O.KIND_AE, -1, 60, 0, 1, None),
+    (O.KIND_ELASTIC, 3, 97, 0, 1, 1 + 96 + 12 + 1 + 1),
+    (O.KIND_ELASTIC, 14, 60, 7, 1, None),
+    (O.KIND_ACOUSTIC, 3, 60, 7, 0, None),
+])
+def test_plan_info_counts_the_launches(kind, shape, nt, every, compensated, adjoint):
+    """The counts of a plan that has not run are those its passes then capture
+    (init, steps, flushes, final flush, scatter of one shot)."""
+    nx, nz, d = 60, 64, 0.01
+    base = O.KIND_ELASTIC if kind == O.KIND_AE else kind
+    mc = K.converted(base, K.model_case(base, nx, nz, d, seed=11))
+    oz = 19 * d if kind == O.KIND_AE else 0.0
+    sl, rl = K.geometry(nx, nz, d, nr=8, sz=0.2)
+    pd = K.par_dict(nt=nt, dt=1e-3)
+    kw = {}
+    if kind == O.KIND_AE:
+        pd.update(nza=20, acoustic_source=0)
+        kw = dict(water_rcv_x=rl[0], water_rcv_z=rl[1])
+    P = F.Propagator(0)
+    P.set_model(kind, mc, d, d, 0.0, oz)
+    P.set_shots(F.make_params(**pd, tile_shape=shape, checkpoint_every=every, compensated=compensated),
+                [F.ShotSpec(0, nx, nt, sl[0], sl[1] + np.float32(oz), rl[0], rl[1] + np.float32(oz), **kw)])
+    before = P.plan_info()
+    rcv = P.forward([K.sources(P.ncomp(), nt, 1e-3)], store=True)
+    P.adjoint(rcv)
+    after = P.plan_info()
+    P.close()
+    assert before == after
+    assert adjoint is None or after["launches_adjoint"] == adjoint

@@ -561,7 +561,10 @@ static bool band_split_for(int nshots, int nz)
 // Microseconds a step, forward / adjoint, launch-per-step plan as tuned -> fused:
 // one 801 x 401 shot 16.1 / 21.5 -> 8.3 / 11.9, eight of them 87 / 139 -> 48 / 81;
 // one 81 x 61 shot 14.6 / 15 or more -> 4.8 / 7.1; three acoustic 401 x 301 shots
-// 23 / 30 -> 11.5 / 19.1.
+// 23 / 30 -> 11.5 / 19.1.  Compensated accumulation cuts its adjoint into launches
+// of 8 steps and stays ahead, adjoint: one 401 x 301 shot 16.0 -> 11.6 (acoustic
+// 15.1 -> 10.4), one 801 x 401 24.2 -> 15.1, eight 401 x 301 64.0 -> 38.1, one
+// 2001 x 801 99.9 -> 58.4.
 static int fused_shape() { return elastic_tile_count() + kNumMarch + kNumFramed; }
 static int shape_count() { return fused_shape() + 1; }
 static bool is_march_shape(int s) { return s >= elastic_tile_count() && s < elastic_tile_count() + kNumMarch; }
@@ -1378,8 +1381,9 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
         P->wIR.upload(wir, ctx->st);
     }
 
-    // shape: the requested one, else the marching kernel where it has enough
-    // units to fill the GPU, else the first tile shape that fits every shot
+    // shape: the requested one, else the fused time loop, else the first tile
+    // shape that fits every shot (marching and framed shapes fit no grid that the
+    // loop does not: they are taken on request only)
     auto shape_ok = [&](int i) {
         if ((acoustic || ae) && !acoustic_shape_ok(i) && i != fused_shape()) return false;
         for (int s = 0; s < nshots; s++)
@@ -1389,13 +1393,6 @@ static void set_shots_impl(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, 
     int shape = p.tile_shape;
     if (shape < 0 || shape >= shape_count()) {
         shape = shape_ok(fused_shape()) ? fused_shape() : -1;
-        const int m0 = elastic_tile_count();
-        if (shape < 0 && !acoustic && !ae && shape_ok(m0)) {
-            long long units = 0;
-            for (int s = 0; s < nshots; s++)
-                units += (long long)make_units(m0, s, shots[s].nx, M.nz, false).marches.size();
-            if (units >= 148) shape = m0;
-        }
         for (int i = 0; i < elastic_tile_count() && shape < 0; i++)
             if (shape_ok(i)) shape = i;
         REQ(shape >= 0, "no tile shape fits the grid (an axis needs n == T or n >= T + 8)");
@@ -1957,10 +1954,11 @@ static void tune_file_store(const std::string &key, int shape)
     std::fclose(f);
 }
 
-// Tile-shape autotuner: for plans that leave the shape open (tile_shape < 0),
-// time forward steps of every shape that tiles the grids -- plus adjoint
-// steps with the imaging condition for plans that keep snapshots (gradients)
-// -- and keep the fastest.  The forward is sampled in kTuneWindows windows
+// Tile-shape autotuner: for plans that leave the shape open (tile_shape < 0) on
+// grids that the fused time loop does not take (32 rows; acoustic shots of 17 to
+// 23 columns), time forward steps of every tile shape that fits the grids -- plus
+// adjoint steps with the imaging condition for plans that keep snapshots
+// (gradients) -- and keep the fastest.  The forward is sampled in kTuneWindows windows
 // centred on equal parts of the whole time loop, so that a batch whose
 // shorter records end early is judged on its emptier late steps too (there,
 // units fewer than a wave favour narrower shapes); the adjoint, timed with
@@ -2009,7 +2007,7 @@ static void set_shots(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, const
     const int fshape = ctx->M.kind == KIND_ACOUSTIC ? kAcousticTile : fused_shape();
     bool fused = true;
     for (int i = 0; i < nshots && fused; i++) fused = shape_fits(fshape, shots[i].nx, ctx->M.nz);
-    // the fused time loop is the fastest shape wherever it fits: nothing to time
+    // the fused time loop is the fastest shape wherever it fits (fused_shape): nothing to time
     if (p.tile_shape < 0 && ctx->M.kind >= 0 && !fused) {
         static std::vector<std::pair<std::string, int>> cache;
         const bool grad = p.sub > 0;
@@ -2032,7 +2030,7 @@ static void set_shots(fwi2d_ctx *ctx, const fwi2d_params *par, int nshots, const
         if (chosen < 0 && cells >= 20000000LL) {
             float best = 1e30f;
             std::vector<std::pair<float, int>> scored;
-            for (int s = 0; s < shape_count(); s++) {
+            for (int s = 0; s < elastic_tile_count(); s++) {
                 fwi2d_params q = p;
                 q.tile_shape = s;
                 q.sub = 0;

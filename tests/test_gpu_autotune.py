@@ -1,6 +1,6 @@
 """The tile-shape autotuner on gradient plans large enough to be tuned
-(>= 2e7 cell-steps) and on grids that the fused time loop does not take (32 rows;
-acoustic shots of 17 to 23 columns): two shots of different record lengths,
+(>= 2e7 cell-steps) and on grids that the fused time loop does not take (elastic
+grids of 32 rows, acoustic shots of 17 to 23 columns): two shots of different record lengths,
 tile_shape = -1.
 
 The tuner builds and times candidate plans (sampled forward windows, adjoint

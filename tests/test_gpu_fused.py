@@ -233,3 +233,50 @@ def test_plan_info_counts_the_launches(kind, shape, nt, every, compensated, adjo
     P.close()
     assert before == after
     assert adjoint is None or after["launches_adjoint"] == adjoint
+
+
+def _spots(limit, per, pivots, corner, over):
+    """Points whose 3 x 3 footprints put exactly `limit` entries (beyond it: two
+    corner ones more) into one unit: `per` entries a point inside it, one cell's
+    for each point around `corner`."""
+    n = limit // (9 * per)
+    k = (limit - n * 9 * per) // per + 2 * over
+    pts = [pivots[i % len(pivots)] for i in range(n)] + [corner] * k
+    return [(x + 0.3 - 0.011 * i % 0.5, z + 0.2 - 0.007 * i % 0.4) for i, (x, z) in enumerate(pts)]
+
+
+@pytest.mark.parametrize("kind,mt", [(O.KIND_ELASTIC, 0), (O.KIND_ELASTIC, 1), (O.KIND_VTI, 0), (O.KIND_ACOUSTIC, 0)])
+@pytest.mark.parametrize("over", [0, 1, 30])
+def test_fused_dense_arrays_vs_oracle(kind, mt, over):
+    """As many injection entries as a unit stages, and more: windows 256, bands 512
+    in the adjoint and 256 in the forward, acoustic tiles 512."""
+    nx, nz, d, nt = 45, 75, 0.01, 60
+    mc = K.converted(kind, K.model_case(kind, nx, nz, d, seed=3))
+    if kind == O.KIND_ACOUSTIC:
+        inner = [(x, z) for x in range(2, 14) for z in range(2, 30, 3)]
+        s = r = _spots(512, 1, inner, (16, 32), over)
+    else:
+        window = [(x, z) for x in range(24, 36, 2) for z in range(38, 64, 3)]   # cells 22..37, 36..67
+        band = [(x, z) for x in range(1, 5) for z in range(1, 23)]           # cells 0..5, 0..24
+        top = [(x, 2) for x in range(8, 32)]                                 # cells 6..33, 0..5
+        s = (_spots(256, 2, window, (38, 68), over) + _spots(256, 2, band, (6, 25), over) +
+             _spots(256, 2, top, (34, 6), over))
+        r = (_spots(256, 2, window, (38, 68), over) + _spots(512, 2, band, (6, 25), over) +
+             _spots(512, 2, top, (34, 6), over))
+    sl, rl = (tuple(np.array([p[c] * d for p in q], np.float32) for c in (0, 1)) for q in (s, r))
+    pd = K.par_dict(nt=nt, dt=1e-3, mt=mt, taper=(0, 6, 5, 6))
+    nc = 1 if kind == O.KIND_ACOUSTIC else (3 if mt else 2)
+    src = np.repeat(K.sources(nc, nt, 1e-3, f0=25.0, t0=0.03), len(s), axis=1)
+    src = (src * np.random.default_rng(2).normal(size=(1, len(s), 1))).astype(np.float32)
+    port = O.Port(32)
+    par = O.make_par(**pd, ns=len(s), nr=len(r))
+    rcv_o, full_o = K.oracle_forward(port, kind, mc, src, par, nx, nz, d, sl, rl, mt=mt)
+    adj = np.ascontiguousarray(rcv_o[:, :, ::-1])
+    ng = 5 if kind == O.KIND_VTI else (2 if kind == O.KIND_ACOUSTIC else 3)
+    g_o = np.zeros((ng, nx, nz), np.float32)
+    port.propagate(kind, 1, mc, adj, np.zeros((nc, len(s), nt), np.float32), par, nx, nz, d, d, 0.0, 0.0, rl, sl,
+                   inj_type=0, full=full_o, grad=g_o)
+    rcv_g, g_g, _ = run_gpu(kind, mc, src, pd, nx, nz, d, sl, rl, adj_src=adj, mt=mt, shape=fused_shape())
+    assert np.abs(g_o).max() > 0
+    assert np.array_equal(rcv_g, rcv_o)
+    assert np.array_equal(g_g, g_o[:3])

@@ -1955,8 +1955,8 @@ static void tune_file_store(const std::string &key, int shape)
 }
 
 // Tile-shape autotuner: for plans that leave the shape open (tile_shape < 0) on
-// grids that the fused time loop does not take (32 rows; acoustic shots of 17 to
-// 23 columns), time forward steps of every tile shape that fits the grids -- plus
+// grids that the fused time loop does not take (elastic grids of 32 rows, acoustic
+// shots of 17 to 23 columns), time forward steps of every tile shape that fits the grids -- plus
 // adjoint steps with the imaging condition for plans that keep snapshots
 // (gradients) -- and keep the fastest.  The forward is sampled in kTuneWindows windows
 // centred on equal parts of the whole time loop, so that a batch whose

@@ -126,8 +126,10 @@ __device__ __forceinline__ float2 mulx(float ax, float ay, float2 b) { return ma
 // x / b rounded to nearest single precision from inv, 1/b in double precision
 // with a relative error below 2^-51: the quotient of two 24-bit significands
 // lies at least 2^-49 (relative) away from every midpoint of two neighbouring
-// single-precision numbers, so the double product rounds to the same number.
-// No branch, any magnitude, signed zeros included.
+// normal single-precision numbers, so the double product rounds to the same
+// number.  No branch, signed zeros included.  A subnormal quotient has fewer bits
+// and can be such a midpoint itself: it may then round to the other neighbour,
+// 2^-149 away.
 __device__ __forceinline__ float div64(float x, double inv) { return (float)((double)x * inv); }
 
 // Both components of a z-pair over the pair's densities b, with r = 1/b rounded

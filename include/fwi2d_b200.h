@@ -72,7 +72,7 @@ typedef struct fwi2d_params {
                                                             * each such partial sum joins a running (hi, lo) pair by
                                                             * Neumaier's compensated summation; 0: the reference's
                                                             * plain FP32 accumulation (bitwise) */
-    int tile_shape;                                        /* -1: autotuned; else fwi2d_tile_shape index */
+    int tile_shape;                                        /* -1: the fused time loop, else an autotuned tile shape; or a fwi2d_tile_shape index */
 } fwi2d_params;
 
 /* Public tables of the reference's injector (src/include/injector.hpp:9-13). */
@@ -241,7 +241,7 @@ int fwi2d_copy_gradient(fwi2d_ctx *ctx, float *dst_device);
  * adjoint time loops, in milliseconds (-1 if none ran). */
 int fwi2d_last_timing(fwi2d_ctx *ctx, float *forward_ms, float *adjoint_ms);
 
-/* Work shapes offered to the autotuner: tile shapes of the tile kernel over
+/* Work shapes: tile shapes of the tile kernel over
  * whole shot grids (tz x tx cells), then marching shapes (tz threads, one z
  * cell each, marching runs of tx rows) for the cells clear of the boundary
  * bands, then framed tile shapes (tz x tx tiles of the tile kernel's interior

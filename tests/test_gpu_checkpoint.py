@@ -57,6 +57,11 @@ CASES = [
     (O.KIND_ELASTIC, 14, F.SNAP_FP16, (72, 80)),     # framed plans: interior windows + frame kernels
     (O.KIND_VTI, 14, F.SNAP_FP32, (72, 80)),
     (O.KIND_ELASTIC, 16, F.SNAP_FP32, (72, 100)),
+    (O.KIND_ELASTIC, -1, F.SNAP_FP32, (72, 80)),     # the time loop, cut at the segments
+    (O.KIND_ELASTIC, -1, F.SNAP_FP16, (47, 41)),
+    (O.KIND_VTI, -1, F.SNAP_BF16, (72, 80)),
+    (O.KIND_ACOUSTIC, -1, F.SNAP_FP32, (72, 80)),
+    (O.KIND_ACOUSTIC, -1, F.SNAP_FP16, (72, 80)),
 ]
 
 

@@ -280,3 +280,36 @@ def test_fused_dense_arrays_vs_oracle(kind, mt, over):
     assert np.abs(g_o).max() > 0
     assert np.array_equal(rcv_g, rcv_o)
     assert np.array_equal(g_g, g_o[:3])
+
+
+def test_two_contexts_run_their_loops_at_once():
+    """Two threads, a context and a stream each, both with more units than the GPU
+    holds CTAs: a cooperative launch starts with all of its CTAs or waits, so
+    neither loop starves the other, and results are those of each alone."""
+    import threading
+    nx, nz, d, nt = 400, 300, 0.01, 150
+    jobs = []
+    for k, kind in enumerate((O.KIND_ELASTIC, O.KIND_ACOUSTIC)):
+        mc = K.converted(kind, K.model_case(kind, nx, nz, d, seed=3 + k))
+        sl, rl = K.geometry(nx, nz, d, nr=20)
+        P = F.Propagator(0)
+        P.set_model(kind, mc, d, d)
+        P.set_shots(F.make_params(**K.par_dict(nt=nt, dt=1e-3)), [F.ShotSpec(0, nx, nt, sl[0], sl[1], rl[0], rl[1])] * 2)
+        src = [K.sources(P.ncomp(), nt, 1e-3)] * 2
+        obs = [np.zeros((P.ncomp(), 20, nt), np.float32)] * 2
+        jobs.append((P, mc, src, obs, P.fwi_gradient(mc, src, obs)))
+    bad = []
+
+    def work(P, mc, src, obs, want):
+        for _ in range(8):
+            g, f = P.fwi_gradient(mc, src, obs)
+            if f != want[1] or not np.array_equal(g, want[0]):
+                bad.append(f)
+    threads = [threading.Thread(target=work, args=j) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for j in jobs:
+        j[0].close()
+    assert not bad

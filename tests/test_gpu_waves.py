@@ -9,8 +9,8 @@ shots.  FWI2D_SNAPSHOT_BUDGET replaces the budget so that a small batch
 splits here.
 
 Checks, for the elastic and VTI propagators on the tile and the marching
-plans, and for the acoustic and acoustic-elastic propagators on their tile
-plans: a batch of uneven shots (cropped grids, uneven record lengths) split
+plans, for the acoustic and acoustic-elastic propagators on their tile plans,
+and for all four on the time loop: a batch of uneven shots (cropped grids, uneven record lengths) split
 into three or more waves gives the same gradient and misfit as the same
 batch in one wave, bitwise; its plan holds the snapshots of one wave only;
 the forward without snapshots still runs every shot at once, while a forward
@@ -80,7 +80,8 @@ def _gradient(kind, raw, true, specs, srcs, pd, d, shape):
 
 
 @pytest.mark.parametrize("kind,shape", [(O.KIND_ELASTIC, 3), (O.KIND_ELASTIC, 8), (O.KIND_VTI, 3), (O.KIND_VTI, 8),
-                                        (O.KIND_ACOUSTIC, 3), (O.KIND_AE, 3)])
+                                        (O.KIND_ACOUSTIC, 3), (O.KIND_AE, 3), (O.KIND_ELASTIC, -1),
+                                        (O.KIND_VTI, -1), (O.KIND_ACOUSTIC, -1), (O.KIND_AE, -1)])
 def test_waves_match_one_wave(kind, shape, monkeypatch):
     raw, true, specs, srcs, pd, d = _batch(kind)
     P1, g1, phi1, info1 = _gradient(kind, raw, true, specs, srcs, pd, d, shape)

@@ -84,10 +84,9 @@ def peaks():
 # Per framed plan of the single-shot grid: DRAM bytes (dram__bytes_read.sum +
 # dram__bytes_write.sum) of the core, x-band and z-band launches of one
 # adjoint step, and the core launch's L1-to-L2 bytes, cold duration and L2
-# throughput, from the captures summarised in
-# profiles/elastic_step_framed_single_shot_401x801.md and, for the split band
-# kernels that one shot takes, profiles/elastic_band_split_single_shot_401x801.md
-# (cold caches: ncu flushes L2 before each pass).
+# throughput, from the captures summarised under profiles/ (framed step and, for
+# the band kernels that one shot takes, split bands; cold caches: ncu flushes L2
+# before each pass).
 FRAMED_CAPTURES = {
     16: dict(core="elastic_step<RZ=2, CORE> (64 x 8 z-pair windows)",
              traffic={"core": 21.133312e6, "x_bands": 0.554496e6, "z_bands": 3.61984e6},
@@ -138,8 +137,7 @@ def l2_note(shape, config):
         return None
     return {"kernel": cap["core"] + " adjoint", "l1_to_l2_bytes_per_launch": cap["l2_bytes"],
             "achieved_gbs": cap["l2_bytes"] / (cap["core_cold_us"] * 1e-6) / 1e9, "lts_throughput_pct": cap["lts_pct"],
-            "source": "ncu capture, cold caches (profiles/elastic_step_framed_single_shot_401x801.md, "
-                      "profiles/elastic_band_split_single_shot_401x801.md)"}
+            "source": "ncu capture, cold caches (summaries under profiles/)"}
 
 
 # ---------------------------------------------------------------------------
